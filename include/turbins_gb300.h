@@ -224,9 +224,11 @@ int turb_set_mg_sweeps(turb_ctx *ctx, int npre, int npost);
 /* levels from_level and coarser (0 = the finest, >= 1) of the current
  * pressure mode's V-cycle smooth with npre / npost sweeps (1..16) instead */
 int turb_set_mg_coarse_sweeps(turb_ctx *ctx, int from_level, int npre, int npost);
-/* the V-cycle from the first level of at most max_cells cells (default
- * 4096; 0: never) down to the coarsest and back runs as one single-block
- * kernel instead of a launch per half sweep; results are bit-identical */
+/* the V-cycle from the first level of at most max_cells cells (0: never;
+ * default 32768) down to the coarsest and back runs as one launch instead of
+ * a launch per half sweep: one thread-block cluster with the levels in
+ * shared memory where they fit, else a single block (by default only from
+ * 4096 cells on); results are bit-identical */
 int turb_set_mg_tail(turb_ctx *ctx, long long max_cells);
 /* with TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level of at most
  * max_cells cells (default 131072; 0: never) runs as one thread-block

@@ -427,19 +427,22 @@ template <typename T>
 __device__ __forceinline__ void restrict_cell(const MgDevLevel &Lf, const MgDevLevel &Lc, const T *__restrict__ rf,
                                               T *__restrict__ bc, int I, int J, int K)
 {
+    // the lists are padded with weight 0 to four entries, so the sixteen loads
+    // of a plane are independent
     long long c = ((long long)K * Lc.ny + J) * Lc.nx + I;
-    const T *rwx = rw_of<T>(Lf.tx), *rwy = rw_of<T>(Lf.ty), *rwz = rw_of<T>(Lf.tz);
-    int nxx = Lf.tx.rcnt[I], nyy = Lf.ty.rcnt[J], nzz = Lf.tz.rcnt[K];
+    const T *rwx = rw_of<T>(Lf.tx) + 4 * I, *rwy = rw_of<T>(Lf.ty) + 4 * J, *rwz = rw_of<T>(Lf.tz) + 4 * K;
+    const bool cx = Lc.nx != Lf.nx;   // else one entry of weight 1 along x
+    const int nzz = Lf.tz.rcnt[K];
     T s = 0;
-    for (int c3 = 0; c3 < nzz; c3++) {
-        int k = Lf.tz.rf[4 * K + c3];
-        T wz = rwz[4 * K + c3];
-        for (int b = 0; b < nyy; b++) {
-            int j = Lf.ty.rf[4 * J + b];
-            T wyz = rmul(wz, rwy[4 * J + b]);
-            const T *row = rf + ((long long)k * Lf.ny + j) * Lf.nx;
-            for (int a = 0; a < nxx; a++) s = rfma(rmul(wyz, rwx[4 * I + a]), row[Lf.tx.rf[4 * I + a]], s);
-        }
+    for (int h = 0; h < nzz; h++) {
+        const T *plane = rf + (long long)Lf.tz.rf[4 * K + h] * Lf.ny * Lf.nx;
+        T val[4][4];
+#pragma unroll
+        for (int d = 0; d < 4; d++)
+#pragma unroll
+            for (int f = 0; f < 4; f++)
+                if (f == 0 || cx) val[d][f] = plane[Lf.ty.rf[4 * J + d] * Lf.nx + Lf.tx.rf[4 * I + f]];
+        s = mg_restrict16<T>(s, val, rwz[h], rwy, rwx, cx);
     }
     bc[lev_at(Lc, c, I, J, K)] = s;
 }
@@ -450,23 +453,14 @@ __device__ __forceinline__ void prolong_cell(const MgDevLevel &Lf, const MgDevLe
 {
     long long c = ((long long)k * Lf.ny + j) * Lf.nx + i;
     int Ix[2] = {Lf.tx.I0[i], Lf.tx.I1[i]}, Iy[2] = {Lf.ty.I0[j], Lf.ty.I1[j]}, Iz[2] = {Lf.tz.I0[k], Lf.tz.I1[k]};
-    T wx[2] = {pw0_of<T>(Lf.tx)[i], pw1_of<T>(Lf.tx)[i]};
-    T wy[2] = {pw0_of<T>(Lf.ty)[j], pw1_of<T>(Lf.ty)[j]};
-    T wz[2] = {pw0_of<T>(Lf.tz)[k], pw1_of<T>(Lf.tz)[k]};
-    T acc = 0;
+    T val[8];
 #pragma unroll
-    for (int d = 0; d < 2; d++) {
-        if (wz[d] == T(0)) continue;
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            if (wy[b] == T(0)) continue;
-            long long row = ((long long)Iz[d] * Lc.ny + Iy[b]) * Lc.nx;
-            T wyz = rmul(wz[d], wy[b]);
-#pragma unroll
-            for (int a = 0; a < 2; a++)
-                if (wx[a] != T(0)) acc = rfma(rmul(wyz, wx[a]), xc[lev_at(Lc, row + Ix[a], Ix[a], Iy[b], Iz[d])], acc);
-        }
+    for (int e = 0; e < 8; e++) {
+        const int a = e & 1, b = (e >> 1) & 1, d = e >> 2;
+        val[e] = xc[lev_at(Lc, ((long long)Iz[d] * Lc.ny + Iy[b]) * Lc.nx + Ix[a], Ix[a], Iy[b], Iz[d])];
     }
+    const T acc = mg_prolong8<T>(val, pw0_of<T>(Lf.tx)[i], pw1_of<T>(Lf.tx)[i], pw0_of<T>(Lf.ty)[j], pw1_of<T>(Lf.ty)[j],
+                                 pw0_of<T>(Lf.tz)[k], pw1_of<T>(Lf.tz)[k]);
     long long o = lev_at(Lf, c, i, j, k);
     xf[o] = radd(xf[o], acc);
 }
@@ -538,14 +532,22 @@ __global__ void k_restrict_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *__rest
     for (int c3 = 0; c3 < nzz; c3++) {
         const int k = Lf.tz.rf[4 * K + c3];
         const float wz = Lf.tz.rwf[4 * K + c3];
-        for (int b = 0; b < nyy; b++) {
-            const int j = Lf.ty.rf[4 * J + b];
-            const float wyz = __fmul_rn(wz, Lf.ty.rwf[4 * J + b]);
-            const float *row = rf + ((size_t)(k * Lf.ny + j) * Lf.nx + i0);
-            const float4 a0 = *reinterpret_cast<const float4 *>(row), a1 = *reinterpret_cast<const float4 *>(row + 4);
-            const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        float4 a0[4], a1[4];
 #pragma unroll
-            for (int e = 0; e < 8; e++) s[e] = __fmaf_rn(wyz, v[e], s[e]);
+        for (int b = 0; b < 4; b++) {
+            const float *row = rf + ((size_t)(k * Lf.ny + Lf.ty.rf[4 * J + b]) * Lf.nx + i0);
+            if (b < nyy) {
+                a0[b] = *reinterpret_cast<const float4 *>(row);
+                a1[b] = *reinterpret_cast<const float4 *>(row + 4);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (b >= nyy) continue;
+            const float w = __fmul_rn(wz, Lf.ty.rwf[4 * J + b]);
+            const float v[8] = {a0[b].x, a0[b].y, a0[b].z, a0[b].w, a1[b].x, a1[b].y, a1[b].z, a1[b].w};
+#pragma unroll
+            for (int e = 0; e < 8; e++) s[e] = __fmaf_rn(w, v[e], s[e]);
         }
     }
     st8(Lc, bc, i0, J, K, s);
@@ -561,19 +563,15 @@ __global__ void k_prolong_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *__restr
     const int i0 = 8 * q;
     const int Iy[2] = {Lf.ty.I0[j], Lf.ty.I1[j]}, Iz[2] = {Lf.tz.I0[k], Lf.tz.I1[k]};
     const float wy[2] = {Lf.ty.w0f[j], Lf.ty.w1f[j]}, wz[2] = {Lf.tz.w0f[k], Lf.tz.w1f[k]};
+    float v[4][8];
+#pragma unroll
+    for (int d = 0; d < 4; d++) ld8(Lc, xc, i0, Iy[d & 1], Iz[d >> 1], v[d]);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int d = 0; d < 2; d++) {
-        if (wz[d] == 0.0f) continue;
+    for (int d = 0; d < 4; d++) {   // mg_prolong8 with the x weights 1 and 0
+        const float w = __fmul_rn(wz[d >> 1], wy[d & 1]);
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            if (wy[b] == 0.0f) continue;
-            const float wyz = __fmul_rn(wz[d], wy[b]);
-            float v[8];
-            ld8(Lc, xc, i0, Iy[b], Iz[d], v);
-#pragma unroll
-            for (int e = 0; e < 8; e++) acc[e] = __fmaf_rn(wyz, v[e], acc[e]);
-        }
+        for (int e = 0; e < 8; e++) acc[e] = __fmaf_rn(w, v[d][e], acc[e]);
     }
     float x8[8];
     ld8(Lf, xf, i0, j, k, x8);
@@ -596,9 +594,7 @@ __global__ void k_coarse(int n, const double *__restrict__ ainv, const T *__rest
 {
     pdl_trigger();
     pdl_wait();
-    int r = threadIdx.x;
-    if (r >= n) return;
-    coarse_row<T>(n, ainv, b, x, r);
+    for (int r = threadIdx.x; r < n; r += blockDim.x) coarse_row<T>(n, ainv, b, x, r);
 }
 
 // The V-cycle from level l0 down to the coarsest and back in one block of
@@ -946,6 +942,7 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
     const MgDevLevel &L = H.lev[l];
     const int npre = pre[l], npost = post[l];
     long long n = (long long)L.nx * L.ny * L.nz;
+    if (H.tail_from >= 0 && l == H.tail_from && l < H.nl - 1 && mg_low<T>(s, H, l, pre, post)) return;
     if (H.tail_from >= 0 && l == H.tail_from && H.nl - l <= MG_TAIL_MAXLEV && l < H.nl - 1) {
         TailArgs<T> a;
         a.nlev = H.nl - l;
@@ -1069,7 +1066,7 @@ double mg_vcycle_bytes(const MgHier<T> &H, int l, const int *pre, const int *pos
     for (; l < H.nl; l++) {
         const MgDevLevel &L = H.lev[l];
         double n = (double)L.nx * L.ny * L.nz;
-        bool tail = H.tail_from >= 0 && l == H.tail_from && H.nl - l <= MG_TAIL_MAXLEV && l < H.nl - 1;
+        bool tail = H.tail_from >= 0 && l == H.tail_from && l < H.nl - 1;
         if (tail || l == H.nl - 1) {
             for (int t = l; t < H.nl; t++) {
                 const MgDevLevel &M = H.lev[t];
@@ -1110,7 +1107,7 @@ int mg_vcycle_launches(int nl, const int *pre, const int *post, int tail_from, i
     int n = 1;
     for (int l = 0; l < nl - 1; l++) {
         if (cluster_from >= 0 && l == cluster_from && nl - l <= MG_CLUSTER_MAXLEV) return n;
-        if (tail_from >= 0 && l == tail_from && nl - l <= MG_TAIL_MAXLEV) return n;
+        if (tail_from >= 0 && l == tail_from) return n;
         n += 2 * pre[l] + 3 + 2 * post[l];
         if (l == 0 && tb0) n -= 3 * ((pre[l] / 4) * 2 + (post[l] / 4) * 2);
     }

@@ -174,6 +174,7 @@ struct turb_ctx {
     // kernel variants (TURB_KV_*): FP32 sweeps marching along k through
     // shared-memory plane tiles, ENO y / z lines walked in segments
     int kvariant = TURB_KV_ENO_SEGMENTS | TURB_KV_PDL;
+    long long mg_tail_cells = -1;   // turb_set_mg_tail (-1: the default rule of place_tail)
     long long mg_cluster_cells = 1 << 17;   // TURB_KV_CLUSTER_VCYCLE from the first level of at most this many cells
     // TURB_KV_SWEEP_PAIRS: the finest FP32 level's two-sweeps-per-pass smoother
     RbTbPlan tbplan;
@@ -667,7 +668,7 @@ std::vector<HostLev> mg_host(turb_ctx *c)
 
 // linear prolongation along one direction between cell centres (positions
 // accumulated from the widths) and its transpose
-Xfer1D mk_xfer(DevBuf &m, const std::vector<double> &Df, const std::vector<double> &Dc, int coarsened)
+Xfer1D mk_xfer(DevBuf &m, const std::vector<double> &Df, const std::vector<double> &Dc, int coarsened, MgXferHost &host)
 {
     int nf = (int)Df.size(), nc = (int)Dc.size();
     std::vector<double> xf(nf), xc(nc);
@@ -705,6 +706,7 @@ Xfer1D mk_xfer(DevBuf &m, const std::vector<double> &Df, const std::vector<doubl
     t.I0 = m.upload(I0); t.I1 = m.upload(I1);
     t.w0d = m.upload(w0); t.w1d = m.upload(w1); t.w0f = m.upload(w0f); t.w1f = m.upload(w1f);
     t.rcnt = m.upload(rcnt); t.rf = m.upload(rf); t.rwd = m.upload(rw); t.rwf = m.upload(rwf);
+    host = MgXferHost{I0, I1, rf, w0, w1, rw};
     return t;
 }
 
@@ -725,6 +727,33 @@ static void set_cluster_from(turb_ctx *c)
             }
         }
     c->H32.cluster_from = c->H64.cluster_from = from;
+}
+
+// Where the V-cycle goes on as one launch: from the first level of at most
+// max_cells cells (turb_set_mg_tail; 0: never) that either fits the
+// shared-memory cluster kernel (k_mglow.cu) or leaves at most MG_TAIL_MAXLEV
+// levels for the single-block one.  By default max_cells is MG_LOW_CELLS32 /
+// MG_LOW_CELLS64 for the former, 4096 for the latter and beside the opt-in
+// global-memory cluster V-cycle.
+template <typename T>
+static int tail_level(const turb_ctx *c, const MgHier<T> &H, long long low_cells)
+{
+    const bool def = c->mg_tail_cells < 0;
+    const long long old_cells = def ? 4096 : c->mg_tail_cells;
+    if (def && H.cluster_from >= 0) low_cells = 4096;
+    if (!def) low_cells = c->mg_tail_cells;
+    for (int l = 0; l + 1 < H.nl; l++) {
+        const MgDevLevel &m = H.lev[l];
+        const long long n = (long long)m.nx * m.ny * m.nz;
+        if (n <= low_cells && mg_low_fits<T>(H, l)) return l;
+        if (n <= old_cells && H.nl - l <= MG_TAIL_MAXLEV) return l;
+    }
+    return -1;
+}
+static void place_tail(turb_ctx *c)
+{
+    c->H64.tail_from = tail_level<double>(c, c->H64, MG_LOW_CELLS64);
+    c->H32.tail_from = tail_level<float>(c, c->H32, MG_LOW_CELLS32);
 }
 
 // With TURB_KV_SWEEP_PAIRS, the finest FP32 level smooths two sweeps per
@@ -761,10 +790,11 @@ int build_mg(turb_ctx *c)
         m.nx = h.nx; m.ny = h.ny; m.nz = h.nz;
         m.cx = h.cx; m.cy = h.cy; m.cz = h.cz;
         m.pin = h.pin;
+        MgXferHost xh[3];
         if (l + 1 < nl) {
-            m.tx = mk_xfer(c->mem, h.D[0], L[l + 1].D[0], h.cx);
-            m.ty = mk_xfer(c->mem, h.D[1], L[l + 1].D[1], h.cy);
-            m.tz = mk_xfer(c->mem, h.D[2], L[l + 1].D[2], h.cz);
+            m.tx = mk_xfer(c->mem, h.D[0], L[l + 1].D[0], h.cx, xh[0]);
+            m.ty = mk_xfer(c->mem, h.D[1], L[l + 1].D[1], h.cy, xh[1]);
+            m.tz = mk_xfer(c->mem, h.D[2], L[l + 1].D[2], h.cz, xh[2]);
         }
         std::vector<double> rf[3];
         std::vector<float> Df[3], rff[3];
@@ -790,6 +820,12 @@ int build_mg(turb_ctx *c)
                     rrp[par * hx + q] = i + 1 < (int)rff[0].size() ? rff[0][i + 1] : 0.0f;
                 }
             m.dxpf = c->mem.upload(dxp); m.rlpf = c->mem.upload(rlp); m.rrpf = c->mem.upload(rrp);
+        }
+        if (l + 1 < nl) {
+            MgDevLevel next{};
+            next.nx = L[l + 1].nx; next.ny = L[l + 1].ny; next.nz = L[l + 1].nz;
+            m.lowf = c->mem.upload(mg_low_tables<float>(m, next, Df, rff, xh));
+            m.lowd = c->mem.upload(mg_low_tables<double>(m, next, h.D, rf, xh));
         }
         c->H64.lev[l] = m;
         // FP32 levels store x, b, invd colour-split where nx is even (not on
@@ -866,20 +902,12 @@ int build_mg(turb_ctx *c)
     c->H64.x[0] = c->pz;   // FP64 V-cycle writes z directly
     c->H64.b[0] = c->pr;   // and reads r directly
     c->sc = c->mem.alloc<PcgScal>(1);
-    // levels of at most 4096 cells finish the V-cycle in one block
-    // (turb_set_mg_tail; at 512x256x256 larger tails ran slower than a
-    // launch per half sweep, one SM having too little memory parallelism)
-    c->H64.tail_from = c->H32.tail_from = -1;
-    for (int l = 0; l + 1 < nl; l++) {
-        const MgDevLevel &m = c->H32.lev[l];
-        if ((long long)m.nx * m.ny * m.nz <= 4096 && nl - l <= MG_TAIL_MAXLEV) {
-            c->H64.tail_from = c->H32.tail_from = l;
-            break;
-        }
-    }
     c->H64.cluster_ctas = mg_cluster_ctas<double>();
     c->H32.cluster_ctas = mg_cluster_ctas<float>();
+    c->H64.low_ctas = mg_low_ctas<double>();
+    c->H32.low_ctas = mg_low_ctas<float>();
     set_cluster_from(c);
+    place_tail(c);
     set_tb(c);
     return c->mem.err == cudaSuccess ? TURB_OK : TURB_ERR_ALLOC;
 }
@@ -1328,6 +1356,7 @@ int turb_set_sweep_kernels(turb_ctx *c, int variants)
     c->H64.pdl = (variants & TURB_KV_PDL) ? 1 : 0;
     c->H32.pdl = c->H64.pdl;
     set_cluster_from(c);
+    place_tail(c);
     set_tb(c);
     return TURB_OK;
 }
@@ -1705,25 +1734,12 @@ int turb_Outflow_copy_data_into_2D_array(turb_ctx *c, char which, int ic)
     return check_launch(c);
 }
 
-// the first level with at most max_cells cells (and at most MG_TAIL_MAXLEV
-// levels from it to the coarsest) runs the rest of the V-cycle in one block
-static void set_tail(turb_ctx *c, long long max_cells)
-{
-    int from = -1;
-    for (int l = 0; l + 1 < c->H32.nl && max_cells > 0; l++) {
-        const MgDevLevel &m = c->H32.lev[l];
-        if ((long long)m.nx * m.ny * m.nz <= max_cells && c->H32.nl - l <= MG_TAIL_MAXLEV) { from = l; break; }
-    }
-    c->H32.tail_from = c->H64.tail_from = from;
-    for (int m = 0; m < 2; m++)
-        if (c->g_mg[m]) { cudaGraphExecDestroy(c->g_mg[m]); c->g_mg[m] = nullptr; }
-}
-
 int turb_set_mg_cluster(turb_ctx *c, long long max_cells)
 {
     if (!c || max_cells < 0) return TURB_ERR_ARG;
     c->mg_cluster_cells = max_cells;
     set_cluster_from(c);
+    place_tail(c);
     for (int m = 0; m < 2; m++)
         if (c->g_mg[m]) { cudaGraphExecDestroy(c->g_mg[m]); c->g_mg[m] = nullptr; }
     return TURB_OK;
@@ -1732,7 +1748,10 @@ int turb_set_mg_cluster(turb_ctx *c, long long max_cells)
 int turb_set_mg_tail(turb_ctx *c, long long max_cells)
 {
     if (!c || max_cells < 0) return TURB_ERR_ARG;
-    set_tail(c, max_cells);
+    c->mg_tail_cells = max_cells;
+    place_tail(c);
+    for (auto &g : c->g_mg)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     return TURB_OK;
 }
 

@@ -2,11 +2,24 @@
 #pragma once
 #include <cuda.h>
 
+#include <vector>
+
 #include "turb_internal.cuh"
 
 #define TURB_MG_MAXLEV 24
 #define MG_TAIL_MAXLEV 6   // levels a fused single-block V-cycle tail may hold
 #define MG_CLUSTER_MAXLEV 8   // levels a one-cluster V-cycle launch may hold
+// the shared-memory V-cycle of the lower levels (k_mglow.cu): levels it may
+// hold, cells of the level it starts from by default (FP32, FP64), cells up
+// to which a level is swept by one block, cells of a coarsest level whose
+// inverse is staged, and the most shared memory a block may take
+#define MG_LOW_MAXLEV 8
+#define MG_LOW_CELLS32 32768
+#define MG_LOW_CELLS64 32768
+#define MG_LOW_ONE32 4096
+#define MG_LOW_ONE64 512
+#define MG_LOW_INV 64
+#define MG_LOW_SMEM (220 * 1024)   // beside 4 KB of static shared memory
 
 // 1-D transfer tables between a level and the next coarser one along one
 // direction: prolongation weights per fine index (two coarse cells) and the
@@ -20,6 +33,12 @@ struct Xfer1D {
     const float *rwf;
 };
 
+// the host's copy of the tables of one direction
+struct MgXferHost {
+    std::vector<int> I0, I1, rf;
+    std::vector<double> w0, w1, rw;
+};
+
 struct MgDevLevel {
     int nx, ny, nz;
     int cx, cy, cz;                                   // coarsened into next level
@@ -30,6 +49,8 @@ struct MgDevLevel {
     // par * nx/2 + m is cell i = 2m + par: dx[i], 1/f of its left face
     // (rfx[i]) and of its right face (rfx[i+1])
     const float *dxpf = nullptr, *rlpf = nullptr, *rrpf = nullptr;
+    // the 1-D tables packed for k_vcycle_low (mg_low_tables), FP32 and FP64
+    const unsigned char *lowf = nullptr, *lowd = nullptr;
     double pin;
     // colour-split storage (x, b, invd; not r): with nx even, cell c of colour
     // (i+j+k)&1 lives at colour*(n/2) + c/2, so a red-black half sweep reads
@@ -58,9 +79,11 @@ struct MgHier {
     MgDevLevel lev[TURB_MG_MAXLEV];
     T *x[TURB_MG_MAXLEV], *b[TURB_MG_MAXLEV], *r[TURB_MG_MAXLEV], *invd[TURB_MG_MAXLEV];
     const double *coarse_inv;
-    // from this level on (-1: never) the V-cycle runs as one single-block
-    // kernel (k_vcycle_tail); it must leave at most MG_TAIL_MAXLEV levels
+    // from this level on (-1: never) the V-cycle runs as one launch: of one
+    // cluster with x in shared memory (k_vcycle_low) where mg_low_fits, else
+    // of a single block (k_vcycle_tail, at most MG_TAIL_MAXLEV levels)
     int tail_from = -1;
+    int low_ctas = 0;   // blocks of k_vcycle_low's cluster (mg_low_ctas; 0: not used)
     // 1: FP32 half sweeps after the first of a cycle march along k (k_rbgs4z)
     int marching = 0;
     // 1: the V-cycle's kernels use programmatic dependent launch
@@ -81,8 +104,57 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
 int mg_vcycle_launches(int nl, const int *pre, const int *post, int tail_from, int cluster_from = -1, int tb0 = 0);
 template <typename T>
 int mg_cluster_ctas();
+// the shared-memory V-cycle of level l and below (k_mglow.cu): mg_low launches
+// it and returns 1, or returns 0 where those levels do not fit
+template <typename T>
+int mg_low_ctas();
+// a level's 1-D tables packed for it: widths, 1/face distances and the
+// transfer tables to the next level, each along x, y, z
+template <typename T>
+std::vector<unsigned char> mg_low_tables(const MgDevLevel &F, const MgDevLevel &C, const std::vector<T> (&dd)[3],
+                                         const std::vector<T> (&rf)[3], const MgXferHost (&x)[3]);
+template <typename T>
+int mg_low_fits(const MgHier<T> &H, int l);
+template <typename T>
+int mg_low(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const int *post);
 template <typename T>
 double mg_vcycle_bytes(const MgHier<T> &H, int l, const int *pre, const int *post);
+
+// Linear prolongation of the eight coarse values around a cell (x fastest,
+// then y, z; w*0, w*1 the weights of the lower and upper one), summed in that
+// order with every rounding explicit, so that every kernel gives the same
+// bits (an absent neighbour has weight 0 and the value of its pair)
+__device__ __forceinline__ float mg_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mg_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mg_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mg_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <typename T>
+__device__ __forceinline__ T mg_prolong8(const T (&v)[8], T wx0, T wx1, T wy0, T wy1, T wz0, T wz1)
+{
+    T acc = 0;
+#pragma unroll
+    for (int e = 0; e < 8; e++)
+        acc = mg_fma(mg_mul(mg_mul(e & 4 ? wz1 : wz0, e & 2 ? wy1 : wy0), e & 1 ? wx1 : wx0), v[e], acc);
+    return acc;
+}
+// the 4 x 4 entries of one plane of a restriction (weights wz * wy[d] *
+// wx[f]) added to s, in that order; cx 0: x is not coarsened, entry f = 0 of
+// weight 1 alone
+template <typename T>
+__device__ __forceinline__ T mg_restrict16(T s, const T (&v)[4][4], T wz, const T *wy, const T *wx, bool cx)
+{
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const T w = mg_mul(wz, wy[d]);
+        if (cx) {
+#pragma unroll
+            for (int f = 0; f < 4; f++) s = mg_fma(mg_mul(w, wx[f]), v[d][f], s);
+        } else {
+            s = mg_fma(w, v[d][0], s);
+        }
+    }
+    return s;
+}
 
 // FP64 CG vector kernels on the compact level-0 layout (k_pcg.cu)
 struct PcgScal {
