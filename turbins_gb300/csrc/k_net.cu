@@ -575,15 +575,15 @@ int loss(TurbNet *n, cudaStream_t s, const MgDevLevel &L0, const double *invd, c
     long long V = n->V[0];
     int np = pcg_stencil_parts(L0);
     k_loss_in<<<nblk(V), 256, 0, s>>>(V, n->hout, invd, snap, n->x64, n->r64);
-    pcg_resid(s, L0, n->r64, n->x64, n->rr, n->part);
+    pcg_resid(s, L0, n->r64, n->x64, n->rr, n->part, nullptr, nullptr);
     pcg_reduce(s, n->part, 1, n->sc + 2, np);
     if (want_grad) {
-        pcg_apply(s, L0, n->rr, n->q64, n->part);
+        pcg_apply(s, L0, n->rr, n->q64, n->part, nullptr, nullptr);
         k_loss_grad<<<nblk(V), 256, 0, s>>>(V, n->q64, invd, n->gout);
         if (n->wr != 1.0) k_scale_f<<<nblk(V), 256, 0, s>>>(V, (float)n->wr, n->gout);
     }
     k_energy_in<<<nblk(V), 256, 0, s>>>(V, n->hout, snap + 3 * V, invd, n->x64);
-    pcg_apply(s, L0, n->x64, n->q64, n->part);
+    pcg_apply(s, L0, n->x64, n->q64, n->part, nullptr, nullptr);
     pcg_reduce(s, n->part, 1, n->sc + 3, np);
     if (want_grad && n->we != 0.0) k_grad_add<<<nblk(V), 256, 0, s>>>(V, n->we, e0, n->q64, invd, n->gout);
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
@@ -652,7 +652,7 @@ int net_snapshot_finish(TurbSnaps *sn, cudaStream_t st, const MgDevLevel &L0, co
     float *t = sn->data + (long long)k * SNAP_CH * V + 3 * V;
     k_target<<<nblk(V), 256, 0, st>>>(V, p, sn->base, invd, sn->sc, t);
     k_t64<<<nblk(V), 256, 0, st>>>(V, t, invd, sn->x64);
-    pcg_apply(st, L0, sn->x64, sn->q64, sn->part);
+    pcg_apply(st, L0, sn->x64, sn->q64, sn->part, nullptr, nullptr);
     pcg_reduce(st, sn->part, 1, sn->e0 + k, pcg_stencil_parts(L0));
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
 }

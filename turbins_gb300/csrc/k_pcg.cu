@@ -2,8 +2,11 @@
 // (volume-weighted system on the compact physical-cell layout).  Dot products
 // reduce by warp shuffles into a fixed set of per-block partials that one
 // block sums in a fixed order, so results are run-to-run deterministic.
+#include <algorithm>
+
 #include "turb_internal.cuh"
 #include "turb_mg.cuh"
+#include "turb_sum.cuh"
 
 namespace {
 
@@ -29,6 +32,63 @@ __device__ __forceinline__ void block_store(double v, double *dst)
         if (lt == 0) *dst = r;
     }
     __syncthreads();
+}
+
+// Sums of the blocks' partials by the block that finishes last: it adds them
+// as one block of 1024 threads would (thread t takes partials t, t + 1024, ..,
+// then a shuffle tree per warp and one over the warps), whatever its own
+// size, so the sums do not depend on which block it is.  Partials
+// [nblk, nper) are those of blocks that would have no elements: zeros, which
+// adding leaves out.  nval values, value v's partials at part + v * stride.
+// A launch for the sums cost 6 us at every size; this costs one round trip.
+__device__ __forceinline__ bool last_block(unsigned *count, unsigned nblk)
+{
+    __shared__ bool last;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        __threadfence();
+        last = atomicAdd(count, 1u) == nblk - 1;
+        if (last) {
+            *count = 0u;   // ready for the next launch
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last;
+}
+
+template <int NVAL>
+__device__ __forceinline__ void sum_parts(const double *part, long long stride, int nblk, double *dst)
+{
+    __shared__ double sm[NVAL][32];
+    const int lt = threadIdx.y * blockDim.x + threadIdx.x, lane = lt & 31, nw = (blockDim.x * blockDim.y) >> 5;
+    for (int w = lt >> 5; w < 32; w += nw) {
+#pragma unroll
+        for (int v = 0; v < NVAL; v++) {
+            double acc = 0.0;
+            for (int t = w * 32 + lane; t < nblk; t += 1024) acc += __ldcg(part + v * stride + t);
+            acc = warp_sum(acc);
+            if (lane == 0) sm[v][w] = acc;
+        }
+    }
+    __syncthreads();
+    if (lt < 32) {
+#pragma unroll
+        for (int v = 0; v < NVAL; v++) {
+            const double r = warp_sum(sm[v][lt]);
+            if (lt == 0) dst[v] = r;
+        }
+    }
+}
+
+// block_store of NV values of a 256-thread block to dst + n * stride
+template <int NV>
+__device__ __forceinline__ void block_store256(const double (&v)[NV], double *dst, long long stride)
+{
+    double s[NV];
+    block_sum256<NV>(v, s);
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+#pragma unroll
+        for (int n = 0; n < NV; n++) dst[n * stride] = s[n];
 }
 
 constexpr int KC = 4;   // planes per thread in the 3-D stencil kernels
@@ -122,7 +182,7 @@ __global__ void k_scatter(Dims d, MgDevLevel L, const double *__restrict__ x, do
 
 // r = W b - S x with partial |r|^2 per block (3-D launch, KC planes per thread)
 __global__ void k_resid(MgDevLevel L, const double *__restrict__ bw, const double *__restrict__ x,
-                        double *__restrict__ r, double *__restrict__ part)
+                        double *__restrict__ r, double *__restrict__ part, double *dst, unsigned *count)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     __shared__ SPlane sp[KC];
@@ -140,12 +200,17 @@ __global__ void k_resid(MgDevLevel L, const double *__restrict__ bw, const doubl
             acc += v * v;
         }
     }
-    block_store(acc, part + blk3());
+    block_store256<1>({acc}, part + blk3(), 0);
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    if (count && last_block(count, nb)) sum_parts<1>(part, 0, (int)nb, dst);
 }
 
-// q = S p with partial p.q per block
-__global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part)
+// q = S p with partial p.q per block, then alpha = rz / p.q
+__global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part,
+                        PcgScal *sc, unsigned *count)
 {
+    pdl_trigger();
+    pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     __shared__ SPlane sp[KC];
     s_planes(L, sp);
@@ -162,28 +227,44 @@ __global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__re
             acc += p[c] * v;
         }
     }
-    block_store(acc, part + blk3());
+    block_store256<1>({acc}, part + blk3(), 0);
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    if (count && last_block(count, nb)) {
+        sum_parts<1>(part, 0, (int)nb, &sc->pq);
+        if (threadIdx.x == 0 && threadIdx.y == 0) {
+            sc->alpha = sc->pq != 0.0 ? sc->rz / sc->pq : 0.0;
+            sc->rz_old = sc->rz;
+        }
+    }
 }
 
-__global__ void k_dot(long long n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ part)
+__global__ void k_dot(long long n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ part,
+                      double *dst, unsigned *count)
 {
     double acc = 0.0;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
         acc += a[c] * b[c];
-    block_store(acc, part + blockIdx.x);
+    block_store256<1>({acc}, part + blockIdx.x, 0);
+    if (last_block(count, gridDim.x)) sum_parts<1>(part, 0, gridDim.x, dst);
 }
 
+// rz = r.z and zr_old = z.r_old, then beta (0 on a restart)
 __global__ void k_dot2(long long n, const double *__restrict__ r, const double *__restrict__ z,
-                       const double *__restrict__ ro, double *__restrict__ part)
+                       const double *__restrict__ ro, double *__restrict__ part, PcgScal *sc, int restart, unsigned *count)
 {
+    pdl_trigger();
+    pdl_wait();
     double a = 0.0, b = 0.0;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
         double zc = z[c];
         a += r[c] * zc;
         b += ro[c] * zc;
     }
-    block_store(a, part + blockIdx.x);
-    block_store(b, part + NP + blockIdx.x);
+    block_store256<2>({a, b}, part + blockIdx.x, NP);
+    if (last_block(count, gridDim.x)) {
+        sum_parts<2>(part, NP, gridDim.x, &sc->rz);   // rz and, next to it, zr_old
+        if (threadIdx.x == 0 && !restart) sc->beta = sc->rz_old != 0.0 ? (sc->rz - sc->zr_old) / sc->rz_old : 0.0;
+    }
 }
 
 __global__ void k_reduce(const double *__restrict__ part, int nvals, int nper, double *__restrict__ dst)
@@ -195,28 +276,21 @@ __global__ void k_reduce(const double *__restrict__ part, int nvals, int nper, d
     }
 }
 
-__global__ void k_scalars(PcgScal *sc, int what)
-{
-    if (threadIdx.x != 0) return;
-    if (what == 0) {
-        sc->beta = sc->rz_old != 0.0 ? (sc->rz - sc->zr_old) / sc->rz_old : 0.0;
-    } else {
-        sc->alpha = sc->pq != 0.0 ? sc->rz / sc->pq : 0.0;
-        sc->rz_old = sc->rz;
-    }
-}
-
 __global__ void k_pupdate(long long n, const double *__restrict__ z, double *__restrict__ p, const PcgScal *sc, int first)
 {
+    pdl_trigger();
+    pdl_wait();
     double beta = first ? 0.0 : sc->beta;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
         p[c] = first ? z[c] : z[c] + beta * p[c];
 }
 
 __global__ void k_xrupdate(long long n, double *__restrict__ x, double *__restrict__ r, double *__restrict__ ro,
-                           const double *__restrict__ p, const double *__restrict__ q, const PcgScal *sc,
-                           double *__restrict__ part)
+                           const double *__restrict__ p, const double *__restrict__ q, PcgScal *sc,
+                           double *__restrict__ part, double *host_rr, unsigned *count)
 {
+    pdl_trigger();
+    pdl_wait();
     double alpha = sc->alpha, acc = 0.0;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
         double rc = r[c];
@@ -226,7 +300,11 @@ __global__ void k_xrupdate(long long n, double *__restrict__ x, double *__restri
         r[c] = rc;
         acc += rc * rc;
     }
-    block_store(acc, part + blockIdx.x);
+    block_store256<1>({acc}, part + blockIdx.x, 0);
+    if (last_block(count, gridDim.x)) {
+        sum_parts<1>(part, 0, gridDim.x, &sc->rr);
+        if (threadIdx.x == 0) *host_rr = sc->rr;   // page-locked: the host reads it after its wait
+    }
 }
 
 __global__ void k_lincomb(long long n, double a, const double *__restrict__ x, double b, const double *__restrict__ y,
@@ -288,8 +366,9 @@ __global__ void __launch_bounds__(BS) k_gal_dots(long long n, GalDirs dd, const 
 #pragma unroll
     for (int a = 0; a < GAL_MAX; a++) {
 #pragma unroll
-        for (int b = 0; b < GAL_MAX; b++) block_store(G[a][b], part + (long long)(a * GAL_MAX + b) * GAL_NP + blockIdx.x);
-        block_store(gv[a], part + (long long)(GAL_MAX * GAL_MAX + a) * GAL_NP + blockIdx.x);
+        for (int b = 0; b < GAL_MAX; b++)
+            block_store256<1>({G[a][b]}, part + (long long)(a * GAL_MAX + b) * GAL_NP + blockIdx.x, 0);
+        block_store256<1>({gv[a]}, part + (long long)(GAL_MAX * GAL_MAX + a) * GAL_NP + blockIdx.x, 0);
     }
 }
 
@@ -357,6 +436,8 @@ long long ncell(const MgDevLevel &L) { return (long long)L.nx * L.ny * L.nz; }
 }  // namespace
 
 
+static unsigned nblk(long long n);
+
 void pcg_gal_dots(cudaStream_t s, long long n, const GalDirs &dd, const double *x0, const double *r1,
                   const double *bw, double *part, double *dst)
 {
@@ -366,10 +447,28 @@ void pcg_gal_dots(cudaStream_t s, long long n, const GalDirs &dd, const double *
 
 void pcg_gal_update(cudaStream_t s, long long n, const GalDirs &dd, const GalCoef &al, const double *x0, double *x)
 {
-    k_gal_update<<<NP, BS, 0, s>>>(n, dd, al, x0, x);
+    k_gal_update<<<nblk(n), BS, 0, s>>>(n, dd, al, x0, x);
 }
 
 int pcg_nparts() { return NP; }
+// blocks of the grid-stride kernels: NP, or as many as have elements
+static unsigned nblk(long long n) { return (unsigned)std::min<long long>(NP, (n + BS - 1) / BS); }
+
+// a launch with the programmatic stream serialisation attribute
+template <typename... P, typename... A>
+static void launch_pdl(void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
 
 static dim3 g3k(const MgDevLevel &L)
 {
@@ -398,24 +497,27 @@ void pcg_scatter(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const doub
     k_scatter<<<dim3((d.NX + 31) / 32, (d.NY + 7) / 8, d.NZ), dim3(32, 8), 0, s>>>(d, L0, x, phi_da);
 }
 
-void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part)
+void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part,
+               double *dst, unsigned *count)
 {
-    k_resid<<<g3k(L0), dim3(32, 8), 0, s>>>(L0, bw, x, r, part);
+    k_resid<<<g3k(L0), dim3(32, 8), 0, s>>>(L0, bw, x, r, part, dst, count);
 }
 
-void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part)
+void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc,
+               unsigned *count)
 {
-    k_apply<<<g3k(L0), dim3(32, 8), 0, s>>>(L0, p, q, part);
+    launch_pdl(k_apply, g3k(L0), dim3(32, 8), s, L0, p, q, part, sc, count);
 }
 
-void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part)
+void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part, double *dst, unsigned *count)
 {
-    k_dot<<<NP, BS, 0, s>>>(n, a, b, part);
+    k_dot<<<nblk(n), BS, 0, s>>>(n, a, b, part, dst, count);
 }
 
-void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part)
+void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part,
+              PcgScal *sc, int restart, unsigned *count)
 {
-    k_dot2<<<NP, BS, 0, s>>>(n, r, z, rold, part);
+    launch_pdl(k_dot2, dim3(nblk(n)), dim3(BS), s, n, r, z, rold, part, sc, restart, count);
 }
 
 void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper)
@@ -425,21 +527,19 @@ void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int 
 
 void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first)
 {
-    k_pupdate<<<NP, BS, 0, s>>>(n, z, p, sc, first);
+    launch_pdl(k_pupdate, dim3(nblk(n)), dim3(BS), s, n, z, p, sc, first);
 }
 
 void pcg_xrupdate(cudaStream_t s, long long n, double *x, double *r, double *rold, const double *p,
-                  const double *q, const PcgScal *sc, double *part)
+                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count)
 {
-    k_xrupdate<<<NP, BS, 0, s>>>(n, x, r, rold, p, q, sc, part);
+    launch_pdl(k_xrupdate, dim3(nblk(n)), dim3(BS), s, n, x, r, rold, p, q, sc, part, host_rr, count);
 }
 
-void pcg_scalars(cudaStream_t s, PcgScal *sc, int what) { k_scalars<<<1, 32, 0, s>>>(sc, what); }
-
-void pcg_to_float(cudaStream_t s, long long n, const double *a, float *b) { k_f2<<<NP, BS, 0, s>>>(n, a, b); }
-void pcg_to_double(cudaStream_t s, long long n, const float *a, double *b) { k_d2<<<NP, BS, 0, s>>>(n, a, b); }
-void pcg_copy(cudaStream_t s, long long n, const double *a, double *b) { k_copy<<<NP, BS, 0, s>>>(n, a, b); }
+void pcg_to_float(cudaStream_t s, long long n, const double *a, float *b) { k_f2<<<nblk(n), BS, 0, s>>>(n, a, b); }
+void pcg_to_double(cudaStream_t s, long long n, const float *a, double *b) { k_d2<<<nblk(n), BS, 0, s>>>(n, a, b); }
+void pcg_copy(cudaStream_t s, long long n, const double *a, double *b) { k_copy<<<nblk(n), BS, 0, s>>>(n, a, b); }
 void pcg_lincomb(cudaStream_t s, long long n, double a, const double *x, double b, const double *y, double *out)
 {
-    k_lincomb<<<NP, BS, 0, s>>>(n, a, x, b, y, out);
+    k_lincomb<<<nblk(n), BS, 0, s>>>(n, a, x, b, y, out);
 }

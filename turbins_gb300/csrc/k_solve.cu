@@ -11,6 +11,7 @@
 // solution); the squared residual norm is reduced in the sweep itself.
 #include "turb_internal.cuh"
 #include "turb_kernels.cuh"
+#include "turb_sum.cuh"
 
 namespace {
 
@@ -132,8 +133,9 @@ __global__ void k_helm_jacobi(Dims d, HelmTab h, const uint8_t *__restrict__ st,
             r2 = fma(r, r, r2);
         }
     }
-    double bs = block_sum(r2);
-    if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs;
+    double bs[1];
+    block_sum256<1>({r2}, bs);
+    if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs[0];
 }
 
 __global__ void k_ib_jacobi(IbDev ib, const double *__restrict__ b, const double *__restrict__ x,
@@ -150,8 +152,9 @@ __global__ void k_ib_jacobi(IbDev ib, const double *__restrict__ b, const double
         xn[im] = x[im] + r / ib.diag[t];
         r2 = r * r;
     }
-    double bs = block_sum(r2);
-    if (threadIdx.x == 0) part[blockIdx.x] = bs;
+    double bs[1];
+    block_sum256<1>({r2}, bs);
+    if (threadIdx.x == 0) part[blockIdx.x] = bs[0];
 }
 
 __global__ void k_sum_final(long long n, const double *__restrict__ part, double *__restrict__ out)
@@ -214,8 +217,9 @@ __global__ void k_helm_resid64(Dims d, HelmTab h, const uint8_t *__restrict__ st
             r2 = fma(r, r, r2);
         }
     }
-    double bs = block_sum(r2);
-    if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs;
+    double bs[1];
+    block_sum256<1>({r2}, bs);
+    if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs[0];
 }
 
 __global__ void k_ib_resid64(IbDev ib, const double *__restrict__ b, const double *__restrict__ x,
@@ -232,8 +236,9 @@ __global__ void k_ib_resid64(IbDev ib, const double *__restrict__ b, const doubl
         rf[im] = (float)r;
         r2 = r * r;
     }
-    double bs = block_sum(r2);
-    if (threadIdx.x == 0) part[blockIdx.x] = bs;
+    double bs[1];
+    block_sum256<1>({r2}, bs);
+    if (threadIdx.x == 0) part[blockIdx.x] = bs[0];
     pdl_wait();   // as in k_ib_jac32: end after the stencil residual
 }
 
@@ -498,8 +503,9 @@ __global__ void k_norm2(long long n, const double *__restrict__ x, double *__res
     double v = 0.0;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
         v += x[p] * x[p];
-    double s = block_sum(v);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    double s[1];
+    block_sum256<1>({v}, s);
+    if (threadIdx.x == 0) part[blockIdx.x] = s[0];
 }
 
 }  // namespace

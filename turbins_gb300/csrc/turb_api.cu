@@ -140,6 +140,7 @@ struct turb_ctx {
     MgHier<float> H32;
     double *px, *pbw, *pr, *pz, *pp, *pq, *pro;
     PcgScal *sc;
+    unsigned *count = nullptr;   // blocks done of a launch that ends in a sum; zero between launches
     double *part, *dscal;
     double *hscal = nullptr;   // pinned host scalars
     long long nparts = 0;
@@ -902,6 +903,7 @@ int build_mg(turb_ctx *c)
     c->H64.x[0] = c->pz;   // FP64 V-cycle writes z directly
     c->H64.b[0] = c->pr;   // and reads r directly
     c->sc = c->mem.alloc<PcgScal>(1);
+    c->count = c->mem.alloc<unsigned>(4);
     c->H64.cluster_ctas = mg_cluster_ctas<double>();
     c->H32.cluster_ctas = mg_cluster_ctas<float>();
     c->H64.low_ctas = mg_low_ctas<double>();
@@ -2602,8 +2604,7 @@ static int galerkin_guess(turb_ctx *c, int st, int with_net, double *nr_out, dou
     }
     *de_out = de;
     pcg_gal_update(s, n0, dd, co, c->px, c->pp);
-    pcg_resid(s, L0, c->pbw, c->pp, c->pro, c->part);
-    pcg_reduce(s, c->part, 1, c->dscal, pcg_stencil_parts(L0));
+    pcg_resid(s, L0, c->pbw, c->pp, c->pro, c->part, c->dscal, c->count);
     TURB_CHECK(cudaMemcpyAsync(c->hscal, c->dscal, sizeof(double), cudaMemcpyDeviceToHost, s));
     TURB_CHECK(cudaStreamSynchronize(s));
     c->launches += 3;
@@ -2622,12 +2623,9 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
     PcgScal *sc = c->sc;
     double *dsc = reinterpret_cast<double *>(sc);   // bb rr rz zr_old rz_old pq alpha beta
     pcg_gather(s, d, L0, c->fld[TURB_F_PHI], c->fld[TURB_F_PB], c->px, c->pbw);
-    pcg_dot(s, n0, c->pbw, c->pbw, c->part);
-    pcg_reduce(s, c->part, 1, dsc + 0);
-    int nsp = pcg_stencil_parts(L0);
-    pcg_resid(s, L0, c->pbw, c->px, c->pr, c->part);
-    pcg_reduce(s, c->part, 1, dsc + 1, nsp);
-    c->launches += 5;
+    pcg_dot(s, n0, c->pbw, c->pbw, c->part, dsc + 0, c->count);
+    pcg_resid(s, L0, c->pbw, c->px, c->pr, c->part, dsc + 1, c->count);
+    c->launches += 3;
     TURB_CHECK(cudaMemcpyAsync(c->hscal, dsc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     TURB_CHECK(cudaStreamSynchronize(s));
     double nb = std::sqrt(c->hscal[0]), nr = std::sqrt(c->hscal[1]);
@@ -2663,9 +2661,8 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             ok = 1;
         }
         if (ok) {
-            pcg_resid(s, L0, c->pbw, c->pz, c->pq, c->part);
-            pcg_reduce(s, c->part, 1, dsc + 1, nsp);
-            c->launches += 2;
+            pcg_resid(s, L0, c->pbw, c->pz, c->pq, c->part, dsc + 1, c->count);
+            c->launches += 1;
             TURB_CHECK(cudaMemcpyAsync(c->hscal + 2, dsc + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
             TURB_CHECK(cudaStreamSynchronize(s));
             nrc = std::sqrt(c->hscal[2]);
@@ -2710,9 +2707,8 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
     for (;;) {
         if (!std::isfinite(nr)) { status = TURB_ERR_NAN; break; }
         if (nr <= tol || it >= c->prm.p_maxit) {
-            pcg_resid(s, L0, c->pbw, c->px, c->pr, c->part);
-            pcg_reduce(s, c->part, 1, dsc + 1, nsp);
-            c->launches += 2;
+            pcg_resid(s, L0, c->pbw, c->px, c->pr, c->part, dsc + 1, c->count);
+            c->launches += 1;
             TURB_CHECK(cudaMemcpyAsync(c->hscal + 1, dsc + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
             TURB_CHECK(cudaStreamSynchronize(s));
             nr = std::sqrt(c->hscal[1]);
@@ -2755,17 +2751,12 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             }
         };
         auto cgstep = [&](int rs) {
-            pcg_dot2(s, n0, c->pr, c->pz, c->pro, c->part);
-            pcg_reduce(s, c->part, 2, dsc + 2);   // rz and z.r_old
-            if (!rs) pcg_scalars(s, sc, 0);
+            pcg_dot2(s, n0, c->pr, c->pz, c->pro, c->part, sc, rs, c->count);   // r.z, z.r_old, beta
             pcg_pupdate(s, n0, c->pz, c->pp, sc, rs);
-            pcg_apply(s, L0, c->pp, c->pq, c->part);
-            pcg_reduce(s, c->part, 1, dsc + 5, nsp);
-            pcg_scalars(s, sc, 1);
-            pcg_xrupdate(s, n0, c->px, c->pr, c->pro, c->pp, c->pq, sc, c->part);
-            pcg_reduce(s, c->part, 1, dsc + 1);
+            pcg_apply(s, L0, c->pp, c->pq, c->part, sc, c->count);               // q = S p, p.q, alpha
+            pcg_xrupdate(s, n0, c->px, c->pr, c->pro, c->pp, c->pq, sc, c->part, c->hscal + 1, c->count);
         };
-        int nmg = vl + (pm ? 2 : 0), ncg = 8 + (restart ? 0 : 1);
+        int nmg = vl + (pm ? 2 : 0), ncg = 4;
         int ph = prof_begin(c, TURB_PROF_MG);
         if (c->use_graphs) {
             if (!c->g_mg[pm]) { int rc = capture(c, &c->g_mg[pm], vcycle); if (rc) return rc; }
@@ -2789,8 +2780,7 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
         }
         prof_end(c, ph, ncg, (restart ? 112.0 : 120.0) * n0);
         c->launches += nmg + ncg;
-        TURB_CHECK(cudaMemcpyAsync(c->hscal + 1, dsc + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
-        TURB_CHECK(cudaStreamSynchronize(s));
+        TURB_CHECK(cudaStreamSynchronize(s));   // |r|^2 is in hscal[1]
         nr = std::sqrt(c->hscal[1]);
         restart = 0;
         it++;

@@ -163,16 +163,21 @@ struct PcgScal {
 void pcg_gather(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const double *phi_da, const double *pb_da,
                 double *x, double *bw);
 void pcg_scatter(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const double *x, double *phi_da);
-void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part);
-void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part);
-void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part);
-void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part);
-void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper = 0);
+// The sums of these end in the launch itself (the last block adds the
+// partials; count: a zero word the launch leaves zero): |r|^2, p.q and alpha,
+// a.b, r.z, z.r_old and beta, |r|^2 (also to the page-locked *host_rr).  With
+// count null, pcg_resid and pcg_apply leave the partials for pcg_reduce
+void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part,
+               double *dst, unsigned *count);
+void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc, unsigned *count);
+void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part, double *dst, unsigned *count);
+void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part,
+              PcgScal *sc, int restart, unsigned *count);
 int pcg_stencil_parts(const MgDevLevel &L);
+void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper = 0);
 void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first);
 void pcg_xrupdate(cudaStream_t s, long long n, double *x, double *r, double *rold, const double *p,
-                  const double *q, const PcgScal *sc, double *part);
-void pcg_scalars(cudaStream_t s, PcgScal *sc, int what);
+                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count);
 void pcg_to_float(cudaStream_t s, long long n, const double *a, float *b);
 void pcg_to_double(cudaStream_t s, long long n, const float *a, double *b);
 // the same into / out of a level's storage order (colour-split or not)
