@@ -12,6 +12,7 @@ namespace {
 
 constexpr int NP = 4096;   // blocks of the grid-stride reductions
 constexpr int BS = 256;
+constexpr int VB = 4;      // blocks of a reduction that a block of its launch stands for
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -59,22 +60,34 @@ __device__ __forceinline__ bool last_block(unsigned *count, unsigned nblk)
 template <int NVAL>
 __device__ __forceinline__ void sum_parts(const double *part, long long stride, int nblk, double *dst)
 {
-    __shared__ double sm[NVAL][32];
-    const int lt = threadIdx.y * blockDim.x + threadIdx.x, lane = lt & 31, nw = (blockDim.x * blockDim.y) >> 5;
-    for (int w = lt >> 5; w < 32; w += nw) {
+    __shared__ double sm[NVAL][1024];
+    const int lt = threadIdx.y * blockDim.x + threadIdx.x, lane = lt & 31;
+    // the 1024 threads' sums, four per thread of this block of 256
 #pragma unroll
-        for (int v = 0; v < NVAL; v++) {
+    for (int v = 0; v < NVAL; v++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
             double acc = 0.0;
-            for (int t = w * 32 + lane; t < nblk; t += 1024) acc += __ldcg(part + v * stride + t);
-            acc = warp_sum(acc);
-            if (lane == 0) sm[v][w] = acc;
+            for (int t = q * 256 + lt; t < nblk; t += 1024) acc += __ldcg(part + v * stride + t);
+            sm[v][q * 256 + lt] = acc;
+        }
+    __syncthreads();
+    // the trees of the 32 warps, each pair added once: warp w's entries stay
+    // at w * 32 .. while their number halves (distances 16, 8, 4, 2, 1)
+    if (lt < 128) {
+        for (int d = 16; d >= 1; d >>= 1) {
+            for (int v = 0; v < NVAL; v++)
+                for (int t = lt; t < 32 * d; t += 128) {
+                    const int at = (t / d) * 32 + (t & (d - 1));
+                    sm[v][at] += sm[v][at + d];
+                }
+            asm volatile("bar.sync 2, 128;" ::: "memory");
         }
     }
-    __syncthreads();
     if (lt < 32) {
 #pragma unroll
         for (int v = 0; v < NVAL; v++) {
-            const double r = warp_sum(sm[v][lt]);
+            const double r = warp_sum(sm[v][lane * 32]);
             if (lt == 0) dst[v] = r;
         }
     }
@@ -138,28 +151,66 @@ __device__ __forceinline__ SPlane s_plane(const MgDevLevel &L, int k)
     return r;
 }
 
-// the KC planes of a block, formed once by its first threads
-__device__ __forceinline__ void s_planes(const MgDevLevel &L, SPlane *sp)
+// the n planes of a block from k0, formed once by its first threads
+__device__ __forceinline__ void s_planes(const MgDevLevel &L, SPlane *sp, int k0, int n)
 {
-    int t = threadIdx.y * blockDim.x + threadIdx.x, k = blockIdx.z * KC + t;
-    if (t < KC && k < L.nz) sp[t] = s_plane(L, k);
+    int t = threadIdx.y * blockDim.x + threadIdx.x, k = k0 + t;
+    if (t < n && k < L.nz) sp[t] = s_plane(L, k);
     __syncthreads();
 }
 
-__device__ __forceinline__ double s_apply(const MgDevLevel &L, const SCol &a, const SPlane &z,
-                                          const double *__restrict__ x, long long c, Cell q)
+// f(group, c, x_c, (S x)_c) over the G groups of KC planes of the thread's
+// column.  A block of G groups forms the column's coefficients (eight FP64
+// operations) once for 4 G cells and reads the cells above and below as the
+// march reaches them; each group's sum is stored apart, so the partials are
+// those of blocks of one group.
+template <int G, typename F>
+__device__ __forceinline__ void s_march(const MgDevLevel &L, const double *__restrict__ x, F f)
 {
-    long long nx = L.nx, nxy = (long long)L.nx * L.ny;
-    double xc = x[c];
-    double xw = x[c - (q.i > 0 ? 1 : 0)], xe = x[c + (q.i < L.nx - 1 ? 1 : 0)];
-    double xs = x[c - (q.j > 0 ? nx : 0)], xn = x[c + (q.j < L.ny - 1 ? nx : 0)];
-    double xb = x[c - (q.k > 0 ? nxy : 0)], xf = x[c + (q.k < L.nz - 1 ? nxy : 0)];
-    double t = fma(a.axw, xw, fma(a.axe, xe, fma(a.ays, xs, a.ayn * xn)));
-    double xy = fma(a.cxy, xc, -t);
-    double sz = fma(z.zs, xc, -fma(z.zb, xb, z.zf * xf));
-    double v = fma(z.dz, xy, a.wz * sz);
-    if (q.i == L.nx - 1 && q.j == L.ny - 1 && q.k == L.nz - 1) v = fma(L.pin, xc, v);
-    return v;
+    __shared__ SPlane sp[KC * G];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k0 = blockIdx.z * KC * G;
+    s_planes(L, sp, k0, KC * G);
+    if (i >= L.nx || j >= L.ny) return;
+    const SCol a = s_col(L, i, j);
+    const long long nx = L.nx, nxy = nx * L.ny;
+    const long long ow = i > 0 ? 1 : 0, oe = i < L.nx - 1 ? 1 : 0, os = j > 0 ? nx : 0, on = j < L.ny - 1 ? nx : 0;
+    const bool corner = i == L.nx - 1 && j == L.ny - 1;
+    long long c = ((long long)k0 * L.ny + j) * nx + i;
+    double xc = x[c], xb = k0 > 0 ? x[c - nxy] : xc;
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+#pragma unroll
+        for (int kk = 0; kk < KC; kk++) {
+            const int k = k0 + g * KC + kk;
+            if (k >= L.nz) return;
+            const SPlane z = sp[g * KC + kk];
+            const double xf = k < L.nz - 1 ? x[c + nxy] : xc;
+            const double xw = x[c - ow], xe = x[c + oe], xs = x[c - os], xn = x[c + on];
+            double t = fma(a.axw, xw, fma(a.axe, xe, fma(a.ays, xs, a.ayn * xn)));
+            double xy = fma(a.cxy, xc, -t);
+            double sz = fma(z.zs, xc, -fma(z.zb, xb, z.zf * xf));
+            double v = fma(z.dz, xy, a.wz * sz);
+            if (corner && k == L.nz - 1) v = fma(L.pin, xc, v);
+            f(g, c, xc, v);
+            xb = xc;
+            xc = xf;
+            c += nxy;
+        }
+    }
+}
+// the G groups' sums to the partials of blocks of one group
+template <int G>
+__device__ __forceinline__ void store_groups(const MgDevLevel &L, const double (&acc)[G], double *part)
+{
+    double s[G];
+    block_sum256<G>(acc, s);
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int b = blockIdx.z * G + g;
+            if (b * KC < L.nz) part[((long long)b * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = s[g];
+        }
 }
 
 __global__ void k_gather(Dims d, MgDevLevel L, const double *__restrict__ phi, const double *__restrict__ pb,
@@ -180,57 +231,36 @@ __global__ void k_scatter(Dims d, MgDevLevel L, const double *__restrict__ x, do
     phi[p] = (i < L.nx && j < L.ny && k < L.nz) ? x[((long long)k * L.ny + j) * L.nx + i] : 0.0;
 }
 
-// r = W b - S x with partial |r|^2 per block (3-D launch, KC planes per thread)
+// r = W b - S x with partial |r|^2 per group of planes
+template <int G>
 __global__ void k_resid(MgDevLevel L, const double *__restrict__ bw, const double *__restrict__ x,
-                        double *__restrict__ r, double *__restrict__ part, double *dst, unsigned *count)
+                        double *__restrict__ r, double *__restrict__ part, int nparts, double *dst, unsigned *count)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    __shared__ SPlane sp[KC];
-    s_planes(L, sp);
-    double acc = 0.0;
-    if (i < L.nx && j < L.ny) {
-        const SCol a = s_col(L, i, j);
-        for (int kk = 0; kk < KC; kk++) {
-            int k = blockIdx.z * KC + kk;
-            if (k >= L.nz) break;
-            long long c = ((long long)k * L.ny + j) * L.nx + i;
-            Cell q{i, j, k};
-            double v = bw[c] - s_apply(L, a, sp[kk], x, c, q);
-            r[c] = v;
-            acc += v * v;
-        }
-    }
-    block_store256<1>({acc}, part + blk3(), 0);
-    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
-    if (count && last_block(count, nb)) sum_parts<1>(part, 0, (int)nb, dst);
+    double acc[G] = {};
+    s_march<G>(L, x, [&](int g, long long c, double, double sx) {
+        double v = bw[c] - sx;
+        r[c] = v;
+        acc[g] += v * v;
+    });
+    store_groups<G>(L, acc, part);
+    if (count && last_block(count, gridDim.x * gridDim.y * gridDim.z)) sum_parts<1>(part, 0, nparts, dst);
 }
 
-// q = S p with partial p.q per block, then alpha = rz / p.q
+// q = S p with partial p.q per group of planes, then alpha = rz / p.q
+template <int G>
 __global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part,
-                        PcgScal *sc, unsigned *count)
+                        int nparts, PcgScal *sc, unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    __shared__ SPlane sp[KC];
-    s_planes(L, sp);
-    double acc = 0.0;
-    if (i < L.nx && j < L.ny) {
-        const SCol a = s_col(L, i, j);
-        for (int kk = 0; kk < KC; kk++) {
-            int k = blockIdx.z * KC + kk;
-            if (k >= L.nz) break;
-            long long c = ((long long)k * L.ny + j) * L.nx + i;
-            Cell cc{i, j, k};
-            double v = s_apply(L, a, sp[kk], p, c, cc);
-            q[c] = v;
-            acc += p[c] * v;
-        }
-    }
-    block_store256<1>({acc}, part + blk3(), 0);
-    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
-    if (count && last_block(count, nb)) {
-        sum_parts<1>(part, 0, (int)nb, &sc->pq);
+    double acc[G] = {};
+    s_march<G>(L, p, [&](int g, long long c, double pc, double v) {
+        q[c] = v;
+        acc[g] += pc * v;
+    });
+    store_groups<G>(L, acc, part);
+    if (count && last_block(count, gridDim.x * gridDim.y * gridDim.z)) {
+        sum_parts<1>(part, 0, nparts, &sc->pq);
         if (threadIdx.x == 0 && threadIdx.y == 0) {
             sc->alpha = sc->pq != 0.0 ? sc->rz / sc->pq : 0.0;
             sc->rz_old = sc->rz;
@@ -238,31 +268,72 @@ __global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__re
     }
 }
 
-__global__ void k_dot(long long n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ part,
-                      double *dst, unsigned *count)
+// The grid-stride reductions are those of NP blocks of BS threads (or as many
+// as have elements); a block of a launch stands for VB of them, so that a
+// thread has VB elements in flight and VB sums share the block's barriers.
+// vb_first: the thread's first element in the u-th of them
+__device__ __forceinline__ long long vb_first(int u) { return ((long long)blockIdx.x * VB + u) * BS + threadIdx.x; }
+template <int NVAL>
+__device__ __forceinline__ void store_vb(const double (&acc)[NVAL * VB], double *part, int nvb)
 {
-    double acc = 0.0;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        acc += a[c] * b[c];
-    block_store256<1>({acc}, part + blockIdx.x, 0);
-    if (last_block(count, gridDim.x)) sum_parts<1>(part, 0, gridDim.x, dst);
+    double s[NVAL * VB];
+    block_sum256<NVAL * VB>(acc, s);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int v = 0; v < NVAL; v++)
+#pragma unroll
+            for (int u = 0; u < VB; u++)
+                if ((int)blockIdx.x * VB + u < nvb) part[(long long)v * NP + blockIdx.x * VB + u] = s[v * VB + u];
+}
+
+__global__ void k_dot(long long n, int nvb, const double *__restrict__ a, const double *__restrict__ b,
+                      double *__restrict__ part, double *dst, unsigned *count)
+{
+    const long long stride = (long long)nvb * BS;
+    double acc[VB] = {};
+    for (long long o = 0; o < n; o += stride) {
+        double av[VB], bv[VB];
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            const bool in = c < n && (int)blockIdx.x * VB + u < nvb;
+            av[u] = in ? a[c] : 0.0;
+            bv[u] = in ? b[c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < VB; u++) acc[u] += av[u] * bv[u];
+    }
+    store_vb<1>(acc, part, nvb);
+    if (last_block(count, gridDim.x)) sum_parts<1>(part, 0, nvb, dst);
 }
 
 // rz = r.z and zr_old = z.r_old, then beta (0 on a restart)
-__global__ void k_dot2(long long n, const double *__restrict__ r, const double *__restrict__ z,
+__global__ void __launch_bounds__(BS, 4) k_dot2(long long n, int nvb, const double *__restrict__ r, const double *__restrict__ z,
                        const double *__restrict__ ro, double *__restrict__ part, PcgScal *sc, int restart, unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
-    double a = 0.0, b = 0.0;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        double zc = z[c];
-        a += r[c] * zc;
-        b += ro[c] * zc;
+    const long long stride = (long long)nvb * BS;
+    double acc[2 * VB] = {};
+    for (long long o = 0; o < n; o += stride) {
+        double zv[VB], rv[VB], ov[VB];
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            const bool in = c < n && (int)blockIdx.x * VB + u < nvb;
+            zv[u] = in ? z[c] : 0.0;
+            rv[u] = in ? r[c] : 0.0;
+            ov[u] = in ? ro[c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            acc[u] += rv[u] * zv[u];
+            acc[VB + u] += ov[u] * zv[u];
+        }
     }
-    block_store256<2>({a, b}, part + blockIdx.x, NP);
+    store_vb<2>(acc, part, nvb);
     if (last_block(count, gridDim.x)) {
-        sum_parts<2>(part, NP, gridDim.x, &sc->rz);   // rz and, next to it, zr_old
+        sum_parts<2>(part, NP, nvb, &sc->rz);   // rz and, next to it, zr_old
         if (threadIdx.x == 0 && !restart) sc->beta = sc->rz_old != 0.0 ? (sc->rz - sc->zr_old) / sc->rz_old : 0.0;
     }
 }
@@ -276,33 +347,67 @@ __global__ void k_reduce(const double *__restrict__ part, int nvals, int nper, d
     }
 }
 
-__global__ void k_pupdate(long long n, const double *__restrict__ z, double *__restrict__ p, const PcgScal *sc, int first)
+__global__ void k_pupdate(long long n, int nvb, const double *__restrict__ z, double *__restrict__ p, const PcgScal *sc,
+                          int first)
 {
     pdl_trigger();
     pdl_wait();
-    double beta = first ? 0.0 : sc->beta;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        p[c] = first ? z[c] : z[c] + beta * p[c];
+    const double beta = first ? 0.0 : sc->beta;
+    const long long stride = (long long)nvb * BS;
+    for (long long o = 0; o < n; o += stride) {
+        double zv[VB], pv[VB];
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            const bool in = c < n && (int)blockIdx.x * VB + u < nvb;
+            zv[u] = in ? z[c] : 0.0;
+            pv[u] = in && !first ? p[c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            if (c < n && (int)blockIdx.x * VB + u < nvb) p[c] = first ? zv[u] : zv[u] + beta * pv[u];
+        }
+    }
 }
 
-__global__ void k_xrupdate(long long n, double *__restrict__ x, double *__restrict__ r, double *__restrict__ ro,
-                           const double *__restrict__ p, const double *__restrict__ q, PcgScal *sc,
-                           double *__restrict__ part, double *host_rr, unsigned *count)
+// x += alpha p, r_old = r, r -= alpha q and |r|^2
+__global__ void __launch_bounds__(BS, 3) k_xrupdate(long long n, int nvb, double *__restrict__ x, double *__restrict__ r,
+                           double *__restrict__ ro, const double *__restrict__ p, const double *__restrict__ q,
+                           PcgScal *sc, double *__restrict__ part, double *host_rr, unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
-    double alpha = sc->alpha, acc = 0.0;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        double rc = r[c];
-        ro[c] = rc;
-        x[c] += alpha * p[c];
-        rc -= alpha * q[c];
-        r[c] = rc;
-        acc += rc * rc;
+    const double alpha = sc->alpha;
+    const long long stride = (long long)nvb * BS;
+    double acc[VB] = {};
+    for (long long o = 0; o < n; o += stride) {
+        double rv[VB], xv[VB], pv[VB], qv[VB];
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            const bool in = c < n && (int)blockIdx.x * VB + u < nvb;
+            rv[u] = in ? r[c] : 0.0;
+            qv[u] = in ? q[c] : 0.0;
+            xv[u] = in ? x[c] : 0.0;
+            pv[u] = in ? p[c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < VB; u++) {
+            const long long c = vb_first(u) + o;
+            if (c < n && (int)blockIdx.x * VB + u < nvb) {
+                double rc = rv[u];
+                ro[c] = rc;
+                x[c] = xv[u] + alpha * pv[u];
+                rc -= alpha * qv[u];
+                r[c] = rc;
+                acc[u] += rc * rc;
+            }
+        }
     }
-    block_store256<1>({acc}, part + blockIdx.x, 0);
+    store_vb<1>(acc, part, nvb);
     if (last_block(count, gridDim.x)) {
-        sum_parts<1>(part, 0, gridDim.x, &sc->rr);
+        sum_parts<1>(part, 0, nvb, &sc->rr);
         if (threadIdx.x == 0) *host_rr = sc->rr;   // page-locked: the host reads it after its wait
     }
 }
@@ -497,43 +602,71 @@ void pcg_scatter(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const doub
     k_scatter<<<dim3((d.NX + 31) / 32, (d.NY + 7) / 8, d.NZ), dim3(32, 8), 0, s>>>(d, L0, x, phi_da);
 }
 
+// plane groups per block of the stencil kernels: as many as leave about seven
+// 256-thread blocks per SM (k_apply at 256x128x128, 4096 partials: 125 us
+// with one group, 109 us with four; at 128x64x64, 512 partials, fewer blocks
+// than one group gives would leave SMs idle)
+static int groups(const MgDevLevel &L0)
+{
+    const int parts = pcg_stencil_parts(L0);
+    return parts >= 4096 ? 4 : parts >= 2048 ? 2 : 1;
+}
+static dim3 g3g(const MgDevLevel &L0, int g)
+{
+    dim3 d = g3k(L0);
+    d.z = (d.z + g - 1) / g;
+    return d;
+}
+
 void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part,
                double *dst, unsigned *count)
 {
-    k_resid<<<g3k(L0), dim3(32, 8), 0, s>>>(L0, bw, x, r, part, dst, count);
+    const int np = pcg_stencil_parts(L0), g = groups(L0);
+    const dim3 gr = g3g(L0, g), b(32, 8);
+    if (g == 4) k_resid<4><<<gr, b, 0, s>>>(L0, bw, x, r, part, np, dst, count);
+    else if (g == 2) k_resid<2><<<gr, b, 0, s>>>(L0, bw, x, r, part, np, dst, count);
+    else k_resid<1><<<gr, b, 0, s>>>(L0, bw, x, r, part, np, dst, count);
 }
 
 void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc,
                unsigned *count)
 {
-    launch_pdl(k_apply, g3k(L0), dim3(32, 8), s, L0, p, q, part, sc, count);
+    const int np = pcg_stencil_parts(L0), g = groups(L0);
+    const dim3 gr = g3g(L0, g), b(32, 8);
+    if (g == 4) launch_pdl(k_apply<4>, gr, b, s, L0, p, q, part, np, sc, count);
+    else if (g == 2) launch_pdl(k_apply<2>, gr, b, s, L0, p, q, part, np, sc, count);
+    else launch_pdl(k_apply<1>, gr, b, s, L0, p, q, part, np, sc, count);
 }
 
 void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part, double *dst, unsigned *count)
 {
-    k_dot<<<nblk(n), BS, 0, s>>>(n, a, b, part, dst, count);
+    const unsigned nb = nblk(n);
+    k_dot<<<(nb + VB - 1) / VB, BS, 0, s>>>(n, (int)nb, a, b, part, dst, count);
 }
 
 void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part,
               PcgScal *sc, int restart, unsigned *count)
 {
-    launch_pdl(k_dot2, dim3(nblk(n)), dim3(BS), s, n, r, z, rold, part, sc, restart, count);
-}
-
-void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper)
-{
-    k_reduce<<<1, 1024, 0, s>>>(part, nvals, nper > 0 ? nper : NP, dst);
+    const unsigned nb = nblk(n);
+    launch_pdl(k_dot2, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, r, z, rold, part, sc, restart, count);
 }
 
 void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first)
 {
-    launch_pdl(k_pupdate, dim3(nblk(n)), dim3(BS), s, n, z, p, sc, first);
+    const unsigned nb = nblk(n);
+    launch_pdl(k_pupdate, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, z, p, sc, first);
 }
 
 void pcg_xrupdate(cudaStream_t s, long long n, double *x, double *r, double *rold, const double *p,
                   const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count)
 {
-    launch_pdl(k_xrupdate, dim3(nblk(n)), dim3(BS), s, n, x, r, rold, p, q, sc, part, host_rr, count);
+    const unsigned nb = nblk(n);
+    launch_pdl(k_xrupdate, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, x, r, rold, p, q, sc, part, host_rr, count);
+}
+
+void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper)
+{
+    k_reduce<<<1, 1024, 0, s>>>(part, nvals, nper > 0 ? nper : NP, dst);
 }
 
 void pcg_to_float(cudaStream_t s, long long n, const double *a, float *b) { k_f2<<<nblk(n), BS, 0, s>>>(n, a, b); }

@@ -2679,9 +2679,7 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             // x0 and the network candidate: it is kept whenever it lowers the
             // residual in the S^-1 norm (de < 0), the norm CG reduces
             fitted = ng > 0.0 && de < 0.0;
-            if (fitted) {   // the fit is in pp / pro
-                std::swap(c->pz, c->pp);
-                std::swap(c->pq, c->pro);
+            if (fitted) {
                 nrc = ng;
                 ok = 1;
             }
@@ -2690,8 +2688,10 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             c->guess_tried++;
             if (nr > 0.0 && nrc > 0.0 && std::isfinite(nrc)) c->guess_logsum += std::log(nrc / nr);
             if (fitted || nrc < nr) {
-                pcg_copy(s, n0, c->pz, c->px);
-                pcg_copy(s, n0, c->pq, c->pr);
+                // the fit is in pp / pro (the captured graphs hold these
+                // buffers by their roles, so they are not swapped)
+                pcg_copy(s, n0, fitted ? c->pp : c->pz, c->px);
+                pcg_copy(s, n0, fitted ? c->pro : c->pq, c->pr);
                 c->launches += 2;
                 nr = nrc;
                 c->guess_taken++;
@@ -2769,12 +2769,13 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
                          : mg_vcycle_bytes<float>(c->H32, 0, npre, npost) + 24.0 * n0);
         ph = prof_begin(c, TURB_PROF_PCG);
         if (c->use_graphs) {
-            if (!c->g_pcg[restart]) {
+            cudaGraphExec_t &g = c->g_pcg[restart];
+            if (!g) {
                 int rs = restart;
-                int rc = capture(c, &c->g_pcg[restart], [&]() { cgstep(rs); });
+                int rc = capture(c, &g, [&]() { cgstep(rs); });
                 if (rc) return rc;
             }
-            TURB_CHECK(cudaGraphLaunch(c->g_pcg[restart], s));
+            TURB_CHECK(cudaGraphLaunch(g, s));
         } else {
             cgstep(restart);
         }
