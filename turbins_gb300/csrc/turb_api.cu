@@ -302,8 +302,14 @@ W2 mk_w2(DevBuf &m, int n, int first, int last, const std::vector<double> &X0, c
         w1[t] = 1.0 - w0[t];
     }
     W2 o;
+    o.half = 1;
+    for (int t = first; t <= last; t++)
+        if (w0[t] != 0.5 || w1[t] != 0.5) o.half = 0;
     o.w0 = m.upload(w0);
     o.w1 = m.upload(w1);
+    for (int t = 0; t < n; t++) { w0[t] *= 0.5; w1[t] *= 0.5; }
+    o.h0 = m.upload(w0);
+    o.h1 = m.upload(w1);
     return o;
 }
 
@@ -361,20 +367,6 @@ EnoTab mk_eno(DevBuf &m, int r, const std::vector<double> &pos, int s0, int e0, 
             g3[3 * c + t] = (xi - a) * (xi - bb) + (xi - bb) * (xi - e) + (xi - a) * (xi - e);
         }
     }
-    T.h1 = m.upload(h1);
-    T.h2 = m.upload(h2);
-    T.h3 = m.upload(h3);
-    std::vector<double> r1(nb), r2(nb), r3(nb), l1(nb), l2(nb), l3(nb);
-    for (int b = 0; b < nb; b++) {
-        r1[b] = 1.0 / h1[b]; r2[b] = 1.0 / h2[b]; r3[b] = 1.0 / h3[b];
-        l1[b] = recip_low(h1[b], r1[b]); l2[b] = recip_low(h2[b], r2[b]); l3[b] = recip_low(h3[b], r3[b]);
-    }
-    T.rh1 = m.upload(r1);
-    T.rh2 = m.upload(r2);
-    T.rh3 = m.upload(r3);
-    T.rl1 = m.upload(l1);
-    T.rl2 = m.upload(l2);
-    T.rl3 = m.upload(l3);
     T.fastdiv = 1;   // reciprocal-based, correctly rounded (turb_div.cuh); 0 = IEEE division
     // power-of-two spacings (uniform grids with 2^k cells per unit length):
     // the reciprocal is exact and a/h = a*(1/h) is the same real number, so
@@ -384,16 +376,42 @@ EnoTab mk_eno(DevBuf &m, int r, const std::vector<double> &pos, int s0, int e0, 
         return h > 0.0 && std::isfinite(h) && std::frexp(h, &e) == 0.5;
     };
     // other spacings whose two-term quotient alone rounds as the division
-    // for every numerator (div_two_term_exact, turb_div.cuh): bits 3-5
-    std::vector<uint8_t> p2(nb, 0);
+    // for every numerator (div_two_term_exact, turb_div.cuh): form 2
+    auto divs = [&](const std::vector<double> &h) {
+        std::vector<EnoDiv> t(nb);
+        for (int b = 0; b < nb; b++) {
+            const double y = 1.0 / h[b], yl = recip_low(h[b], y);
+            t[b] = EnoDiv{y, yl, h[b], pow2(h[b]) ? 1 : (div_two_term_exact(h[b], y, yl) ? 2 : 3), 0};
+        }
+        return m.upload(t);
+    };
+    T.d1 = divs(h1);
+    T.d2 = divs(h2);
+    T.d3 = divs(h3);
+    // one power-of-two spacing throughout: a quotient by h or 2h is one exact
+    // scaling, and the products with g2 and g3 are exact too
+    const double h = h1[0];
+    bool uni = pow2(h) && h > 1e-30 && h < 1e30;
     for (int b = 0; b < nb; b++) {
-        int f = (pow2(h1[b]) ? 1 : 0) | (pow2(h2[b]) ? 2 : 0) | (pow2(h3[b]) ? 4 : 0);
-        if (!(f & 1) && div_two_term_exact(h1[b], r1[b], l1[b])) f |= 8;
-        if (!(f & 2) && div_two_term_exact(h2[b], r2[b], l2[b])) f |= 16;
-        if (!(f & 4) && div_two_term_exact(h3[b], r3[b], l3[b])) f |= 32;
-        p2[b] = (uint8_t)f;
+        if (b < nb - 1) uni = uni && h1[b] == h;
+        if (b > 0 && b < nb - 1) uni = uni && h2[b] == 2.0 * h;
+        if (b > 0 && b < nb - 2) uni = uni && h3[b] == 3.0 * h;
+        if (b >= r && b < nb - r) {
+            uni = uni && g2[2 * b] == h && g2[2 * b + 1] == -h;
+            if (r > 2)
+                uni = uni && g3[3 * b] == 2.0 * h * h && g3[3 * b + 1] == -h * h && g3[3 * b + 2] == 2.0 * h * h;
+        }
     }
-    T.p2 = m.upload(p2);
+    T.uni = uni ? 1 : 0;
+    T.uh = h;
+    T.uh3 = 3.0 * h;
+    T.ru1 = 1.0 / h;
+    T.ru2 = 0.5 / h;
+    T.ru3 = 1.0 / T.uh3;
+    T.ru3l = recip_low(T.uh3, T.ru3);
+    T.ug3 = 2.0 * h * h;
+    T.ug3m = -h * h;
+    T.uni = T.uni && div_two_term_exact(T.uh3, T.ru3, T.ru3l);
     T.g2 = m.upload(g2);
     T.g3 = m.upload(g3);
     return T;

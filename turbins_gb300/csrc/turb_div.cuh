@@ -23,11 +23,25 @@
 
 #include <cmath>
 
+// The words of a double as the integer pipe sees them: the compiler turns
+// tests on the bits of a bitcast double (== 0 without the sign, ordered
+// magnitudes) back into FP64 compares, which cost an FP64 operation each
+struct DWords {
+    unsigned lo, hi;
+};
+__device__ __forceinline__ DWords dwords(double a)
+{
+    DWords w;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(w.lo), "=r"(w.hi) : "d"(a));
+    return w;
+}
+__device__ __forceinline__ bool dw_zero(DWords w) { return ((w.hi << 1) | w.lo) == 0u; }
+
 __device__ __forceinline__ double div_by_spacing(double a, double h, double y, double yl)
 {
-    unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-    unsigned e = (unsigned)(bits >> 52) & 0x7FFu;
-    if ((bits << 1) == 0ull) return a;
+    const DWords w = dwords(a);
+    unsigned e = (w.hi >> 20) & 0x7FFu;
+    if (dw_zero(w)) return a;
     if (e < 123u || e > 1923u) return __ddiv_rn(a, h);
     double q = __fma_rn(a, y, __dmul_rn(a, yl));
     double r = __fma_rn(-q, h, a);
@@ -45,9 +59,9 @@ __host__ __device__ inline double recip_low(double h, double y)
 // numerators and the exponent range as in div_by_spacing.
 __device__ __forceinline__ double div_by_spacing_2t(double a, double h, double y, double yl)
 {
-    unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-    unsigned e = (unsigned)(bits >> 52) & 0x7FFu;
-    if ((bits << 1) == 0ull) return a;
+    const DWords w = dwords(a);
+    unsigned e = (w.hi >> 20) & 0x7FFu;
+    if (dw_zero(w)) return a;
     if (e < 123u || e > 1923u) return __ddiv_rn(a, h);
     return __fma_rn(a, y, __dmul_rn(a, yl));
 }

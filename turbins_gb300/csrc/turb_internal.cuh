@@ -63,6 +63,17 @@ struct Interp2 {
 // W0 = |(xq - X0) / (X1 - X0)| (as a_D * (xq - X0)), W1 = 1 - W0.
 struct W2 {
     const double *w0, *w1;
+    const double *h0 = nullptr, *h1 = nullptr;   // half of each (exact)
+    int half = 0;                                // 1: every weight in use is 1/2
+};
+
+// Division by one spacing h of an ENO line, as two 16-byte loads: y = RN(1/h),
+// its correction yl = RN((1 - y h)/h), and the form that rounds as the
+// division: 1 a power of two (a y is exact), 2 the two-term quotient alone
+// (div_two_term_exact), 3 with its correction
+struct alignas(16) EnoDiv {
+    double y, yl, h;
+    int form, pad;
 };
 
 // ENO line tables of one (quantity, direction): buffer index b in [0, nb),
@@ -72,17 +83,18 @@ struct W2 {
 // *_ENO_ghost_cells routines), so device results round identically.
 struct EnoTab {
     int r, s0, e0, nb;
-    const double *h1;    // P[b+1]-P[b]
-    const double *h2;    // P[b+1]-P[b-1]
-    const double *h3;    // P[b+2]-P[b-1]
+    const EnoDiv *d1;    // by h1 = P[b+1]-P[b]
+    const EnoDiv *d2;    // by h2 = P[b+1]-P[b-1]
+    const EnoDiv *d3;    // by h3 = P[b+2]-P[b-1]
     const double *g2;    // [nb*2]: k=b-1, k=b  -> (x_i-x_k)+(x_i-x_k1)
     const double *g3;    // [nb*3]: kstar=b-2,b-1,b -> three-product sum
-    const double *rh1, *rh2, *rh3;   // RN(1/h*) for the reciprocal-based division
-    const double *rl1, *rl2, *rl3;   // and its correction RN((1 - RN(1/h) h)/h)
     int fastdiv;         // 1: div_by_spacing (turb_div.cuh), 0: IEEE division
-    const uint8_t *p2;   // per b: bit 0/1/2 set when h1/h2/h3 is a power of two, so that
-                         // a/h = a*RN(1/h) exactly; bit 3/4/5 when the two-term
-                         // quotient alone is exact (div_two_term_exact; fastdiv only)
+    int uni;             // 1: every spacing is the same power of two (with the positions dyadic, so the
+                         // differences' factors g2 = +-h and g3 = 2h^2, -h^2, 2h^2 are exact), fastdiv only
+    double uh, uh3;      // that spacing h, and 3h
+    double ru1, ru2;     // 1/h, 1/(2h)
+    double ru3, ru3l;    // RN(1/(3h)) and its correction
+    double ug3, ug3m;    // 2h^2, -h^2
     int gsrc[6];         // ghost b<r: [0..r), ghost b>=nb-r: [3..3+r) by ex
     double gm[6];        // 0: zero, 1: m*q[s0], 2: m*q[e0], 3: glo[line], 4: ghi[line]
     const double *glo = nullptr, *ghi = nullptr;   // x lines at open faces: [NZ][NY] planes

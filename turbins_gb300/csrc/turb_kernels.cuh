@@ -51,6 +51,10 @@ struct AdvSrc {
     // outflow planes replace u at i = 0 / i = nx ([NZ][NY], null when closed)
     const double *pin = nullptr, *pout = nullptr;
     int pNY = 0, nx = 0;
+    // filled by launch_eno_pass for kinds 2..7: offsets of the four values
+    // from the node, and the axis (0 i, 1 j, 2 k) that indexes wx and wy
+    long long off[4] = {0, 0, 0, 0};
+    int ax = 0, ay = 0;
 };
 void launch_eno_pass(cudaStream_t s, const Dims &d, int dir, const EnoTab &tab, const double *q, AdvSrc adv,
                      int t1a, int t1b, int t2a, int t2b, int first, double *conv, int segments = 0);
