@@ -1,16 +1,19 @@
 // k_conv.cu -- 3x3x3 convolutions (stride 1, zero padding 1) as implicit
 // GEMMs on the tcgen05 tensor cores: BF16 operands, FP32 accumulators in
-// TMEM, operands staged by TMA, one producer warp, one MMA warp and four
-// epilogue warps per CTA, persistent CTAs with a double-buffered accumulator.
+// TMEM, four producer warps, one MMA thread and four epilogue warps per CTA,
+// persistent CTAs.
 //
 // Forward (and data gradient, the same kernel on mirrored weights):
 //   out[v][co] = sum_tap sum_ci W[tap][co][ci] * in[v + off(tap)][ci]
-// GEMM view per output tile: M = 128 voxels, N = cout, K = 27 taps x cin.
-// On grids at least 128 voxels wide a tile is one x row and, per channel
-// chunk, ONE TMA box (130 x 3 x 3 voxels) feeds all 27 taps: the A operand of
-// tap (dx, dy, dz) is the same shared-memory slab at a 16-byte-granular offset.
-// Narrower grids load one 128-voxel box per tap (TMA fills the padding with
-// zeros either way).
+// GEMM view: M = 128 voxels, N = output channels, K = taps x cin.  Two kernels:
+// k_conv_rows (cin, cout <= 32: resident weights, taps of one axis stacked
+// along N) and k_conv_wide (more channels: weights staged per tap, the output
+// channels split over CTAs where there are few tiles).  Both read 128-byte
+// swizzled K-major operands and load a voxel row once for its three x taps.
+// Against one load per tap into unswizzled operands (a K step then took 150-230
+// cycles whatever N is, and a 16-byte-wide box one cycle per voxel) and a row
+// kernel that formed its descriptors at run time, the network's forward pass
+// went from 329 to 190 us at 64x32x32 and from 1318 to 704 us at 256x128x128.
 //
 // Weight gradient: dW[tap][co][ci] = sum_v dy[v][co] * in[v + off(tap)][ci];
 // M = (taps of a group) x cin = 128 rows, N = cout, K = voxels, both operands
@@ -30,23 +33,12 @@ namespace {
 
 char g_conv_err[256] = "";
 
-// barrier slots
-constexpr int FA = 0, EA = 4, FB = 8, EB = 16, AF = 24, AE = 26, WB = 28, FIN = 29, NBAR = 30;
-
-struct ConvArgs {
-    int X, Y, Z, cin, cout, kc, nkc;
-    int slab, bx, by, bz, ntx, nty, ntz, ntiles;
-    int wres, sa, sb;
-    uint32_t abytes, bbytes, astride, bstride, wbytes, a_lbo;
-    const bf16 *wpk;
-    const float *bias;
-    int relu;
-    const bf16 *skip, *mask;
-    bf16 *out;
-    const float *headw, *headb;
-    float *hout;
-    int *err;
-};
+// barrier waits that must outlive an abort: copies and MMAs in flight
+__device__ __forceinline__ void settle(uint32_t bar, uint32_t parity)
+{
+    volatile int never = 0;
+    tc::mbar_wait(bar, parity, &never);
+}
 
 __device__ __forceinline__ void fail(volatile int *abort_, int *err, int code)
 {
@@ -56,291 +48,71 @@ __device__ __forceinline__ void fail(volatile int *abort_, int *err, int code)
 
 // last fill of stage s among `n` fills of an S-stage ring, waited for so that
 // no copy is still landing when the CTA exits
-__device__ __forceinline__ void drain(uint32_t bars, int base, uint32_t n, int S, volatile int *abort_)
+__device__ __forceinline__ void drain(uint32_t bars, int base, uint32_t n, int S)
 {
     for (int s = 0; s < S; s++) {
         if ((uint32_t)s >= n) break;
         uint32_t last = (uint32_t)s + (uint32_t)S * ((n - 1 - (uint32_t)s) / (uint32_t)S);
-        tc::mbar_wait(bars + 8 * (base + s), (last / S) & 1, abort_);
+        settle(bars + 8 * (base + s), (last / S) & 1);
     }
 }
 
-// epilogue of one 128-voxel tile: this thread's accumulator row (all cout
-// columns from TMEM, loaded by the whole warp) -> bias, skip, ReLU, mask,
-// BF16 store, optional 1x1x1 head
+// what is done to 16 output channels of one voxel: bias, ReLU, mask, BF16
+// store, optional 1x1x1 head (hsum)
 struct EpiP {
     const float *bias;
     int relu;
-    const bf16 *skip, *mask;
+    const bf16 *mask;
     bf16 *out;
     const float *headw, *headb;
     float *hout;
-    int cout;
     size_t plane;
 };
 
-__device__ __forceinline__ void epilogue(const EpiP &a, uint32_t taddr, size_t vox, bool valid)
+__device__ __forceinline__ void epilogue16(const EpiP &a, int ch, const uint32_t (&rr)[16], const float (&bias)[16],
+                                           const float (&hw)[16], size_t vox, float &hsum)
 {
-    float hsum = 0.f;
-    for (int ch = 0; ch < (a.cout >> 4); ch++) {
-        uint32_t rr[16];
-        tc::tmem_ld16(taddr + (uint32_t)ch * 16u, rr);
-        tc::tmem_wait_ld();
-        if (!valid) continue;
-        float v[16];
+    float v[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(rr[j]);
-        if (a.bias) {
+    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(rr[j]) + bias[j];
+    const size_t o0 = ((size_t)(2 * ch) * a.plane + vox) * 8, o1 = o0 + a.plane * 8;
+    if (a.relu) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] += a.bias[ch * 16 + j];
-        }
-        size_t o0 = ((size_t)(2 * ch) * a.plane + vox) * 8, o1 = o0 + a.plane * 8;
-        if (a.skip) {
-            uint4 s0 = *reinterpret_cast<const uint4 *>(a.skip + o0);
-            uint4 s1 = *reinterpret_cast<const uint4 *>(a.skip + o1);
-            const bf16 *p0 = reinterpret_cast<const bf16 *>(&s0), *p1 = reinterpret_cast<const bf16 *>(&s1);
+        for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.f);
+    }
+    if (a.mask) {
+        uint4 m0 = *reinterpret_cast<const uint4 *>(a.mask + o0);
+        uint4 m1 = *reinterpret_cast<const uint4 *>(a.mask + o1);
+        const bf16 *p0 = reinterpret_cast<const bf16 *>(&m0), *p1 = reinterpret_cast<const bf16 *>(&m1);
 #pragma unroll
-            for (int j = 0; j < 8; j++) { v[j] += __bfloat162float(p0[j]); v[8 + j] += __bfloat162float(p1[j]); }
-        }
-        if (a.relu) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.f);
-        }
-        if (a.mask) {
-            uint4 m0 = *reinterpret_cast<const uint4 *>(a.mask + o0);
-            uint4 m1 = *reinterpret_cast<const uint4 *>(a.mask + o1);
-            const bf16 *p0 = reinterpret_cast<const bf16 *>(&m0), *p1 = reinterpret_cast<const bf16 *>(&m1);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                if (!(__bfloat162float(p0[j]) > 0.f)) v[j] = 0.f;
-                if (!(__bfloat162float(p1[j]) > 0.f)) v[8 + j] = 0.f;
-            }
-        }
-        uint4 w0, w1;
-        bf16 *q0 = reinterpret_cast<bf16 *>(&w0), *q1 = reinterpret_cast<bf16 *>(&w1);
-#pragma unroll
-        for (int j = 0; j < 8; j++) { q0[j] = __float2bfloat16_rn(v[j]); q1[j] = __float2bfloat16_rn(v[8 + j]); }
-        if (a.out) {
-            *reinterpret_cast<uint4 *>(a.out + o0) = w0;
-            *reinterpret_cast<uint4 *>(a.out + o1) = w1;
-        }
-        if (a.headw) {
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                hsum = fmaf(a.headw[ch * 16 + j], __bfloat162float(q0[j]), hsum);
-                hsum = fmaf(a.headw[ch * 16 + 8 + j], __bfloat162float(q1[j]), hsum);
-            }
+        for (int j = 0; j < 8; j++) {
+            if (!(__bfloat162float(p0[j]) > 0.f)) v[j] = 0.f;
+            if (!(__bfloat162float(p1[j]) > 0.f)) v[8 + j] = 0.f;
         }
     }
-    if (valid && a.hout) a.hout[vox] = hsum + *a.headb;
+    uint4 w0, w1;
+    bf16 *q0 = reinterpret_cast<bf16 *>(&w0), *q1 = reinterpret_cast<bf16 *>(&w1);
+#pragma unroll
+    for (int j = 0; j < 8; j++) { q0[j] = __float2bfloat16_rn(v[j]); q1[j] = __float2bfloat16_rn(v[8 + j]); }
+    if (a.out) {
+        *reinterpret_cast<uint4 *>(a.out + o0) = w0;
+        *reinterpret_cast<uint4 *>(a.out + o1) = w1;
+    }
+    if (a.headw) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            hsum = fmaf(hw[j], __bfloat162float(q0[j]), hsum);
+            hsum = fmaf(hw[8 + j], __bfloat162float(q1[j]), hsum);
+        }
+    }
 }
 
-__global__ void __launch_bounds__(192) k_conv(const __grid_constant__ CUtensorMap mapA, ConvArgs a)
-{
-    extern __shared__ uint8_t dsm[];
-    __shared__ __align__(8) uint64_t bar[NBAR];
-    __shared__ uint32_t tslot;
-    __shared__ int abort_s;
-    volatile int *abort_ = &abort_s;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t sraw = tc::smem_u32(dsm);
-    const uint32_t sA = (sraw + 1023u) & ~1023u;
-    const uint32_t nA = a.slab ? 2u : (uint32_t)a.sa;
-    const uint32_t sB = sA + nA * a.astride;
-    const uint32_t bars = tc::smem_u32(bar);
-    const uint32_t ncols = a.cout * 2 < 32 ? 32u : (uint32_t)(a.cout * 2);
-
-    if (threadIdx.x == 0) {
-        abort_s = 0;
-        for (int i = 0; i < NBAR; i++) tc::mbar_init(bars + 8 * i, (i == AE || i == AE + 1) ? 4u : 1u);
-        tc::mbar_fence_init();
-        tc::prefetch_map(&mapA);
-    }
-    if (warp == 1) {
-        tc::tmem_alloc(tc::smem_u32(&tslot), ncols);
-        tc::tmem_relinquish();
-    }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tbase = tslot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            uint32_t ua = 0, ub = 0;
-            bool ok = true;
-            if (a.wres) {
-                tc::mbar_expect_tx(bars + 8 * WB, a.wbytes);
-                tc::bulk_load(sB, a.wpk, a.wbytes, bars + 8 * WB);
-            }
-            for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x) {
-                int tx = t % a.ntx, r = t / a.ntx, ty = r % a.nty, tz = r / a.nty;
-                int x0 = tx * a.bx, y0 = ty * a.by, z0 = tz * a.bz;
-                for (int kci = 0; ok && kci < a.nkc; kci++) {
-                    int cb = kci * (a.kc >> 3);
-                    if (a.slab) {
-                        uint32_t s = ua & 1u;
-                        if (!tc::mbar_wait(bars + 8 * (EA + s), ((ua >> 1) & 1u) ^ 1u, abort_)) { ok = false; break; }
-                        tc::mbar_expect_tx(bars + 8 * (FA + s), a.abytes);
-                        tc::tma_load5(sA + s * a.astride, &mapA, 0, x0 - 1, y0 - 1, z0 - 1, cb, bars + 8 * (FA + s));
-                        ua++;
-                    }
-                    for (int tap = 0; tap < 27; tap++) {
-                        if (!a.slab) {
-                            uint32_t s = ua % (uint32_t)a.sa;
-                            if (!tc::mbar_wait(bars + 8 * (EA + s), ((ua / a.sa) & 1u) ^ 1u, abort_)) { ok = false; break; }
-                            int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-                            tc::mbar_expect_tx(bars + 8 * (FA + s), a.abytes);
-                            tc::tma_load5(sA + s * a.astride, &mapA, 0, x0 + dx - 1, y0 + dy - 1, z0 + dz - 1, cb,
-                                          bars + 8 * (FA + s));
-                            ua++;
-                        }
-                        if (!a.wres) {
-                            uint32_t s = ub % (uint32_t)a.sb;
-                            if (!tc::mbar_wait(bars + 8 * (EB + s), ((ub / a.sb) & 1u) ^ 1u, abort_)) { ok = false; break; }
-                            tc::mbar_expect_tx(bars + 8 * (FB + s), a.bbytes);
-                            tc::bulk_load(sB + s * a.bstride, a.wpk + (size_t)(kci * 27 + tap) * a.kc * a.cout, a.bbytes,
-                                          bars + 8 * (FB + s));
-                            ub++;
-                        }
-                    }
-                }
-            }
-            if (!ok) fail(abort_, a.err, 1);
-            drain(bars, FA, ua, (int)nA, abort_);
-            if (!a.wres) drain(bars, FB, ub, a.sb, abort_);
-            if (a.wres) tc::mbar_wait(bars + 8 * WB, 0, abort_);
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = tc::idesc_bf16(128, a.cout, 0, 0);
-            const uint32_t b_lbo = (uint32_t)a.cout * 16u;
-            uint32_t ua = 0, ub = 0, it = 0;
-            bool ok = true;
-            if (a.wres && !tc::mbar_wait(bars + 8 * WB, 0, abort_)) ok = false;
-            for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x, it++) {
-                uint32_t ab = it & 1u;
-                if (!tc::mbar_wait(bars + 8 * (AE + ab), ((it >> 1) & 1u) ^ 1u, abort_)) { ok = false; break; }
-                tc::fence_after();
-                uint32_t dt = tbase + ab * (uint32_t)a.cout;
-                for (int kci = 0; ok && kci < a.nkc; kci++) {
-                    uint32_t abuf = 0, sa_slab = 0;
-                    if (a.slab) {
-                        sa_slab = ua & 1u;
-                        if (!tc::mbar_wait(bars + 8 * (FA + sa_slab), (ua >> 1) & 1u, abort_)) { ok = false; break; }
-                        abuf = sA + sa_slab * a.astride;
-                    }
-                    for (int tap = 0; tap < 27; tap++) {
-                        uint32_t s_a = 0, s_b = 0, bbuf, aoff = 0;
-                        if (!a.slab) {
-                            s_a = ua % (uint32_t)a.sa;
-                            if (!tc::mbar_wait(bars + 8 * (FA + s_a), (ua / a.sa) & 1u, abort_)) { ok = false; break; }
-                            abuf = sA + s_a * a.astride;
-                        } else {
-                            int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-                            aoff = (uint32_t)(((dz * 3 + dy) * (a.bx + 2) + dx) * 16);
-                        }
-                        if (!a.wres) {
-                            s_b = ub % (uint32_t)a.sb;
-                            if (!tc::mbar_wait(bars + 8 * (FB + s_b), (ub / a.sb) & 1u, abort_)) { ok = false; break; }
-                            bbuf = sB + s_b * a.bstride;
-                        } else {
-                            bbuf = sB + (uint32_t)((kci * 27 + tap) * a.kc * a.cout * 2);
-                        }
-                        tc::fence_after();
-                        for (int ks = 0; ks < (a.kc >> 4); ks++) {
-                            uint64_t ad = tc::sdesc(abuf + aoff + (uint32_t)ks * 2u * a.a_lbo, a.a_lbo, 128);
-                            uint64_t bd = tc::sdesc(bbuf + (uint32_t)ks * 2u * b_lbo, b_lbo, 128);
-                            tc::mma_bf16(dt, ad, bd, idesc, (kci | tap | ks) != 0);
-                        }
-                        if (!a.wres) { tc::mma_commit(bars + 8 * (EB + s_b)); ub++; }
-                        if (!a.slab) { tc::mma_commit(bars + 8 * (EA + s_a)); ua++; }
-                    }
-                    if (ok && a.slab) { tc::mma_commit(bars + 8 * (EA + sa_slab)); ua++; }
-                }
-                if (ok) tc::mma_commit(bars + 8 * (AF + ab));
-            }
-            if (!ok) fail(abort_, a.err, 1);
-            tc::mma_commit(bars + 8 * FIN);
-            tc::mbar_wait(bars + 8 * FIN, 0, abort_);
-        }
-    } else if (warp >= 2) {
-        const int q = warp & 3, row = q * 32 + lane;
-        const int xx = row % a.bx, yy = (row / a.bx) % a.by, zz = row / (a.bx * a.by);
-        const size_t plane = (size_t)a.X * a.Y * a.Z;
-        uint32_t it = 0;
-        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, it++) {
-            uint32_t ab = it & 1u;
-            if (!tc::mbar_wait(bars + 8 * (AF + ab), (it >> 1) & 1u, abort_)) { fail(abort_, a.err, 1); break; }
-            tc::fence_after();
-            int tx = t % a.ntx, r = t / a.ntx, ty = r % a.nty, tz = r / a.nty;
-            int gx = tx * a.bx + xx, gy = ty * a.by + yy, gz = tz * a.bz + zz;
-            bool valid = zz < a.bz && gx < a.X && gy < a.Y && gz < a.Z;
-            size_t vox = ((size_t)gz * a.Y + gy) * a.X + gx;
-            uint32_t taddr = tbase + ((uint32_t)(q * 32) << 16) + ab * (uint32_t)a.cout;
-            epilogue(EpiP{a.bias, a.relu, a.skip, a.mask, a.out, a.headw, a.headb, a.hout, a.cout, plane}, taddr, vox,
-                     valid);
-            tc::fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(bars + 8 * (AE + ab));
-        }
-    }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    if (warp == 1) tc::tmem_dealloc(tbase, ncols);
-}
-
-
-// ---- row-ring convolution (grids at least 128 voxels wide, cin <= 32) ------------
-// A CTA takes items of (x tile of 128 voxels, z, a run of consecutive y rows).
-// Operands use the 128-byte-swizzle K-major layout, the one the tensor core
-// fetches fastest: every shared-memory row is one voxel holding 64 K elements,
-// here the channels of its three z planes (K = dz * cin + ci, zero padded),
-// 16-byte chunk c of row p stored at chunk c ^ (p % 8).  One input y row of
-// the tile (136 voxel rows, x0 - 1 ...) is a ring slot, filled by 16-byte
-// cp.async (producer warp L % 4 loads row L).  The A operand of tap dx is the
-// slot shifted by dx rows; dz and the channels are the K steps.  Every input row r feeds the output rows r+1, r, r-1
-// (dy = 0, 1, 2): the weights of the three dy taps are stacked along N, so
-// one MMA (M = 128 voxels, N = 3 cout, K = 16) per dx and K step covers all
-// of them; the three targets are consecutive blocks of a TMEM ring of NBLK
-// accumulator blocks (block of virtual row v = NBLK-1 - v mod NBLK, so rows
-// r+1, r, r-1 are ascending; a wrap splits the MMA).  Accumulation is always
-// on: the epilogue zeroes a block after draining it.  Weights are resident.
-constexpr int RING = 4, RW = 130, RROWS = 136;   // ring slots, voxels used / stored per slot
-constexpr int NBLK = 8;                          // TMEM accumulator blocks
-
-struct RowArgs {
-    int X, Y, Z, cin, cout;
-    int ntx, ych, nyc, nitems;
-    int nkb;                      // 128-byte K blocks per voxel row: ceil(3 cin / 64)
-    uint32_t slot_bytes, slab_bytes, wbytes;
-    const bf16 *in, *wpk;
-    EpiP epi;
-    int *err;
-};
-
-__host__ __device__ inline int rows_nkb(int cin) { return (3 * cin + 63) / 64; }
-// resident weights of the row kernel: per dx and K block, 3 cout rows of 128 bytes
-__host__ __device__ inline uint32_t rows_wbytes(int cin, int cout) { return 3u * (uint32_t)rows_nkb(cin) * 3u * cout * 128u; }
 // 128-byte-swizzle K-major operand at saddr (8-row groups 1024 bytes apart);
 // the swizzle follows the absolute address, so shifted starts need no offset
 __host__ __device__ inline uint64_t sw128_desc(uint32_t saddr)
 {
     return tc::sdesc(saddr, 16, 1024) | (2ull << 61);
 }
-
-// barrier slots of k_conv_rows
-constexpr int RF = 0, RE = RING, BRDY = 2 * RING, BFREE = 2 * RING + NBLK, RWB = 2 * RING + 2 * NBLK,
-              RFIN = RWB + 1, RNBAR = RWB + 2;
-
-__host__ __device__ inline uint32_t rows_ncols(int cout)
-{
-    uint32_t n = 32;
-    while (n < (uint32_t)(NBLK * cout)) n <<= 1;
-    return n;
-}
-__device__ __forceinline__ int blk_of(uint32_t v) { return NBLK - 1 - (int)(v % NBLK); }
 
 __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr)
 {
@@ -357,41 +129,322 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void row_item(const RowArgs &a, int it, int &x0, int &z, int &yb, int &ny)
+constexpr int SROWS = 136;                 // voxel rows of 128 bytes in a slot, SUSED of them read
+constexpr int SUSED = 130;
+constexpr uint32_t SBYTES = SROWS * 128;   // a multiple of 1024
+
+// ---- row-ring convolution (cin, cout <= 32) ----------------------------------------
+// Axes: x; the ring axis r (y where X >= 128, else z); the stack axis q (the
+// other one).  A CTA takes items of 128 consecutive positions of the (q, x)
+// line times a run of consecutive r.  The line holds a padding position either
+// side of each q's X voxels unless X is a multiple of 128, so that short x
+// extents fill the 128 rows of an MMA too.
+// Operands use the 128-byte-swizzle K-major layout, the one the tensor core
+// fetches fastest: every shared-memory row is one voxel holding 64 K elements,
+// here the channels of its three q planes (K = dq * cin + ci, zero padded),
+// 16-byte chunk c of row p stored at chunk c ^ (p % 8).  One r of the line (130
+// voxel rows, from position s0 - 1) is a ring slot, filled by 16-byte cp.async
+// (producer warp L % 4 loads slot L).  The A operand of tap dx is the slot
+// shifted by dx rows; dq and the channels are the K steps.  Input r feeds the
+// outputs r+1, r, r-1 (dr = 0, 1, 2): the weights of the three dr taps are
+// stacked along N, so one MMA (M = 128 voxels, N = 3 cout, K = 16) per dx and
+// K step covers all of them; the three targets are consecutive blocks of a
+// TMEM ring of NBLK accumulator blocks (block of output v = NBLK-1 - v mod
+// NBLK, so r+1, r, r-1 are ascending; a wrap splits the MMA).  Accumulation is
+// always on: the epilogue zeroes a block as soon as it has read it.  Weights
+// are resident.  Order of the sums: dr, dx, dq where X >= 128; dr, dq, dx
+// below.
+constexpr int RING = 4;   // ring slots
+constexpr int NBLK = 8;   // TMEM accumulator blocks
+
+struct RowArgs {
+    int X, W;             // voxels and positions per q of the line
+    int R, rs, Q, qs;     // ring and stack axis: extent, voxels between neighbours
+    int ntx, rch, nitems; // line tiles, r per item
+    const bf16 *in, *wpk;
+    EpiP epi;
+    int *err;
+};
+
+constexpr int rows_nkb(int cin) { return (3 * cin + 63) / 64; }
+// resident weights of the row kernel: per dx and K block, 3 cout rows of 128 bytes
+constexpr uint32_t rows_wbytes(int cin, int cout) { return 3u * (uint32_t)rows_nkb(cin) * 3u * (uint32_t)cout * 128u; }
+constexpr uint32_t rows_smem(int cin, int cout)
 {
-    int tx = it % a.ntx, r = it / a.ntx;
-    z = r % a.Z;
-    int yc = r / a.Z;
-    x0 = tx * 128;
-    yb = yc * a.ych;
-    ny = min(a.ych, a.Y - yb);
+    return RING * (uint32_t)rows_nkb(cin) * SBYTES + rows_wbytes(cin, cout) + 1024u;
 }
 
-__global__ void __launch_bounds__(288) k_conv_rows(RowArgs a)
+// barrier slots of k_conv_rows
+constexpr int RF = 0, RE = RING, BRDY = 2 * RING, BFREE = 2 * RING + NBLK, RWB = 2 * RING + 2 * NBLK,
+              RFIN = RWB + 1, RNBAR = RWB + 2;
+
+__device__ __forceinline__ uint32_t blk_of(uint32_t v) { return NBLK - 1 - v % NBLK; }
+
+template <int CIN, int COUT, int ZRING>
+__global__ void __launch_bounds__(288) k_conv_rows(const RowArgs a)
 {
     extern __shared__ uint8_t dsm[];
     __shared__ __align__(8) uint64_t bar[RNBAR];
     __shared__ uint32_t tslot;
     __shared__ int abort_s;
+    constexpr int NKB = rows_nkb(CIN);
+    constexpr int NKG = CIN / 8;           // channel blocks of 8
+    constexpr int NREAL = 3 * NKG;         // real 16-byte chunks per voxel row (3 q planes)
+    constexpr uint32_t SLOT = NKB * SBYTES;
+    constexpr uint32_t NCOLS = NBLK * COUT;
     volatile int *abort_ = &abort_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t sS = (tc::smem_u32(dsm) + 1023u) & ~1023u;   // slab ring
-    const uint32_t sW = sS + ((a.slab_bytes + 1023u) & ~1023u);  // resident stacked weights
+    const uint32_t sS = (tc::smem_u32(dsm) + 1023u) & ~1023u;   // slot ring
+    const uint32_t sW = sS + RING * SLOT;                       // resident stacked weights
     const uint32_t bars = tc::smem_u32(bar);
-    const uint32_t ncols = rows_ncols(a.cout);
-    const int nkg = a.cin >> 3;           // channel blocks of 8
-    const int nreal = 3 * nkg;            // real 16-byte chunks per voxel row (3 z planes)
 
     if (threadIdx.x == 0) {
         abort_s = 0;
         for (int i = 0; i < RNBAR; i++) {
             uint32_t cnt = 1;
-            if (i >= RF && i < RF + RING) cnt = 32;             // the producer warp of the row
-            if (i >= BFREE && i < BFREE + NBLK) cnt = 4;       // epilogue warps
+            if (i >= RF && i < RF + RING) cnt = 32;             // the producer warp of the slot
+            if (i >= BFREE && i < BFREE + NBLK) cnt = 4;        // epilogue warps
             tc::mbar_init(bars + 8 * i, cnt);
         }
+        tc::mbar_fence_init();
+    }
+    if (warp == 8) {
+        tc::tmem_alloc(tc::smem_u32(&tslot), NCOLS);
+        tc::tmem_relinquish();
+    }
+    if (warp >= 4 && warp < 8) {   // K padding chunks of the slots are never loaded: zero them once
+        uint8_t *g = dsm + (sS - tc::smem_u32(dsm));
+        constexpr int NPAD = 8 * NKB - NREAL;
+        for (int i = threadIdx.x - 128; i < RING * SROWS * NPAD; i += 128) {
+            const int c = NREAL + i % NPAD, r = i / NPAD, p = r % SROWS, slot = r / SROWS;
+            *reinterpret_cast<uint4 *>(g + (uint32_t)slot * SLOT + (uint32_t)(c >> 3) * SBYTES + (uint32_t)p * 128u +
+                                       (uint32_t)(((c & 7) ^ (p & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+        tc::fence_proxy_async();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tbase = tslot;
+    if (warp < 4) {   // accumulators start at zero
+        for (uint32_t c = 0; c < NCOLS; c += 16) tmem_st16_zero(tbase + ((uint32_t)(warp * 32) << 16) + c);
+        tmem_wait_st();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+
+    if (warp >= 4 && warp < 8) {
+        // ---- producers
+        const int pw = warp - 4;
+        if (pw == 0 && lane == 0) {
+            tc::mbar_expect_tx(bars + 8 * RWB, rows_wbytes(CIN, COUT));
+            tc::bulk_load(sW, a.wpk, rows_wbytes(CIN, COUT), bars + 8 * RWB);
+        }
+        const uint32_t sbase = sS + (uint32_t)pw * SLOT;
+        uint32_t L = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
+            const int s0 = (it % a.ntx) * 128, rb = (it / a.ntx) * a.rch, nr = min(a.rch, a.R - rb);
+            // this lane's voxel rows: position, plane, which of the planes q-1, q, q+1 exist
+            const bf16 *src[5];
+            uint32_t have[5];
+#pragma unroll
+            for (int i = 0; i < 5; i++) {
+                const int p = lane + 32 * i;
+                int q, x;
+                if (a.W == a.X) {
+                    q = s0 / a.X;
+                    x = s0 - q * a.X - 1 + p;
+                } else {
+                    const int s = s0 - 1 + p;
+                    q = s < 0 ? 0 : s / a.W;
+                    x = s < 0 ? -1 : s - q * a.W - 1;
+                }
+                const bool v = p < SUSED && x >= 0 && x < a.X && q < a.Q;
+                src[i] = a.in + (v ? ((size_t)q * a.qs + x) * 8 : 0);
+                have[i] = v ? (q > 0 ? 1u : 0u) | 2u | (q + 1 < a.Q ? 4u : 0u) : 0u;
+            }
+            for (int j = 0; j < nr + 2; j++, L++) {
+                if ((int)(L & 3u) != pw) continue;
+                if (L >= RING && !tc::mbar_wait(bars + 8 * (RE + pw), ((L / RING) & 1u) ^ 1u, abort_)) {
+                    ok = false;
+                    break;
+                }
+                // chunk c = dq * NKG + cb of voxel row p comes from channel block cb
+                // of plane q + dq - 1; zero outside the grid
+                const int rr = rb - 1 + j;
+                const bool rok = rr >= 0 && rr < a.R;
+                const long long ro = (long long)(rok ? rr : 0) * a.rs;
+#pragma unroll
+                for (int c = 0; c < NREAL; c++) {
+                    constexpr int G = NKG;
+                    const int d = c / G, cb = c % G;
+                    const long long co = ((long long)cb * (long long)a.epi.plane + ro + (long long)(d - 1) * a.qs) * 8;
+                    const uint32_t rdst = sbase + (uint32_t)(c >> 3) * SBYTES + (uint32_t)lane * 128u +
+                                          (uint32_t)(((c & 7) ^ (lane & 7)) << 4);
+#pragma unroll
+                    for (int i = 0; i < 5; i++) {
+                        if (i == 4 && lane >= SUSED - 128) continue;
+                        const bool v = rok && (have[i] >> d & 1u);
+                        cp_async16(rdst + 4096u * i, v ? src[i] + co : a.in, v ? 16u : 0u);
+                    }
+                }
+                cp_async_commit();
+                cp_async_wait<0>();
+                tc::fence_proxy_async();
+                tc::mbar_arrive(bars + 8 * (RF + pw));
+            }
+        }
+        cp_async_wait<0>();
+        if (!ok) fail(abort_, a.err, 3);
+        if (pw == 0 && lane == 0) settle(bars + 8 * RWB, 0);
+    } else if (warp == 8) {
+        if (lane == 0) {
+            constexpr uint32_t WREG = 3u * COUT * 128u;   // weights of one (dx, K block)
+            constexpr uint32_t IDESC0 = tc::idesc_bf16(128, 0, 0, 0);
+            const uint64_t wdesc = sw128_desc(sW), sdesc0 = sw128_desc(sS);
+            uint32_t L = 0, V = 0;
+            bool ok = tc::mbar_wait(bars + 8 * RWB, 0, abort_);
+            // taps k0 .. k0+n-1 of the input slot into n consecutive blocks from b0
+            auto issue = [&](uint32_t slot, uint32_t k0, uint32_t n, uint32_t b0) {
+                const uint32_t idesc = IDESC0 + ((n * COUT >> 3) << 17), dt = tbase + b0 * COUT;
+                const uint64_t ad0 = sdesc0 + slot * (SLOT >> 4), bd0 = wdesc + k0 * (COUT * 128u >> 4);
+#pragma unroll
+                for (int e = 0; e < 9 * (CIN / 16); e++) {
+                    constexpr int NC = CIN / 16;
+                    const int dx = ZRING ? e / NC % 3 : e / (3 * NC), ks = ZRING ? e / (3 * NC) * NC + e % NC : e % (3 * NC);
+                    const uint32_t ao = (uint32_t)(ks >> 2) * SBYTES + (uint32_t)dx * 128u + (uint32_t)(ks & 3) * 32u;
+                    const uint32_t bo = (uint32_t)(dx * NKB + (ks >> 2)) * WREG + (uint32_t)(ks & 3) * 32u;
+                    tc::mma_bf16(dt, ad0 + (ao >> 4), bd0 + (bo >> 4), idesc, 1u);
+                }
+            };
+            for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
+                const int rb = (it / a.ntx) * a.rch, nr = min(a.rch, a.R - rb);
+                for (int j = 0; j < nr + 2; j++, L++) {
+                    if (j < nr) {   // output j is touched for the first time
+                        const uint32_t g = V + (uint32_t)j;
+                        if (!tc::mbar_wait(bars + 8 * (BFREE + blk_of(g)), ((g / NBLK) & 1u) ^ 1u, abort_)) { ok = false; break; }
+                    }
+                    const uint32_t slot = L % RING;
+                    if (!tc::mbar_wait(bars + 8 * (RF + slot), (L / RING) & 1u, abort_)) { ok = false; break; }
+                    tc::fence_after();
+                    // outputs j, j-1, j-2 (k = dr) that exist: taps k0 .. k1-1, their blocks
+                    // ascending from output j - k0 up to a wrap
+                    const uint32_t k0 = j < nr ? 0u : (uint32_t)(j - nr + 1), k1 = j < 2 ? (uint32_t)j + 1u : 3u;
+                    const uint32_t b0 = blk_of(V + (uint32_t)j - k0);
+                    const uint32_t n1 = min(k1 - k0, (uint32_t)NBLK - b0);
+                    issue(slot, k0, n1, b0);
+                    if (n1 < k1 - k0) issue(slot, k0 + n1, k1 - k0 - n1, 0u);
+                    tc::mma_commit(bars + 8 * (RE + slot));                                            // input slot done
+                    if (j >= 2) tc::mma_commit(bars + 8 * (BRDY + blk_of(V + (uint32_t)(j - 2))));     // output j-2 done
+                }
+                V += (uint32_t)nr;
+            }
+            if (!ok) fail(abort_, a.err, 3);
+            tc::mma_commit(bars + 8 * RFIN);
+            settle(bars + 8 * RFIN, 0);
+        }
+    } else if (warp < 4) {
+        // ---- epilogue: read each output's block, zero it, store the voxels
+        const int row = warp * 32 + lane;
+        float bias[COUT / 16][16], hw[16];
+#pragma unroll
+        for (int c = 0; c < COUT; c++) bias[c / 16][c % 16] = a.epi.bias ? a.epi.bias[c] : 0.f;
+#pragma unroll
+        for (int c = 0; c < 16; c++) hw[c] = a.epi.headw ? a.epi.headw[c] : 0.f;
+        const float hb = a.epi.hout ? *a.epi.headb : 0.f;
+        uint32_t V = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
+            const int s = (it % a.ntx) * 128 + row, rb = (it / a.ntx) * a.rch, nr = min(a.rch, a.R - rb);
+            const int q = s / a.W, x = s - q * a.W - (a.W == a.X ? 0 : 1);
+            const bool valid = q < a.Q && x >= 0 && x < a.X;
+            size_t vox = (size_t)q * a.qs + x + (size_t)rb * a.rs;
+            for (int j = 0; j < nr; j++, vox += a.rs) {
+                const uint32_t g = V + (uint32_t)j, b = blk_of(g);
+                if (!__all_sync(0xffffffffu, tc::mbar_wait(bars + 8 * (BRDY + b), (g / NBLK) & 1u, abort_))) { fail(abort_, a.err, 3); ok = false; break; }
+                tc::fence_after();
+                const uint32_t taddr = tbase + ((uint32_t)(warp * 32) << 16) + b * COUT;
+                uint32_t rr[COUT / 16][16];
+#pragma unroll
+                for (int ch = 0; ch < COUT / 16; ch++) tc::tmem_ld16(taddr + (uint32_t)ch * 16u, rr[ch]);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int ch = 0; ch < COUT / 16; ch++) tmem_st16_zero(taddr + (uint32_t)ch * 16u);
+                tmem_wait_st();
+                tc::fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(bars + 8 * (BFREE + b));
+                if (!valid) continue;
+                float hsum = 0.f;
+#pragma unroll
+                for (int ch = 0; ch < COUT / 16; ch++) epilogue16(a.epi, ch, rr[ch], bias[ch], hw, vox, hsum);
+                if (a.epi.hout) a.epi.hout[vox] = hsum + hb;
+            }
+            V += (uint32_t)nr;
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    if (warp == 8) tc::tmem_dealloc(tbase, NCOLS);
+}
+
+// ---- tap-staged convolution (more channels) ------------------------------------------
+// A tile is 128 consecutive positions of the line (z, y, x) with a padding
+// position either side of each x row, and nt of the output channels.  A stage
+// is one (channel chunk, dz, dy): the 130 voxel rows of the line at that offset
+// (up to 64 channels, 128-byte-swizzled K-major rows, zero outside the grid)
+// and the weights of its three dx taps.  The A operand of tap dx is the stage
+// shifted by dx rows, so a voxel row is loaded 9 times instead of 27.  Four
+// producer warps keep two stages in flight behind the one they fill; the
+// accumulator is double buffered.  Order of the sums: chunk, dz, dy, dx, channel.
+struct WideArgs {
+    int X, Y, Z, W;
+    int cin, cout, kc, nkc, nt, nsplit;
+    int ntiles, stages;
+    uint32_t stride;
+    const bf16 *in, *wpk;
+    EpiP epi;
+    int *err;
+};
+constexpr int WSTAGES = 8, WLAG = 2;
+// barrier slots: A full, weights full, stage empty, accumulator full / empty
+constexpr int WFA = 0, WFB = WSTAGES, WE = 2 * WSTAGES, WAF = 3 * WSTAGES, WAE = WAF + 2, WFIN = WAE + 2, WNBAR = WFIN + 1;
+
+// position s of the padded line: voxel (x, y, z); false on a padding position or past the end
+__device__ __forceinline__ bool line_at(int s, int W, int X, int Y, int Z, int &x, int &y, int &z)
+{
+    if (s < 0) { x = y = z = 0; return false; }
+    const int r = s / W;
+    x = s - r * W - 1;
+    z = r / Y;
+    y = r - z * Y;
+    return x >= 0 && x < X && z < Z;
+}
+
+__global__ void __launch_bounds__(288) k_conv_wide(const WideArgs a)
+{
+    extern __shared__ uint8_t dsm[];
+    __shared__ __align__(8) uint64_t bar[WNBAR];
+    __shared__ uint32_t tslot;
+    __shared__ int abort_s;
+    volatile int *abort_ = &abort_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t s0 = (tc::smem_u32(dsm) + 1023u) & ~1023u;
+    const uint32_t bars = tc::smem_u32(bar);
+    uint32_t ncols = 32;
+    while (ncols < 2u * (uint32_t)a.nt) ncols <<= 1;
+    const int nwork = a.ntiles * a.nsplit, nst = 9 * a.nkc;
+
+    if (threadIdx.x == 0) {
+        abort_s = 0;
+        for (int i = 0; i < WNBAR; i++)
+            tc::mbar_init(bars + 8 * i, i < WFB ? 128u : (i == WAE || i == WAE + 1) ? 4u : 1u);
         tc::mbar_fence_init();
     }
     if (warp == 8) {
@@ -402,158 +455,124 @@ __global__ void __launch_bounds__(288) k_conv_rows(RowArgs a)
     __syncthreads();
     tc::fence_after();
     const uint32_t tbase = tslot;
-    if (warp < 4) {   // accumulators start at zero
-        for (int b = 0; b < NBLK; b++)
-            for (int ch = 0; ch < (a.cout >> 4); ch++)
-                tmem_st16_zero(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * a.cout + ch * 16));
-        tmem_wait_st();
-    } else if (warp < 8) {   // K padding chunks of the slab are never loaded: zero them once
-        uint8_t *g = dsm + (sS - tc::smem_u32(dsm));
-        int npad = 8 * a.nkb - nreal;
-        for (int i = threadIdx.x - 128; i < RING * RROWS * npad; i += 128) {
-            int c = nreal + i % npad, r = i / npad, p = r % RROWS, slot = r / RROWS;
-            int kb = c >> 3, cc = c & 7;
-            uint32_t off = (uint32_t)slot * a.slot_bytes + (uint32_t)kb * (RROWS * 128) + (uint32_t)p * 128u +
-                           (uint32_t)((cc ^ (p & 7)) << 4);
-            *reinterpret_cast<uint4 *>(g + off) = make_uint4(0, 0, 0, 0);
-        }
-        tc::fence_proxy_async();
-    }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
+    const uint32_t S = (uint32_t)a.stages;
 
     if (warp >= 4 && warp < 8) {
-        // ---- producers
-        const int pw = warp - 4;
-        if (pw == 0 && lane == 0) {
-            tc::mbar_expect_tx(bars + 8 * RWB, a.wbytes);
-            tc::bulk_load(sW, a.wpk, a.wbytes, bars + 8 * RWB);
-        }
-        uint32_t L = 0;
+        // ---- producers: thread t loads voxel row t; the first 16 also a chunk of rows 128, 129
+        const int t = threadIdx.x - 128;
+        const int p2 = 128 + (t >> 3), c2 = t & 7;
+        uint32_t u = 0, slot = 0, par = 1;          // fills issued; slot u % S and its empty parity
+        uint32_t aslot = 0;                         // slot of the next fill to report
         bool ok = true;
-        for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
-            int x0, z, yb, ny;
-            row_item(a, it, x0, z, yb, ny);
-            for (int j = 0; j < ny + 2; j++, L++) {
-                if ((int)(L & 3u) != pw) continue;
-                uint32_t slot = L % RING;
-                if (L >= RING && !tc::mbar_wait(bars + 8 * (RE + slot), ((L / RING) & 1u) ^ 1u, abort_)) {
-                    ok = false;
-                    break;
+        for (int w = blockIdx.x; ok && w < nwork; w += gridDim.x) {
+            const int tile = w / a.nsplit, n0 = (w - tile * a.nsplit) * a.nt;
+            int x, y, z, x2, y2, z2;
+            const bool v = line_at(tile * 128 - 1 + t, a.W, a.X, a.Y, a.Z, x, y, z);
+            const bool v2 = t < 16 && line_at(tile * 128 - 1 + p2, a.W, a.X, a.Y, a.Z, x2, y2, z2);
+            const long long vox = v ? ((long long)z * a.Y + y) * a.X + x : 0;
+            const long long vox2 = v2 ? ((long long)z2 * a.Y + y2) * a.X + x2 : 0;
+            for (int st = 0; st < nst; st++, u++) {
+                if (!tc::mbar_wait(bars + 8 * (WE + slot), par, abort_)) { ok = false; break; }
+                const int kci = st / 9, e = st - kci * 9, dz = e / 3 - 1, dy = e % 3 - 1;
+                const uint32_t buf = s0 + slot * a.stride;
+                if (t == 0) {   // three dx taps' weights of the nt channels
+                    const uint32_t bytes = (uint32_t)a.nt * 128u;
+                    tc::mbar_expect_tx(bars + 8 * (WFB + slot), 3u * bytes);
+                    for (int dx = 0; dx < 3; dx++)
+                        tc::bulk_load(buf + SBYTES + (uint32_t)dx * bytes,
+                                      a.wpk + ((size_t)(st * 3 + dx) * a.cout + n0) * 64, bytes, bars + 8 * (WFB + slot));
                 }
-                // chunk c = dz * nkg + cb of voxel row p (x = x0 - 1 + p) comes from
-                // channel block cb of plane z + dz - 1; zero outside the grid
-                int yy = yb - 1 + j;
-                bool yok = yy >= 0 && yy < a.Y;
-                uint32_t fullb = bars + 8 * (RF + slot);
-                uint32_t sbase = sS + slot * a.slot_bytes;
-                for (int c = 0; c < nreal; c++) {
-                    int dz = c / nkg, cb = c - dz * nkg, zz = z + dz - 1, kb = c >> 3, cc = c & 7;
-                    bool rok = yok && zz >= 0 && zz < a.Z;
-                    const bf16 *rsrc = a.in + ((((size_t)cb * a.Z + (rok ? zz : 0)) * a.Y + (rok ? yy : 0)) * a.X) * 8;
-                    uint32_t rdst = sbase + (uint32_t)kb * (RROWS * 128);
-                    for (int p = lane; p < RW; p += 32) {
-                        int xg = x0 - 1 + p;
-                        bool v = rok && xg >= 0 && xg < a.X;
-                        cp_async16(rdst + (uint32_t)p * 128u + (uint32_t)((cc ^ (p & 7)) << 4),
-                                   v ? rsrc + (size_t)xg * 8 : a.in, v ? 16u : 0u);
-                    }
+                const int nch = min(a.kc, a.cin - kci * a.kc) >> 3;   // 16-byte chunks of this channel chunk
+                const long long off = ((long long)dz * a.Y + dy) * a.X, cb0 = (long long)kci * (a.kc >> 3);
+                {
+                    const bool in = v && z + dz >= 0 && z + dz < a.Z && y + dy >= 0 && y + dy < a.Y;
+                    const bf16 *src = in ? a.in + (cb0 * (long long)a.epi.plane + vox + off) * 8 : a.in;
+                    const long long step = in ? (long long)a.epi.plane * 8 : 0;
+                    const uint32_t dst = buf + (uint32_t)t * 128u, sw = (uint32_t)(t & 7), n16 = in ? 16u : 0u;
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        if (c < nch) cp_async16(dst + (((uint32_t)c ^ sw) << 4), src + c * step, n16);
+                }
+                if (t < 16 && c2 < nch) {
+                    const bool in = v2 && z2 + dz >= 0 && z2 + dz < a.Z && y2 + dy >= 0 && y2 + dy < a.Y;
+                    cp_async16(buf + (uint32_t)p2 * 128u + (uint32_t)((c2 ^ (p2 & 7)) << 4),
+                               in ? a.in + ((cb0 + c2) * (long long)a.epi.plane + vox2 + off) * 8 : a.in, in ? 16u : 0u);
                 }
                 cp_async_commit();
-                cp_async_wait0();
-                tc::fence_proxy_async();
-                tc::mbar_arrive(fullb);
+                if (u >= WLAG) {
+                    cp_async_wait<WLAG>();
+                    tc::fence_proxy_async();
+                    tc::mbar_arrive(bars + 8 * (WFA + aslot));
+                    if (++aslot == S) aslot = 0;
+                }
+                if (++slot == S) { slot = 0; par ^= 1u; }
             }
         }
-        cp_async_wait0();
-        if (!ok) fail(abort_, a.err, 3);
-        if (pw == 0 && lane == 0) tc::mbar_wait(bars + 8 * RWB, 0, abort_);
+        cp_async_wait<0>();
+        tc::fence_proxy_async();
+        for (uint32_t i = u > WLAG ? u - WLAG : 0u; i < u; i++) {
+            tc::mbar_arrive(bars + 8 * (WFA + aslot));
+            if (++aslot == S) aslot = 0;
+        }
+        if (!ok) fail(abort_, a.err, 1);
+        if (t == 0) drain(bars, WFB, u, (int)S);
     } else if (warp == 8) {
         if (lane == 0) {
-            const uint32_t N3 = 3u * (uint32_t)a.cout;
-            const uint32_t wreg = N3 * 128u;                        // weights of one (dx, K block)
-            const int nks = (3 * a.cin) / 16;                       // K steps of 16 per dx
-            uint32_t L = 0, V = 0;
-            bool ok = tc::mbar_wait(bars + 8 * RWB, 0, abort_);
-            for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
-                int x0, z, yb, ny;
-                row_item(a, it, x0, z, yb, ny);
-                const int nv = ny + 2;   // virtual output rows yb-1 .. yb+ny of this item
-                for (int j = 0; ok && j < nv; j++) {
-                    // blocks touched for the first time: rows j+1 (and j at the start)
-                    for (int v = (j == 0 ? 0 : j + 1); v <= j + 1 && v < nv; v++) {
-                        uint32_t g = V + (uint32_t)v;
-                        if (!tc::mbar_wait(bars + 8 * (BFREE + blk_of(g)), ((g / NBLK) & 1u) ^ 1u, abort_)) { ok = false; break; }
-                    }
-                    uint32_t Lr = L + (uint32_t)j, slot = Lr % RING;
-                    if (!ok || !tc::mbar_wait(bars + 8 * (RF + slot), (Lr / RING) & 1u, abort_)) { ok = false; break; }
+            const uint32_t idesc = tc::idesc_bf16(128, a.nt, 0, 0);
+            const uint32_t bstep = (uint32_t)a.nt * 128u >> 4;
+            uint32_t slot = 0, par = 0, it = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; ok && w < nwork; w += gridDim.x, it++) {
+                const uint32_t ab = it & 1u;
+                if (!tc::mbar_wait(bars + 8 * (WAE + ab), ((it >> 1) & 1u) ^ 1u, abort_)) { ok = false; break; }
+                const uint32_t dt = tbase + ab * (uint32_t)a.nt;
+                for (int st = 0; st < nst; st++) {
+                    if (!tc::mbar_wait(bars + 8 * (WFB + slot), par, abort_) ||
+                        !tc::mbar_wait(bars + 8 * (WFA + slot), par, abort_)) { ok = false; break; }
                     tc::fence_after();
-                    // runs of consecutive valid target blocks among rows j+1, j, j-1 (k = dy)
-                    int kb[3], kv[3];
-                    for (int k = 0; k < 3; k++) {
-                        int row = j + 1 - k;
-                        kv[k] = row >= 0 && row < nv;
-                        kb[k] = kv[k] ? blk_of(V + (uint32_t)row) : -1;
-                    }
-                    const uint32_t sbase = sS + slot * a.slot_bytes;
-                    for (int dx = 0; dx < 3; dx++) {
-                        int k = 0;
-                        while (k < 3) {
-                            if (!kv[k]) { k++; continue; }
-                            int k1 = k + 1;
-                            while (k1 < 3 && kv[k1] && kb[k1] == kb[k1 - 1] + 1) k1++;
-                            uint32_t n = (uint32_t)(k1 - k) * (uint32_t)a.cout;
-                            uint32_t idesc = tc::idesc_bf16(128, (int)n, 0, 0);
-                            uint32_t dt = tbase + (uint32_t)(kb[k] * a.cout);
-                            for (int ks = 0; ks < nks; ks++) {
-                                uint32_t kbk = (uint32_t)(ks >> 2), kk = (uint32_t)(ks & 3);
-                                uint64_t ad = sw128_desc(sbase + kbk * (RROWS * 128) + (uint32_t)dx * 128u + kk * 32u);
-                                uint64_t bd = sw128_desc(sW + ((uint32_t)dx * (uint32_t)a.nkb + kbk) * wreg +
-                                                         (uint32_t)(k * a.cout) * 128u + kk * 32u);
-                                tc::mma_bf16(dt, ad, bd, idesc, 1u);
-                            }
-                            k = k1;
-                        }
-                    }
-                    tc::mma_commit(bars + 8 * (RE + slot));                           // input row done
-                    if (j >= 1) tc::mma_commit(bars + 8 * (BRDY + kb[2]));            // output row j-1 done
+                    const uint64_t ad = sw128_desc(s0 + slot * a.stride), bd = ad + (SBYTES >> 4);
+                    const int nks = min(a.kc, a.cin - st / 9 * a.kc) >> 4;
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                        for (int ks = 0; ks < 4; ks++)
+                            if (ks < nks)
+                                tc::mma_bf16(dt, ad + (uint32_t)(dx * 8 + ks * 2), bd + (uint32_t)dx * bstep + (uint32_t)(ks * 2),
+                                             idesc, (st | dx | ks) != 0);
+                    tc::mma_commit(bars + 8 * (WE + slot));
+                    if (++slot == S) { slot = 0; par ^= 1u; }
                 }
-                if (!ok) break;
-                tc::mma_commit(bars + 8 * (BRDY + blk_of(V + (uint32_t)(nv - 1))));   // partial last row
-                L += (uint32_t)nv;
-                V += (uint32_t)nv;
+                if (ok) tc::mma_commit(bars + 8 * (WAF + ab));
             }
-            if (!ok) fail(abort_, a.err, 3);
-            tc::mma_commit(bars + 8 * RFIN);
-            tc::mbar_wait(bars + 8 * RFIN, 0, abort_);
+            if (!ok) fail(abort_, a.err, 1);
+            tc::mma_commit(bars + 8 * WFIN);
+            settle(bars + 8 * WFIN, 0);
         }
     } else if (warp < 4) {
-        // ---- epilogue: drain each virtual row's block, store the real rows, zero it
-        const int row = warp * 32 + lane;
-        uint32_t V = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; ok && it < a.nitems; it += gridDim.x) {
-            int x0, z, yb, ny;
-            row_item(a, it, x0, z, yb, ny);
-            for (int j = 0; j < ny + 2; j++) {
-                uint32_t g = V + (uint32_t)j;
-                int b = blk_of(g);
-                if (!tc::mbar_wait(bars + 8 * (BRDY + b), (g / NBLK) & 1u, abort_)) { fail(abort_, a.err, 3); ok = false; break; }
-                tc::fence_after();
-                uint32_t taddr = tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * a.cout);
-                if (j >= 1 && j <= ny) {
-                    int gx = x0 + row;
-                    size_t vox = ((size_t)z * a.Y + (yb + j - 1)) * a.X + gx;
-                    epilogue(a.epi, taddr, vox, gx < a.X);
-                }
-                for (int ch = 0; ch < (a.cout >> 4); ch++) tmem_st16_zero(taddr + (uint32_t)ch * 16u);
-                tmem_wait_st();
-                tc::fence_before();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(bars + 8 * (BFREE + b));
+        const float none[16] = {};
+        uint32_t it = 0;
+        for (int w = blockIdx.x; w < nwork; w += gridDim.x, it++) {
+            const int tile = w / a.nsplit, n0 = (w - tile * a.nsplit) * a.nt;
+            int x, y, z;
+            const bool valid = line_at(tile * 128 + warp * 32 + lane, a.W, a.X, a.Y, a.Z, x, y, z);
+            const size_t vox = valid ? ((size_t)z * a.Y + y) * a.X + x : 0;
+            const uint32_t ab = it & 1u;
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(bars + 8 * (WAF + ab), (it >> 1) & 1u, abort_))) { fail(abort_, a.err, 1); break; }
+            tc::fence_after();
+            const uint32_t taddr = tbase + ((uint32_t)(warp * 32) << 16) + ab * (uint32_t)a.nt;
+            float hsum = 0.f;
+            for (int ch = 0; ch < (a.nt >> 4); ch++) {
+                uint32_t rr[16];
+                tc::tmem_ld16(taddr + (uint32_t)ch * 16u, rr);
+                float bias[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) bias[j] = a.epi.bias ? a.epi.bias[n0 + ch * 16 + j] : 0.f;
+                tc::tmem_wait_ld();
+                if (valid) epilogue16(a.epi, (n0 >> 4) + ch, rr, bias, none, vox, hsum);
             }
-            V += (uint32_t)(ny + 2);
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bars + 8 * (WAE + ab));
         }
     }
     tc::fence_before();
@@ -561,6 +580,7 @@ __global__ void __launch_bounds__(288) k_conv_rows(RowArgs a)
     tc::fence_after();
     if (warp == 8) tc::tmem_dealloc(tbase, ncols);
 }
+
 
 // ---- weight gradient --------------------------------------------------------------
 struct WgArgs {
@@ -627,7 +647,7 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorM
                 u++;
             }
             if (!ok) fail(abort_, a.err, 2);
-            drain(bars, F, u, WG_STAGES, abort_);
+            drain(bars, F, u, WG_STAGES);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -803,26 +823,31 @@ __global__ void __launch_bounds__(128) k_umma_selftest(int mn, int swap, unsigne
 }
 
 // ---- weight packing ------------------------------------------------------------------
-// Standard layout (TMA kernel), per (channel chunk, tap) the B operand
-// [kc/8][N][8]:
-//   fwd: wf[((kci*27 + tap)*(kc/8) + kg)*cout + n][e] = W[tap][n][kci*kc + kg*8 + e]
-//   bwd: wd[((kci*27 + tap)*(kcb/8) + kg)*cin + n][e] = W[26 - tap][kci*kcb + kg*8 + e][n]
-// Row-kernel layout (kc = cin): per (dx, 128-byte K block) the rows
-// n' = dy * N + n (three dy taps stacked along N) of 64 K elements
-// K = dz * cin + k, 128-byte swizzled: byte
-//   ((dx * nkb + K / 64) * 3N + n') * 128 + (((K % 64) / 8) ^ (n' % 8)) * 16 + (K % 8) * 2
-__device__ __forceinline__ long long pack_index(int stacked, int kc, int nout, int tap, int n, int k)
+// K elements k of a tap's B operand (rows n of 128 bytes, 128-byte swizzled:
+// 16-byte chunk c of row n at chunk c ^ (n % 8)); W[tap][n][k] forward,
+// W[26 - tap][k][n] for the data gradient.
+// k_conv_wide, per (channel chunk of kc, tap): row n holds k = 0 .. kc-1.
+// k_conv_rows, per (dx, block of 64 K): row dr * N + n, K = dq * cin + k with
+// (r, q) = (y, z) or, zring, (z, y).
+__device__ __forceinline__ long long pack_index(const ConvPlan &p, int kin, int nout, int tap, int n, int k)
 {
-    int kci = k / kc, r = k % kc, kg = r >> 3, e = r & 7;
-    if (!stacked) return ((((long long)kci * 27 + tap) * (kc >> 3) + kg) * nout + n) * 8 + e;
-    int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-    int K = dz * kc + k, kb = K >> 6, k64 = K & 63, np = dy * nout + n, nkb = rows_nkb(kc);
-    long long byte = ((long long)(dx * nkb + kb) * (3 * nout) + np) * 128 + (((k64 >> 3) ^ (np & 7)) << 4) + (k64 & 7) * 2;
-    return byte >> 1;
+    long long row;
+    int k64;
+    if (p.rows) {
+        const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
+        const int K = (p.zring ? dy : dz) * kin + k;
+        row = (long long)(dx * rows_nkb(kin) + (K >> 6)) * (3 * nout) + (p.zring ? dz : dy) * nout + n;
+        k64 = K & 63;
+    } else {
+        const int kci = k / p.kc;
+        row = (long long)(kci * 27 + tap) * nout + n;
+        k64 = k - kci * p.kc;
+    }
+    return row * 64 + (((k64 >> 3) ^ ((int)row & 7)) << 3) + (k64 & 7);
 }
 
-__global__ void k_pack(const float *__restrict__ W, int cin, int cout, int kcf, int kcb, int stf, int stb,
-                       bf16 *__restrict__ wf, bf16 *__restrict__ wd)
+__global__ void k_pack(const float *__restrict__ W, int cin, int cout, ConvPlan pf, ConvPlan pb, bf16 *__restrict__ wf,
+                       bf16 *__restrict__ wd)
 {
     long long n = 27LL * cin * cout;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
@@ -831,8 +856,8 @@ __global__ void k_pack(const float *__restrict__ W, int cin, int cout, int kcf, 
         long long t = idx / cin;
         int co = (int)(t % cout), tap = (int)(t / cout);
         bf16 w = __float2bfloat16_rn(W[idx]);
-        wf[pack_index(stf, kcf, cout, tap, co, ci)] = w;
-        wd[pack_index(stb, kcb, cin, 26 - tap, ci, co)] = w;
+        wf[pack_index(pf, cin, cout, tap, co, ci)] = w;
+        wd[pack_index(pb, cout, cin, 26 - tap, ci, co)] = w;
     }
 }
 
@@ -922,32 +947,10 @@ const char *conv_last_error() { return g_conv_err; }
 ConvPlan conv_plan(int X, int Y, int Z, int cin, int cout)
 {
     ConvPlan p{};
-    p.slab = X >= 128;
-    p.rows = X >= 128 && cin <= 32 && cout <= 32;
-    p.kc = cin < (p.slab ? 32 : 64) ? cin : (p.slab ? 32 : 64);
-    p.nkc = cin / p.kc;
-    if (p.slab) { p.bx = 128; p.by = 1; p.bz = 1; }
-    else tile_dims(X, Y, Z, p.bx, p.by, p.bz);
-    p.nb = p.bx * p.by * p.bz;
-    p.ntx = (X + p.bx - 1) / p.bx; p.nty = (Y + p.by - 1) / p.by; p.ntz = (Z + p.bz - 1) / p.bz;
-    p.ntiles = p.ntx * p.nty * p.ntz;
-    p.wbytes = 27u * cin * cout * 2u;
-    p.wres = p.wbytes <= 65536u;
-    p.sa = 4; p.sb = 4;
-    if (p.slab) {
-        p.abytes = 8u * (p.bx + 2) * 3u * 3u * (p.kc / 8) * 2u;
-        p.a_lbo = (uint32_t)(p.bx + 2) * 9u * 16u;
-    } else {
-        p.abytes = (uint32_t)p.nb * p.kc * 2u;
-        p.a_lbo = (uint32_t)p.nb * 16u;
-    }
-    // a stage always spans 128 rows per 8 channels so that the MMA reads stay in it
-    p.astride = r1024(p.abytes > 256u * p.kc ? p.abytes : 256u * p.kc);
-    p.bbytes = (uint32_t)p.kc * cout * 2u;
-    p.bstride = r1024(p.bbytes);
-    uint32_t na = p.slab ? 2u : (uint32_t)p.sa;
-    p.smem = na * p.astride + (p.wres ? r1024(p.wbytes) : (uint32_t)p.sb * p.bstride) + 1024u;
-    p.ncols = cout * 2 < 32 ? 32 : cout * 2;
+    p.rows = cin <= 32 && cout <= 32;
+    p.zring = X < 128;
+    const int most = X < 128 ? 64 : 32;
+    p.kc = cin < most ? cin : most;
     return p;
 }
 
@@ -956,59 +959,70 @@ void conv_pack_weights(cudaStream_t s, const float *W, int cin, int cout, const 
 {
     long long n = 27LL * cin * cout;
     int nb = (int)((n + 255) / 256);
-    k_pack<<<nb < 2048 ? nb : 2048, 256, 0, s>>>(W, cin, cout, pf.kc, pb.kc, pf.rows, pb.rows, wf, wd);
+    k_pack<<<nb < 2048 ? nb : 2048, 256, 0, s>>>(W, cin, cout, pf, pb, wf, wd);
 }
+
+namespace {
+
+template <int CIN, int COUT, int ZRING>
+int launch_rows(cudaStream_t s, RowArgs r, int nsm)
+{
+    constexpr uint32_t smem = rows_smem(CIN, COUT);
+    static int lim = dyn_smem_limit((const void *)k_conv_rows<CIN, COUT, ZRING>);
+    if ((int)smem > lim) { snprintf(g_conv_err, sizeof(g_conv_err), "conv rows needs %u B of shared memory", smem); return 1; }
+    const int most = nsm * ctas_per_sm(smem, NBLK * COUT);
+    // an item of rch costs rch + 2 inputs: up to 32, fewer where that leaves
+    // CTAs without two items; below 4 only where CTAs would have none
+    const long long lines = (long long)r.ntx * r.R;
+    r.rch = 32;
+    while ((r.rch > 4 && lines / r.rch < 2LL * most) || (r.rch > 1 && lines / r.rch < most)) r.rch >>= 1;
+    r.nitems = r.ntx * ((r.R + r.rch - 1) / r.rch);
+    k_conv_rows<CIN, COUT, ZRING><<<most < r.nitems ? most : r.nitems, 288, smem, s>>>(r);
+    return launch_error("k_conv_rows");
+}
+
+template <int ZRING>
+int launch_rows(cudaStream_t s, const RowArgs &r, int cin, int cout, int nsm)
+{
+    if (cin == 16) return cout == 16 ? launch_rows<16, 16, ZRING>(s, r, nsm) : launch_rows<16, 32, ZRING>(s, r, nsm);
+    return cout == 16 ? launch_rows<32, 16, ZRING>(s, r, nsm) : launch_rows<32, 32, ZRING>(s, r, nsm);
+}
+
+}  // namespace
 
 int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int cout, const bf16 *wpk,
               const ConvEpi &e, int *err, int nsm)
 {
     if (cin % 16 || cout % 16 || cout > 128 || cin > 128) { snprintf(g_conv_err, sizeof(g_conv_err), "conv channels"); return 1; }
-    ConvPlan p = conv_plan(X, Y, Z, cin, cout);
-    CUtensorMap map;
-    int rc = p.slab ? make_map(&map, in, X, Y, Z, cin, p.bx + 2, 3, 3, p.kc / 8)
-                    : make_map(&map, in, X, Y, Z, cin, p.bx, p.by, p.bz, p.kc / 8);
-    if (rc) return 1;
-    ConvArgs a{};
-    a.X = X; a.Y = Y; a.Z = Z; a.cin = cin; a.cout = cout; a.kc = p.kc; a.nkc = p.nkc;
-    a.slab = p.slab; a.bx = p.bx; a.by = p.by; a.bz = p.bz; a.ntx = p.ntx; a.nty = p.nty; a.ntz = p.ntz;
-    a.ntiles = p.ntiles; a.wres = p.wres; a.sa = p.sa; a.sb = p.sb;
-    a.abytes = p.abytes; a.bbytes = p.bbytes; a.astride = p.astride; a.bstride = p.bstride; a.wbytes = p.wbytes;
-    a.a_lbo = p.a_lbo; a.wpk = wpk;
-    a.bias = e.bias; a.relu = e.relu; a.skip = e.skip; a.mask = e.mask; a.out = e.out;
-    a.headw = e.headw; a.headb = e.headb; a.hout = e.hout; a.err = err;
+    const ConvPlan p = conv_plan(X, Y, Z, cin, cout);
+    const EpiP epi{e.bias, e.relu, e.mask, e.out, e.headw, e.headb, e.hout, (size_t)X * Y * Z};
     if (p.rows) {
         RowArgs r{};
-        r.X = X; r.Y = Y; r.Z = Z; r.cin = cin; r.cout = cout;
-        r.ntx = (X + 127) / 128;
-        r.nkb = rows_nkb(cin);
-        r.slot_bytes = (uint32_t)r.nkb * RROWS * 128u;
-        r.slab_bytes = RING * r.slot_bytes;
-        r.wbytes = rows_wbytes(cin, cout);
-        r.in = in; r.wpk = wpk;
-        r.epi = EpiP{e.bias, e.relu, e.skip, e.mask, e.out, e.headw, e.headb, e.hout, cout, (size_t)X * Y * Z};
-        r.err = err;
-        uint32_t smem = ((r.slab_bytes + 1023u) & ~1023u) + ((r.wbytes + 1023u) & ~1023u) + 1024u;
-        static int rlim = dyn_smem_limit((const void *)k_conv_rows);
-        if ((int)smem > rlim) { snprintf(g_conv_err, sizeof(g_conv_err), "conv rows needs %u B of shared memory", smem); return 1; }
-        int bps = ctas_per_sm(smem, (int)rows_ncols(cout));
-        int grid = nsm * bps;
-        // rows per item: up to 32, fewer when that leaves CTAs without two items
-        long long rows = (long long)r.ntx * Z * Y;
-        r.ych = 32;
-        while (r.ych > 4 && rows / r.ych < 2LL * grid) r.ych >>= 1;
-        r.nyc = (Y + r.ych - 1) / r.ych;
-        r.nitems = r.ntx * Z * r.nyc;
-        if (grid > r.nitems) grid = r.nitems;
-        k_conv_rows<<<grid, 288, smem, s>>>(r);
-        return launch_error("k_conv_rows");
+        r.X = X;
+        r.W = X % 128 ? X + 2 : X;
+        r.R = p.zring ? Z : Y; r.rs = p.zring ? X * Y : X;
+        r.Q = p.zring ? Y : Z; r.qs = p.zring ? X : X * Y;
+        r.ntx = (int)(((long long)r.Q * r.W + 127) / 128);
+        r.in = in; r.wpk = wpk; r.epi = epi; r.err = err;
+        return p.zring ? launch_rows<1>(s, r, cin, cout, nsm) : launch_rows<0>(s, r, cin, cout, nsm);
     }
-    static int lim = dyn_smem_limit((const void *)k_conv);
-    if ((int)p.smem > lim) { snprintf(g_conv_err, sizeof(g_conv_err), "conv needs %u B of shared memory", p.smem); return 1; }
-    int bps = ctas_per_sm(p.smem, p.ncols);
-    int grid = nsm * bps;
-    if (grid > p.ntiles) grid = p.ntiles;
-    k_conv<<<grid, 192, p.smem, s>>>(map, a);
-    return launch_error("k_conv");
+    WideArgs a{};
+    a.X = X; a.Y = Y; a.Z = Z; a.W = X + 2;
+    a.cin = cin; a.cout = cout; a.kc = p.kc; a.nkc = (cin + p.kc - 1) / p.kc;
+    a.ntiles = (int)(((long long)Z * Y * a.W + 127) / 128);
+    // output channels per CTA: halved while that still gives every CTA an SM of its own
+    a.nt = cout;
+    while (a.nt % 32 == 0 && (long long)a.ntiles * (cout / a.nt) * 2 <= nsm) a.nt >>= 1;
+    a.nsplit = cout / a.nt;
+    a.stride = SBYTES + 3u * (uint32_t)a.nt * 128u;
+    a.in = in; a.wpk = wpk; a.epi = epi; a.err = err;
+    static int lim = dyn_smem_limit((const void *)k_conv_wide);
+    a.stages = (lim - 1024) / (int)a.stride;
+    if (a.stages > WSTAGES) a.stages = WSTAGES;
+    if (a.stages <= WLAG) { snprintf(g_conv_err, sizeof(g_conv_err), "conv needs %u B of shared memory a stage", a.stride); return 1; }
+    const int nwork = a.ntiles * a.nsplit;
+    k_conv_wide<<<nsm < nwork ? nsm : nwork, 288, (uint32_t)a.stages * a.stride + 1024u, s>>>(a);
+    return launch_error("k_conv_wide");
 }
 
 int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int Z, int cin, int cout, float *dw,

@@ -3,10 +3,9 @@
 //
 // Activation layout ("channel-blocked"): a tensor of C channels on an
 // X x Y x Z voxel grid is stored as [C/8][Z][Y][X][8] BF16, i.e. C/8 planes
-// of 16-byte vectors.  A TMA box of 8 x bx x by x bz x kc/8 elements lands in
-// shared memory as [kc/8][voxel][8], which is directly a tcgen05 operand:
-// K-major (channels = K) for the forward and data-gradient convolutions, and
-// MN-major (voxels = K) for the weight gradient.
+// of 16-byte vectors: 16-byte copies build the K-major operand rows of the
+// forward and data-gradient convolutions, and a TMA box lands in shared memory
+// as [kc/8][voxel][8], the MN-major operand (voxels = K) of the weight gradient.
 #pragma once
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -14,26 +13,19 @@
 
 typedef __nv_bfloat16 bf16;
 
-// how one convolution on one grid is tiled
+// which kernel runs one convolution on one grid, and its weight layout
 struct ConvPlan {
-    int slab;                 // 1: 128-voxel x rows, one halo slab per channel chunk
-    int rows;                 // 1: row-ring kernel (cp.async rows, resident weights)
-    int kc, nkc;              // channels per K chunk, number of chunks
-    int bx, by, bz, nb;       // output tile (nb = bx*by*bz <= 128 voxels)
-    int ntx, nty, ntz, ntiles;
-    int wres;                 // all weights resident in shared memory
-    int sa, sb;               // A / B pipeline stages
-    uint32_t abytes, bbytes, astride, bstride, wbytes, a_lbo, smem;
-    int ncols;                // TMEM columns (2 accumulators)
+    int rows;    // 1: row-ring kernel (cin, cout <= 32), else the tap-staged one
+    int zring;   // row-ring kernel: the ring runs along z (X < 128), else along y
+    int kc;      // tap-staged kernel: channels per K chunk
 };
 ConvPlan conv_plan(int X, int Y, int Z, int cin, int cout);
 
-// Epilogue options of a convolution: out = mask?( relu?( acc + bias + skip ) )
-// and, for a 16-channel output, an optional 1x1x1 head hout = headw . out + headb
+// Epilogue options of a convolution: out = mask?( relu?( acc + bias ) )
+// and, for at most 16 channels in and out, an optional 1x1x1 head hout = headw . out + headb
 struct ConvEpi {
     const float *bias = nullptr;
     int relu = 0;
-    const bf16 *skip = nullptr;
     const bf16 *mask = nullptr;
     bf16 *out = nullptr;
     const float *headw = nullptr;
@@ -47,13 +39,13 @@ struct ConvEpi {
 void conv_pack_weights(cudaStream_t s, const float *W, int cin, int cout, const ConvPlan &pf, const ConvPlan &pb,
                        bf16 *wf, bf16 *wd);
 
-// elements of a weight pack buffer for a conv of (cin, cout) on any grid
-// (the row kernel's layout pads K to 128-byte rows); buffers start zeroed
+// elements of a weight pack buffer for a conv of (cin, cout) on any grid (both
+// layouts pad K to 128-byte rows); buffers start zeroed
 inline long long conv_pack_elems(int cin, int cout)
 {
-    long long std = 27LL * cin * cout;
+    long long wide = 27LL * ((cin + 31) / 32) * cout * 64;
     long long rows = 3LL * ((3 * cin + 63) / 64) * 3 * cout * 64;
-    return std > rows ? std : rows;
+    return wide > rows ? wide : rows;
 }
 
 int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int cout, const bf16 *wpk,
