@@ -43,3 +43,33 @@ def test_conv_tiles(X, Y, Z, cin, cout):
         # one BF16 rounding; FP32 sums of at most 3456 exact products
         assert np.all(np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(ref).max())
         assert bool((buf[:64] == 7).all()) and bool((buf[64 + n:] == 7).all())
+
+
+@pytest.mark.parametrize("shift", range(8))
+def test_umma_swizzle128_mn_row_shift(shift):
+    from turbins_gb300 import build
+    build.build()
+    from turbins_gb300 import net as N
+    assert N.selftest_umma(3, shift) == 0
+
+
+@pytest.mark.parametrize("X,Y,Z,cin,cout", [(16, 1, 1, 16, 16), (8, 2, 3, 32, 32), (64, 7, 9, 16, 16), (62, 8, 21, 16, 32),
+                                            (128, 5, 3, 16, 16), (256, 3, 2, 32, 32), (160, 4, 5, 32, 16)])
+def test_wgrad_tiles(X, Y, Z, cin, cout):
+    from turbins_gb300 import build
+    build.build()
+    from turbins_gb300 import net as N
+    rng = np.random.default_rng(X + 5 * Y + cout)
+    x, dy = (U.bf16_round(rng.normal(size=(c, Z, Y, X))) for c in (cin, cout))
+    dw = torch.zeros((27, cout, cin), dtype=torch.float32, device="cuda")
+    try:
+        N.conv3_wgrad(X, Y, Z, cin, cout, _dev(x), _dev(dy), dw)
+    except RuntimeError:
+        # voxel tiles that are no multiple of 16 are refused
+        bx = min(X, 128)
+        by = min(Y, 128 // bx)
+        assert bx * by * min(Z, 128 // (bx * by)) % 16
+        return
+    # FP32 sums of exact BF16 products: bounded by the sum of |terms|
+    bound = 1e-5 * U.conv3_wgrad(np.abs(x), np.abs(dy)) + 1e-6
+    assert np.all(np.abs(dw.cpu().numpy() - U.conv3_wgrad(x, dy)) <= bound)

@@ -114,6 +114,13 @@ __host__ __device__ inline uint64_t sw128_desc(uint32_t saddr)
     return tc::sdesc(saddr, 16, 1024) | (2ull << 61);
 }
 
+// 128-byte-swizzle MN-major operand: rows of 64 M (or N) elements, one K each;
+// the next 64 elements `atom` bytes on
+__host__ __device__ inline uint64_t mn128_desc(uint32_t saddr, uint32_t atom)
+{
+    return tc::sdesc(saddr, atom, 1024) | (2ull << 61);
+}
+
 __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr)
 {
     asm volatile(
@@ -701,6 +708,176 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorM
     if (warp == 1) tc::tmem_dealloc(tbase, ncols);
 }
 
+// ---- weight gradient, few channels (cin, cout <= 32) ---------------------------------
+// dW[tap][co][ci] by steps of RA rows of x of a 128-position line tile (lines,
+// ring axis r and stack axis q as in k_conv_rows).  Both operands are
+// MN-major, 128-byte swizzled: a shared-memory row is one voxel (K), holding
+// for A the channels of its three q planes of each of the RA rows (M =
+// (row, dq, ci), 128 with padding), for B the gradients of the rows around
+// them (N = (t, co), t = 0 .. RA + 1 from the row before the first).  Tap dx is
+// a shift of A by dx rows, so a step is 3 x 8 MMAs, one accumulator per dx; row
+// a and t belong to tap dr = a - t + 2.  A box per tap of an unswizzled layout
+// (k_wgrad) loads a 16-byte voxel row per cycle and 27 of them per voxel:
+// 141 us at 128x64x64, 16 -> 16 channels, against 33 us here; 37, 41 and 26 us
+// against 13, 17 and 18 us for 32 -> 16, 32 -> 32 and 16 -> 32 at 64x32x32.
+template <int CIN>
+struct WgR {
+    static constexpr int RA = CIN == 16 ? 2 : 1, NB = RA + 2;   // rows of x and of dy a step holds
+};
+struct WgRowArgs {
+    int X, W, R, rs, Q, qs, cstep;   // cstep: voxels of the grid (between channel blocks)
+    int ntx, nsteps, zring;
+    const bf16 *x, *dy;
+    float *dw;
+    int *err;
+};
+constexpr int WRS = 3;   // stages
+constexpr int wgr_batoms(int cin, int cout) { return ((cin == 16 ? 4 : 3) * cout + 63) / 64; }
+constexpr uint32_t wgr_stage(int cin, int cout) { return 2u * SBYTES + (uint32_t)wgr_batoms(cin, cout) * 16384u; }
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
+{
+    constexpr int RA = WgR<CIN>::RA, NB = WgR<CIN>::NB, N = NB * COUT, GA = CIN / 8, GB = COUT / 8;
+    constexpr uint32_t STAGE = wgr_stage(CIN, COUT), NCOLS = 3 * N <= 256 ? 256 : 512;
+    constexpr int FA_ = 0, EM_ = WRS, DONE = 2 * WRS, NB_ = DONE + 1;
+    extern __shared__ uint8_t dsm[];
+    __shared__ __align__(8) uint64_t bar[NB_];
+    __shared__ uint32_t tslot;
+    __shared__ int abort_s;
+    volatile int *abort_ = &abort_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t s0 = (tc::smem_u32(dsm) + 1023u) & ~1023u;
+    const uint32_t bars = tc::smem_u32(bar);
+    if (threadIdx.x == 0) {
+        abort_s = 0;
+        for (int i = 0; i < NB_; i++) tc::mbar_init(bars + 8 * i, i < WRS ? 128u : 1u);
+        tc::mbar_fence_init();
+    }
+    if (warp == 8) {
+        tc::tmem_alloc(tc::smem_u32(&tslot), NCOLS);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tbase = tslot;
+    const int nrow = (a.R + RA - 1) / RA;   // steps per line tile
+
+    if (warp >= 4 && warp < 8) {
+        // ---- producers: thread t loads voxel row t of both operands; the first
+        // also a chunk of A's rows 128, 129
+        constexpr int CA = RA * 3 * GA, CB = NB * GB;   // chunks of a voxel row
+        const int t = threadIdx.x - 128;
+        const int p2 = 128 + t / CA, e2 = t % CA;
+        uint32_t u = 0, slot = 0, par = 1, aslot = 0;
+        bool ok = true;
+        auto place = [&](int s, int &q, int &x) {
+            if (a.W == a.X) { q = s < 0 ? -1 : s / a.X; x = s - q * a.X; }
+            else { q = s < 0 ? -1 : s / a.W; x = s - q * a.W - 1; }
+            return q >= 0 && q < a.Q && x >= 0 && x < a.X;
+        };
+        for (int w = blockIdx.x; w < a.nsteps; w += gridDim.x, u++) {
+            if (!tc::mbar_wait(bars + 8 * (EM_ + slot), par, abort_)) { ok = false; break; }
+            const int tile = w / nrow, r0 = (w - tile * nrow) * RA, line0 = tile * 128;
+            const uint32_t buf = s0 + slot * STAGE;
+            int q, x, q2, x2, qb, xb;
+            bool v = place(line0 - 1 + t, q, x), v2 = t < 2 * CA && place(line0 - 1 + p2, q2, x2);
+            const bool vb = place(line0 + t, qb, xb);
+            if (a.W == a.X) {   // a tile lies within one q: its halo positions are outside the grid or in it
+                const int qt = line0 / a.X, xt = line0 - qt * a.X;
+                q = qt; x = xt - 1 + t; v = x >= 0 && x < a.X;
+                q2 = qt; x2 = xt - 1 + p2; v2 = t < 2 * CA && x2 < a.X;
+            }
+            auto load_a = [&](int p, int e, bool pv, int pq, int px) {
+                const int ra = e / (3 * GA), d = e / GA % 3, cb = e % GA, rr = r0 + ra, qq = pq + d - 1;
+                const bool in = pv && rr < a.R && qq >= 0 && qq < a.Q;
+                // M index of the chunk: row a at 64 a where two rows share an operand
+                const int k8 = (RA == 2 ? ra * 8 : 0) + d * GA + cb;
+                const uint32_t dst = buf + (uint32_t)(k8 >> 3) * SBYTES + (uint32_t)p * 128u + (uint32_t)(((k8 & 7) ^ (p & 7)) << 4);
+                cp_async16(dst, in ? a.x + ((long long)cb * a.cstep + (long long)rr * a.rs + (long long)qq * a.qs + px) * 8 : a.x,
+                           in ? 16u : 0u);
+            };
+#pragma unroll
+            for (int e = 0; e < CA; e++) load_a(t, e, v, q, x);
+            if (t < 2 * CA) load_a(p2, e2, v2, q2, x2);
+#pragma unroll
+            for (int e = 0; e < CB; e++) {
+                const int tt = e / GB, cb = e % GB, rr = r0 - 1 + tt;
+                const bool in = vb && rr >= 0 && rr < a.R;
+                const uint32_t dst = buf + 2u * SBYTES + (uint32_t)(e >> 3) * 16384u + (uint32_t)t * 128u +
+                                     (uint32_t)(((e & 7) ^ (t & 7)) << 4);
+                cp_async16(dst, in ? a.dy + ((long long)cb * a.cstep + (long long)rr * a.rs + (long long)qb * a.qs + xb) * 8 : a.dy,
+                           in ? 16u : 0u);
+            }
+            cp_async_commit();
+            if (u >= 1) {
+                cp_async_wait<1>();
+                tc::fence_proxy_async();
+                tc::mbar_arrive(bars + 8 * (FA_ + aslot));
+                if (++aslot == WRS) aslot = 0;
+            }
+            if (++slot == WRS) { slot = 0; par ^= 1u; }
+        }
+        cp_async_wait<0>();
+        tc::fence_proxy_async();
+        if (u > 0) tc::mbar_arrive(bars + 8 * (FA_ + aslot));
+        if (!ok) fail(abort_, a.err, 2);
+    } else if (warp == 8) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16(128, N, 1, 1);
+            uint32_t slot = 0, par = 0, u = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; w < a.nsteps; w += gridDim.x, u++) {
+                if (!tc::mbar_wait(bars + 8 * (FA_ + slot), par, abort_)) { ok = false; break; }
+                tc::fence_after();
+                const uint32_t buf = s0 + slot * STAGE;
+                const uint64_t ad = mn128_desc(buf, SBYTES), bd = mn128_desc(buf + 2u * SBYTES, 16384u);
+#pragma unroll
+                for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                    for (int ks = 0; ks < 8; ks++)
+                        tc::mma_bf16(tbase + (uint32_t)(dx * N), ad + (uint32_t)(dx * 8 + ks * 128), bd + (uint32_t)(ks * 128),
+                                     idesc, u > 0 || ks > 0);
+                tc::mma_commit(bars + 8 * (EM_ + slot));
+                if (++slot == WRS) { slot = 0; par ^= 1u; }
+            }
+            if (!ok) fail(abort_, a.err, 2);
+            tc::mma_commit(bars + 8 * DONE);
+            settle(bars + 8 * DONE, 0);
+        }
+    } else {
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(bars + 8 * DONE, 0, abort_))) {
+            fail(abort_, a.err, 2);
+        } else {
+            tc::fence_after();
+            const int row = warp * 32 + lane;
+            const int ra = RA == 2 ? row >> 6 : 0, m = RA == 2 ? row & 63 : row, dq = m / CIN, ci = m % CIN;
+            const bool valid = dq < 3 && !*abort_;
+            for (int dx = 0; dx < 3; dx++)
+                for (int t = 0; t < NB; t++) {
+                    const int dr = ra - t + 2;
+                    if (dr < 0 || dr > 2) continue;
+                    const int tap = a.zring ? dr * 9 + dq * 3 + dx : dq * 9 + dr * 3 + dx;
+                    for (int ch = 0; ch < COUT / 16; ch++) {
+                        uint32_t rr[16];
+                        tc::tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dx * N + t * COUT + ch * 16), rr);
+                        tc::tmem_wait_ld();
+                        if (valid)
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                atomicAdd(a.dw + ((size_t)tap * COUT + ch * 16 + j) * CIN + ci, __uint_as_float(rr[j]));
+                        __syncwarp();
+                    }
+                }
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    if (warp == 8) tc::tmem_dealloc(tbase, NCOLS);
+}
+
 // ---- descriptor self-test ------------------------------------------------------------
 // One CTA: A (128 x 32) and B (64 x 32) written by the threads into shared
 // memory in a K-major or MN-major core-matrix layout, two MMAs (K = 16 each)
@@ -720,6 +897,8 @@ __device__ __forceinline__ float st_b(int n, int k) { return (float)(((n * 5 + k
 // four MMAs advancing 32 bytes; A starts `swap` (0..7) rows into a 136-row
 // tile.  The swizzle is applied to absolute shared-memory address bits, so a
 // start that is not 1024-byte aligned needs no base offset (field left 0).
+// mn = 3: both operands in the 128-byte-swizzle MN-major layout (rows of 64 M
+// or N elements, one per K), A of two atoms starting `swap` K rows in.
 constexpr int SW_K = 64;
 __device__ __forceinline__ float sw_a(int p, int k) { return (float)(((p * 5 + k * 3) % 11) - 5) * 0.25f; }
 
@@ -756,13 +935,25 @@ __global__ void __launch_bounds__(128) k_umma_selftest(int mn, int swap, unsigne
             *reinterpret_cast<bf16 *>(g0 + offB + off) = __float2bfloat16_rn(st_b(n, k));
         }
     }
-    for (int i = threadIdx.x; mn != 2 && i < ST_M * ST_K; i += blockDim.x) {
+    if (mn == 3) {
+        for (int i = threadIdx.x; i < 40 * ST_M; i += blockDim.x) {
+            int p = i / ST_M, m = i % ST_M;
+            uint32_t off = (uint32_t)((m >> 6) * 8192 + p * 128 + ((((m & 63) >> 3) ^ (p & 7)) << 4) + (m & 7) * 2);
+            *reinterpret_cast<bf16 *>(g0 + off) = __float2bfloat16_rn(sw_a(p, m));
+        }
+        for (int i = threadIdx.x; i < ST_K * ST_N; i += blockDim.x) {
+            int k = i / ST_N, n = i % ST_N;
+            uint32_t off = (uint32_t)(k * 128 + (((n >> 3) ^ (k & 7)) << 4) + (n & 7) * 2);
+            *reinterpret_cast<bf16 *>(g0 + offB + off) = __float2bfloat16_rn(st_b(n, k));
+        }
+    }
+    for (int i = threadIdx.x; mn < 2 && i < ST_M * ST_K; i += blockDim.x) {
         int m = i / ST_K, k = i % ST_K;
         uint32_t off = mn ? (uint32_t)((m / 8) * (ST_K * 16) + (k / 8) * 128 + (k % 8) * 16 + (m % 8) * 2)
                           : (uint32_t)((k / 8) * (ST_M * 16) + (m / 8) * 128 + (m % 8) * 16 + (k % 8) * 2);
         *reinterpret_cast<bf16 *>(g0 + off) = __float2bfloat16_rn(st_a(m, k));
     }
-    for (int i = threadIdx.x; mn != 2 && i < ST_N * ST_K; i += blockDim.x) {
+    for (int i = threadIdx.x; mn < 2 && i < ST_N * ST_K; i += blockDim.x) {
         int n = i / ST_K, k = i % ST_K;
         uint32_t off = mn ? (uint32_t)((n / 8) * (ST_K * 16) + (k / 8) * 128 + (k % 8) * 16 + (n % 8) * 2)
                           : (uint32_t)((k / 8) * (ST_N * 16) + (n / 8) * 128 + (n % 8) * 16 + (k % 8) * 2);
@@ -782,6 +973,12 @@ __global__ void __launch_bounds__(128) k_umma_selftest(int mn, int swap, unsigne
             uint64_t bd = tc::sdesc(bb, 16, 1024) | (2ull << 61);
             tc::mma_bf16(tbase, ad, bd, idesc, ks > 0);
         }
+        tc::mma_commit(tc::smem_u32(bar));
+    } else if (threadIdx.x == 0 && mn == 3) {
+        uint32_t idesc = tc::idesc_bf16(ST_M, ST_N, 1, 1);
+        for (int ks = 0; ks < ST_K / 16; ks++)
+            tc::mma_bf16(tbase, mn128_desc(s0 + ((uint32_t)swap & 7u) * 128u + (uint32_t)ks * 2048u, 8192u),
+                         mn128_desc(s0 + offB + (uint32_t)ks * 2048u, 8192u), idesc, ks > 0);
         tc::mma_commit(tc::smem_u32(bar));
     } else if (threadIdx.x == 0 && swap != 2) {
         // (K-group stride, M/N-group stride) of the layouts written above
@@ -809,6 +1006,8 @@ __global__ void __launch_bounds__(128) k_umma_selftest(int mn, int swap, unsigne
             float ref = 0.f;
             if (mn == 2) {
                 for (int k = 0; k < SW_K; k++) ref += sw_a(row + (swap & 7), k) * st_b(n, k);
+            } else if (mn == 3) {
+                for (int k = 0; k < ST_K; k++) ref += sw_a(k + (swap & 7), row) * st_b(n, k);
             } else {
                 for (int k = 0; k < ST_K; k++) ref += st_a(row, k) * st_b(n, k);
             }
@@ -1025,6 +1224,21 @@ int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int 
     return launch_error("k_conv_wide");
 }
 
+namespace {
+
+template <int CIN, int COUT>
+int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm)
+{
+    constexpr uint32_t smem = WRS * wgr_stage(CIN, COUT) + 1024u;
+    static int lim = dyn_smem_limit((const void *)k_wgrad_rows<CIN, COUT>);
+    if ((int)smem > lim) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad needs %u B of shared memory", smem); return 1; }
+    r.nsteps = r.ntx * ((r.R + WgR<CIN>::RA - 1) / WgR<CIN>::RA);
+    k_wgrad_rows<CIN, COUT><<<nsm < r.nsteps ? nsm : r.nsteps, 288, smem, s>>>(r);
+    return launch_error("k_wgrad_rows");
+}
+
+}  // namespace
+
 int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int Z, int cin, int cout, float *dw,
                 int *err, int nsm)
 {
@@ -1033,6 +1247,19 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
     tile_dims(X, Y, Z, a.bx, a.by, a.bz);
     a.nb = a.bx * a.by * a.bz;
     if (a.nb % 16) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad grid below 16 voxels"); return 1; }
+    if (cin <= 32 && cout <= 32) {
+        WgRowArgs r{};
+        r.zring = X < 128;
+        r.X = X;
+        r.W = X % 128 ? X + 2 : X;
+        r.R = r.zring ? Z : Y; r.rs = r.zring ? X * Y : X;
+        r.Q = r.zring ? Y : Z; r.qs = r.zring ? X : X * Y;
+        r.cstep = X * Y * Z;
+        r.ntx = (int)(((long long)r.Q * r.W + 127) / 128);
+        r.x = x; r.dy = dy; r.dw = dw; r.err = err;
+        if (cin == 16) return cout == 16 ? launch_wgrad_rows<16, 16>(s, r, nsm) : launch_wgrad_rows<16, 32>(s, r, nsm);
+        return cout == 16 ? launch_wgrad_rows<32, 16>(s, r, nsm) : launch_wgrad_rows<32, 32>(s, r, nsm);
+    }
     a.X = X; a.Y = Y; a.Z = Z; a.cin = cin; a.cout = cout;
     a.G = 128 / cin; a.ngroups = (27 + a.G - 1) / a.G;
     a.ntx = (X + a.bx - 1) / a.bx; a.nty = (Y + a.by - 1) / a.by; a.ntz = (Z + a.bz - 1) / a.bz;
