@@ -28,6 +28,7 @@
 
 #include "tc_ptx.cuh"
 #include "turb_conv.cuh"
+#include "turb_internal.cuh"
 
 namespace {
 
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(288) k_conv_rows(const RowArgs a)
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
+    pdl_trigger();   // with the TMEM taken: the next kernel's blocks wait for what is left of it
     const uint32_t tbase = tslot;
     if (warp < 4) {   // accumulators start at zero
         for (uint32_t c = 0; c < NCOLS; c += 16) tmem_st16_zero(tbase + ((uint32_t)(warp * 32) << 16) + c);
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(288) k_conv_rows(const RowArgs a)
             tc::mbar_expect_tx(bars + 8 * RWB, rows_wbytes(CIN, COUT));
             tc::bulk_load(sW, a.wpk, rows_wbytes(CIN, COUT), bars + 8 * RWB);
         }
+        pdl_wait();   // the weights were packed before the kernel ahead of this one began
         const uint32_t sbase = sS + (uint32_t)pw * SLOT;
         uint32_t L = 0;
         bool ok = true;
@@ -358,6 +361,7 @@ __global__ void __launch_bounds__(288) k_conv_rows(const RowArgs a)
     } else if (warp < 4) {
         // ---- epilogue: read each output's block, zero it, store the voxels
         const int row = warp * 32 + lane;
+        pdl_wait();
         float bias[COUT / 16][16], hw[16];
 #pragma unroll
         for (int c = 0; c < COUT; c++) bias[c / 16][c % 16] = a.epi.bias ? a.epi.bias[c] : 0.f;
@@ -461,6 +465,7 @@ __global__ void __launch_bounds__(288) k_conv_wide(const WideArgs a)
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
+    pdl_trigger();
     const uint32_t tbase = tslot;
     const uint32_t S = (uint32_t)a.stages;
 
@@ -471,6 +476,7 @@ __global__ void __launch_bounds__(288) k_conv_wide(const WideArgs a)
         uint32_t u = 0, slot = 0, par = 1;          // fills issued; slot u % S and its empty parity
         uint32_t aslot = 0;                         // slot of the next fill to report
         bool ok = true;
+        pdl_wait();
         for (int w = blockIdx.x; ok && w < nwork; w += gridDim.x) {
             const int tile = w / a.nsplit, n0 = (w - tile * a.nsplit) * a.nt;
             int x, y, z, x2, y2, z2;
@@ -558,6 +564,7 @@ __global__ void __launch_bounds__(288) k_conv_wide(const WideArgs a)
     } else if (warp < 4) {
         const float none[16] = {};
         uint32_t it = 0;
+        pdl_wait();
         for (int w = blockIdx.x; w < nwork; w += gridDim.x, it++) {
             const int tile = w / a.nsplit, n0 = (w - tile * a.nsplit) * a.nt;
             int x, y, z;
@@ -630,6 +637,8 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorM
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tbase = tslot;
     const uint32_t sbo = (uint32_t)a.nb * 16u;   // next 8 channels
     const int nks = a.nb >> 4;
@@ -761,6 +770,8 @@ __global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tbase = tslot;
     const int nrow = (a.R + RA - 1) / RA;   // steps per line tile
 
@@ -1176,7 +1187,7 @@ int launch_rows(cudaStream_t s, RowArgs r, int nsm)
     r.rch = 32;
     while ((r.rch > 4 && lines / r.rch < 2LL * most) || (r.rch > 1 && lines / r.rch < most)) r.rch >>= 1;
     r.nitems = r.ntx * ((r.R + r.rch - 1) / r.rch);
-    k_conv_rows<CIN, COUT, ZRING><<<most < r.nitems ? most : r.nitems, 288, smem, s>>>(r);
+    net_launch(k_conv_rows<CIN, COUT, ZRING>, most < r.nitems ? most : r.nitems, 1, 288, smem, s, r);
     return launch_error("k_conv_rows");
 }
 
@@ -1220,7 +1231,7 @@ int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int 
     if (a.stages > WSTAGES) a.stages = WSTAGES;
     if (a.stages <= WLAG) { snprintf(g_conv_err, sizeof(g_conv_err), "conv needs %u B of shared memory a stage", a.stride); return 1; }
     const int nwork = a.ntiles * a.nsplit;
-    k_conv_wide<<<nsm < nwork ? nsm : nwork, 288, (uint32_t)a.stages * a.stride + 1024u, s>>>(a);
+    net_launch(k_conv_wide, nsm < nwork ? nsm : nwork, 1, 288, (uint32_t)a.stages * a.stride + 1024u, s, a);
     return launch_error("k_conv_wide");
 }
 
@@ -1233,7 +1244,7 @@ int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm)
     static int lim = dyn_smem_limit((const void *)k_wgrad_rows<CIN, COUT>);
     if ((int)smem > lim) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad needs %u B of shared memory", smem); return 1; }
     r.nsteps = r.ntx * ((r.R + WgR<CIN>::RA - 1) / WgR<CIN>::RA);
-    k_wgrad_rows<CIN, COUT><<<nsm < r.nsteps ? nsm : r.nsteps, 288, smem, s>>>(r);
+    net_launch(k_wgrad_rows<CIN, COUT>, nsm < r.nsteps ? nsm : r.nsteps, 1, 288, smem, s, r);
     return launch_error("k_wgrad_rows");
 }
 
@@ -1280,7 +1291,7 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
     a.nsplit = want < 1 ? 1 : want;
     if (a.nsplit > a.ntiles) a.nsplit = a.ntiles;
     a.dw = dw; a.err = err;
-    k_wgrad<<<a.ngroups * a.nsplit, 192, smem, s>>>(mx, md, a);
+    net_launch(k_wgrad, a.ngroups * a.nsplit, 1, 192, smem, s, mx, md, a);
     return launch_error("k_wgrad");
 }
 

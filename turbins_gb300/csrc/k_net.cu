@@ -75,6 +75,8 @@ __global__ void k_pack_input(long long n, const float *__restrict__ in3, bf16 *_
 // 2x2x2 average; g = coarse grid, C/8 channel blocks
 __global__ void k_pool(G3 g, int ncb, const bf16 *__restrict__ in, bf16 *__restrict__ out)
 {
+    pdl_trigger();
+    pdl_wait();
     long long nc = g.n(), nf = nc * 8;
     GRID_STRIDE(idx, nc * ncb)
     {
@@ -104,6 +106,8 @@ __device__ __forceinline__ long long parent(long long v, const G3 &f)
 __global__ void k_up_add_relu(G3 f, int ncb, const bf16 *__restrict__ c, const bf16 *__restrict__ a,
                               bf16 *__restrict__ s)
 {
+    pdl_trigger();
+    pdl_wait();
     long long nf = f.n(), nc = nf / 8;
     GRID_STRIDE(idx, nf * ncb)
     {
@@ -120,6 +124,8 @@ __global__ void k_up_add_relu(G3 f, int ncb, const bf16 *__restrict__ c, const b
 // adjoint of the nearest upsampling: sum over the 8 children; g = coarse grid
 __global__ void k_down_sum(G3 g, int ncb, const bf16 *__restrict__ d, bf16 *__restrict__ out)
 {
+    pdl_trigger();
+    pdl_wait();
     long long nc = g.n(), nf = nc * 8;
     GRID_STRIDE(idx, nc * ncb)
     {
@@ -141,6 +147,8 @@ __global__ void k_down_sum(G3 g, int ncb, const bf16 *__restrict__ d, bf16 *__re
 __global__ void k_combine(G3 f, int ncb, const bf16 *__restrict__ dzs, const bf16 *__restrict__ dp,
                           const bf16 *__restrict__ a, bf16 *__restrict__ dz)
 {
+    pdl_trigger();
+    pdl_wait();
     long long nf = f.n(), nc = nf / 8;
     GRID_STRIDE(idx, nf * ncb)
     {
@@ -188,6 +196,8 @@ __device__ __forceinline__ void block_add(const float (&acc)[NV], float *const (
 // per-channel sums over voxels (bias gradients): grid (blocks, ncb), 256 threads
 __global__ void k_chan_sum(long long n, const bf16 *__restrict__ d, float *__restrict__ g)
 {
+    pdl_trigger();
+    pdl_wait();
     const int cb = blockIdx.y;
     const bf16 *p = d + (long long)cb * n * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -456,7 +466,7 @@ int wgrad(TurbNet *n, cudaStream_t s, int l, const bf16 *x, const bf16 *dy)
     if (rc) return turb_set_error_text(conv_last_error());
     // four voxels per thread, about two blocks per SM over all channel blocks
     const int want = nblk((n->V[lv] + 3) / 4), most = 2 * n->nsm * 8 / d.cout;
-    k_chan_sum<<<dim3(want < most ? want : most > 1 ? most : 1, d.cout / 8), 256, 0, s>>>(n->V[lv], dy, n->G + n->boff[l]);
+    net_launch(k_chan_sum, want < most ? want : most > 1 ? most : 1, d.cout / 8, 256, 0, s, n->V[lv], dy, n->G + n->boff[l]);
     return TURB_OK;
 }
 G3 g3(const TurbNet *n, int l) { return G3{n->X[l], n->Y[l], n->Z[l]}; }
@@ -486,13 +496,13 @@ int forward(TurbNet *n, cudaStream_t s, const float *in3, float *hout)
     e.relu = 1;
     e.bias = P + n->boff[0]; e.out = n->a0;
     NCHK(conv(n, s, 0, n->x0, e));
-    k_pool<<<nblk(n->V[1] * 2), 256, 0, s>>>(g3(n, 1), 2, n->a0, n->p0);
+    net_launch(k_pool, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->a0, n->p0);
     e.bias = P + n->boff[1]; e.out = n->a1;
     NCHK(conv(n, s, 1, n->p0, e));
-    k_pool<<<nblk(n->V[2] * 4), 256, 0, s>>>(g3(n, 2), 4, n->a1, n->p1);
+    net_launch(k_pool, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->a1, n->p1);
     e.bias = P + n->boff[2]; e.out = n->a2;
     NCHK(conv(n, s, 2, n->p1, e));
-    k_pool<<<nblk(n->V[3] * 8), 256, 0, s>>>(g3(n, 3), 8, n->a2, n->p2);
+    net_launch(k_pool, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->a2, n->p2);
     e.bias = P + n->boff[3]; e.out = n->a3;
     NCHK(conv(n, s, 3, n->p2, e));
     e.bias = P + n->boff[4]; e.out = n->b3;
@@ -500,17 +510,17 @@ int forward(TurbNet *n, cudaStream_t s, const float *in3, float *hout)
     ConvEpi u;
     u.bias = P + n->boff[5]; u.out = n->c2;
     NCHK(conv(n, s, 5, n->b3, u));
-    k_up_add_relu<<<nblk(n->V[2] * 8), 256, 0, s>>>(g3(n, 2), 8, n->c2, n->a2, n->s2);
+    net_launch(k_up_add_relu, nblk(n->V[2] * 8), 1, 256, 0, s, g3(n, 2), 8, n->c2, n->a2, n->s2);
     e.bias = P + n->boff[6]; e.out = n->b2;
     NCHK(conv(n, s, 6, n->s2, e));
     u.bias = P + n->boff[7]; u.out = n->c1;
     NCHK(conv(n, s, 7, n->b2, u));
-    k_up_add_relu<<<nblk(n->V[1] * 4), 256, 0, s>>>(g3(n, 1), 4, n->c1, n->a1, n->s1);
+    net_launch(k_up_add_relu, nblk(n->V[1] * 4), 1, 256, 0, s, g3(n, 1), 4, n->c1, n->a1, n->s1);
     e.bias = P + n->boff[8]; e.out = n->b1;
     NCHK(conv(n, s, 8, n->s1, e));
     u.bias = P + n->boff[9]; u.out = n->c0;
     NCHK(conv(n, s, 9, n->b1, u));
-    k_up_add_relu<<<nblk(n->V[0] * 2), 256, 0, s>>>(g3(n, 0), 2, n->c0, n->a0, n->s0);
+    net_launch(k_up_add_relu, nblk(n->V[0] * 2), 1, 256, 0, s, g3(n, 0), 2, n->c0, n->a0, n->s0);
     ConvEpi h;
     h.relu = 1;
     h.bias = P + n->boff[10];
@@ -529,30 +539,30 @@ int backward(TurbNet *n, cudaStream_t s, const float *gout)
                                                                            n->dz0b, n->G + n->hw_off, n->G + n->hb_off);
     NCHK(wgrad(n, s, 10, n->s0, n->dz0b));
     NCHK(dgrad(n, s, 10, n->dz0b, n->s0, n->dzs0));
-    k_down_sum<<<nblk(n->V[1] * 2), 256, 0, s>>>(g3(n, 1), 2, n->dzs0, n->dc0);
+    net_launch(k_down_sum, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->dzs0, n->dc0);
     NCHK(wgrad(n, s, 9, n->b1, n->dc0));
     NCHK(dgrad(n, s, 9, n->dc0, n->b1, n->dz1b));
     NCHK(wgrad(n, s, 8, n->s1, n->dz1b));
     NCHK(dgrad(n, s, 8, n->dz1b, n->s1, n->dzs1));
-    k_down_sum<<<nblk(n->V[2] * 4), 256, 0, s>>>(g3(n, 2), 4, n->dzs1, n->dc1);
+    net_launch(k_down_sum, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->dzs1, n->dc1);
     NCHK(wgrad(n, s, 7, n->b2, n->dc1));
     NCHK(dgrad(n, s, 7, n->dc1, n->b2, n->dz2b));
     NCHK(wgrad(n, s, 6, n->s2, n->dz2b));
     NCHK(dgrad(n, s, 6, n->dz2b, n->s2, n->dzs2));
-    k_down_sum<<<nblk(n->V[3] * 8), 256, 0, s>>>(g3(n, 3), 8, n->dzs2, n->dc2);
+    net_launch(k_down_sum, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->dzs2, n->dc2);
     NCHK(wgrad(n, s, 5, n->b3, n->dc2));
     NCHK(dgrad(n, s, 5, n->dc2, n->b3, n->dz3b));
     NCHK(wgrad(n, s, 4, n->a3, n->dz3b));
     NCHK(dgrad(n, s, 4, n->dz3b, n->a3, n->dz3));
     NCHK(wgrad(n, s, 3, n->p2, n->dz3));
     NCHK(dgrad(n, s, 3, n->dz3, nullptr, n->dp2));
-    k_combine<<<nblk(n->V[2] * 8), 256, 0, s>>>(g3(n, 2), 8, n->dzs2, n->dp2, n->a2, n->dz2);
+    net_launch(k_combine, nblk(n->V[2] * 8), 1, 256, 0, s, g3(n, 2), 8, n->dzs2, n->dp2, n->a2, n->dz2);
     NCHK(wgrad(n, s, 2, n->p1, n->dz2));
     NCHK(dgrad(n, s, 2, n->dz2, nullptr, n->dp1));
-    k_combine<<<nblk(n->V[1] * 4), 256, 0, s>>>(g3(n, 1), 4, n->dzs1, n->dp1, n->a1, n->dz1);
+    net_launch(k_combine, nblk(n->V[1] * 4), 1, 256, 0, s, g3(n, 1), 4, n->dzs1, n->dp1, n->a1, n->dz1);
     NCHK(wgrad(n, s, 1, n->p0, n->dz1));
     NCHK(dgrad(n, s, 1, n->dz1, nullptr, n->dp0));
-    k_combine<<<nblk(n->V[0] * 2), 256, 0, s>>>(g3(n, 0), 2, n->dzs0, n->dp0, n->a0, n->dz0);
+    net_launch(k_combine, nblk(n->V[0] * 2), 1, 256, 0, s, g3(n, 0), 2, n->dzs0, n->dp0, n->a0, n->dz0);
     NCHK(wgrad(n, s, 0, n->x0, n->dz0));
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
 }
@@ -1008,6 +1018,7 @@ int turb_conv3_test(int X, int Y, int Z, int cin, int cout, const void *in, cons
     cudaMemsetAsync(wd, 0, nwd * 2, s);
     cudaMemsetAsync(err, 0, sizeof(int), s);
     conv_pack_weights(s, W, cin, cout, pf, pb, wf, wd);
+    cudaStreamSynchronize(s);   // the convolution may load its weights before the kernel ahead of it ends
     ConvEpi e;
     e.bias = dgrad_mode ? nullptr : bias;
     e.relu = relu;

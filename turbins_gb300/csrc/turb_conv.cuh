@@ -54,3 +54,24 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
                 int *err, int nsm);
 int conv_selftest_umma(int mn_major, int swap, unsigned long long *mismatches);
 const char *conv_last_error();
+
+// Launches a network kernel as a programmatic dependent of the one before it
+// on the stream: its set-up (barriers, TMEM, resident weights) overlaps that
+// kernel's tail.  Every such kernel calls pdl_trigger and, before it reads or
+// writes anything the others do, pdl_wait; the first kernel of a pass is an
+// ordinary launch, so what was written before the pass is visible to all
+template <typename... P, typename... A>
+inline void net_launch(void (*k)(P...), int gx, int gy, int threads, uint32_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
