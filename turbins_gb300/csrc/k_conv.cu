@@ -725,7 +725,9 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorM
 // (row, dq, ci), 128 with padding), for B the gradients of the rows around
 // them (N = (t, co), t = 0 .. RA + 1 from the row before the first).  Tap dx is
 // a shift of A by dx rows, so a step is 3 x 8 MMAs, one accumulator per dx; row
-// a and t belong to tap dr = a - t + 2.  A box per tap of an unswizzled layout
+// a and t belong to tap dr = a - t + 2.  On large grids a CTA has one dx and
+// three times the steps: the FP32 accumulation chains then stay as long as
+// k_wgrad's, and the gradients within 2e-5 of its sums.  A box per tap of an unswizzled layout
 // (k_wgrad) loads a 16-byte voxel row per cycle and 27 of them per voxel:
 // 141 us at 128x64x64, 16 -> 16 channels, against 33 us here; 37, 41 and 26 us
 // against 13, 17 and 18 us for 32 -> 16, 32 -> 32 and 16 -> 32 at 64x32x32.
@@ -735,7 +737,7 @@ struct WgR {
 };
 struct WgRowArgs {
     int X, W, R, rs, Q, qs, cstep;   // cstep: voxels of the grid (between channel blocks)
-    int ntx, nsteps, zring;
+    int ntx, nsteps, zring, ndx;     // ndx: x taps per CTA, 3 or 1
     const bf16 *x, *dy;
     float *dw;
     int *err;
@@ -774,6 +776,7 @@ __global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
     pdl_wait();
     const uint32_t tbase = tslot;
     const int nrow = (a.R + RA - 1) / RA;   // steps per line tile
+    const int ng = 3 / a.ndx, dx0 = blockIdx.x % ng, dx1 = dx0 + a.ndx, w0 = blockIdx.x / ng, wstep = gridDim.x / ng;
 
     if (warp >= 4 && warp < 8) {
         // ---- producers: thread t loads voxel row t of both operands; the first
@@ -788,7 +791,7 @@ __global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
             else { q = s < 0 ? -1 : s / a.W; x = s - q * a.W - 1; }
             return q >= 0 && q < a.Q && x >= 0 && x < a.X;
         };
-        for (int w = blockIdx.x; w < a.nsteps; w += gridDim.x, u++) {
+        for (int w = w0; w < a.nsteps; w += wstep, u++) {
             if (!tc::mbar_wait(bars + 8 * (EM_ + slot), par, abort_)) { ok = false; break; }
             const int tile = w / nrow, r0 = (w - tile * nrow) * RA, line0 = tile * 128;
             const uint32_t buf = s0 + slot * STAGE;
@@ -839,13 +842,14 @@ __global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
             constexpr uint32_t idesc = tc::idesc_bf16(128, N, 1, 1);
             uint32_t slot = 0, par = 0, u = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < a.nsteps; w += gridDim.x, u++) {
+            for (int w = w0; w < a.nsteps; w += wstep, u++) {
                 if (!tc::mbar_wait(bars + 8 * (FA_ + slot), par, abort_)) { ok = false; break; }
                 tc::fence_after();
                 const uint32_t buf = s0 + slot * STAGE;
                 const uint64_t ad = mn128_desc(buf, SBYTES), bd = mn128_desc(buf + 2u * SBYTES, 16384u);
 #pragma unroll
                 for (int dx = 0; dx < 3; dx++)
+                    if (dx >= dx0 && dx < dx1)
 #pragma unroll
                     for (int ks = 0; ks < 8; ks++)
                         tc::mma_bf16(tbase + (uint32_t)(dx * N), ad + (uint32_t)(dx * 8 + ks * 128), bd + (uint32_t)(ks * 128),
@@ -865,7 +869,7 @@ __global__ void __launch_bounds__(288) k_wgrad_rows(const WgRowArgs a)
             const int row = warp * 32 + lane;
             const int ra = RA == 2 ? row >> 6 : 0, m = RA == 2 ? row & 63 : row, dq = m / CIN, ci = m % CIN;
             const bool valid = dq < 3 && !*abort_;
-            for (int dx = 0; dx < 3; dx++)
+            for (int dx = dx0; dx < dx1; dx++)
                 for (int t = 0; t < NB; t++) {
                     const int dr = ra - t + 2;
                     if (dr < 0 || dr > 2) continue;
@@ -1244,7 +1248,9 @@ int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm)
     static int lim = dyn_smem_limit((const void *)k_wgrad_rows<CIN, COUT>);
     if ((int)smem > lim) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad needs %u B of shared memory", smem); return 1; }
     r.nsteps = r.ntx * ((r.R + WgR<CIN>::RA - 1) / WgR<CIN>::RA);
-    net_launch(k_wgrad_rows<CIN, COUT>, nsm < r.nsteps ? nsm : r.nsteps, 1, 288, smem, s, r);
+    r.ndx = r.nsteps > 20 * nsm ? 1 : 3;
+    const int ng = 3 / r.ndx, per = nsm / ng < r.nsteps ? nsm / ng : r.nsteps;
+    net_launch(k_wgrad_rows<CIN, COUT>, ng * (per > 0 ? per : 1), 1, 288, smem, s, r);
     return launch_error("k_wgrad_rows");
 }
 
