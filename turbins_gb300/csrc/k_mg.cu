@@ -208,6 +208,69 @@ __global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, int planes, con
     }
 }
 
+// The same for the small levels (one plane), which are bound by latency: 1/diag
+// and the metric tables belong to the grid and are loaded while the half sweep
+// before this one still runs, b and x after it (their pointers are not
+// __restrict__: what the kernels before write must not be read early)
+__global__ void __launch_bounds__(256) k_rbgs4s(MgDevLevel Ld, int color, int zero_init, const float *b,
+                                                const float *__restrict__ invd, float *x)
+{
+    pdl_trigger();
+    const int nx = Ld.nx, ny = Ld.ny, nz = Ld.nz, hx = nx >> 1;
+    const int q4 = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (j >= ny || 4 * q4 >= hx) return;   // the other threads wait
+    const int half = (int)(((long long)nx * ny * nz) >> 1), hxy = hx * ny;
+    const float dyj = Ld.dyf[j], ryj = Ld.rfyf[j], ryj1 = Ld.rfyf[j + 1];
+    const int k = blockIdx.z, p = (color + j + k) & 1, m0 = (k * ny + j) * hx + 4 * q4;
+    const float4 dd = *reinterpret_cast<const float4 *>(invd + (size_t)color * half + m0);
+    const float4 dx4 = *reinterpret_cast<const float4 *>(Ld.dxpf + p * hx + 4 * q4);
+    const float4 rl4 = *reinterpret_cast<const float4 *>(Ld.rlpf + p * hx + 4 * q4);
+    const float4 rr4 = *reinterpret_cast<const float4 *>(Ld.rrpf + p * hx + 4 * q4);
+    const float dzk = Ld.dzf[k], rzk = Ld.rfzf[k], rzk1 = Ld.rfzf[k + 1];
+    pdl_wait();
+    const float4 bb = *reinterpret_cast<const float4 *>(b + (size_t)color * half + m0);
+    if (zero_init) {
+        *reinterpret_cast<float4 *>(x + (size_t)color * half + m0) =
+            make_float4(rmul(bb.x, dd.x), rmul(bb.y, dd.y), rmul(bb.z, dd.z), rmul(bb.w, dd.w));
+        return;
+    }
+    const float *oth = x + (size_t)(1 - color) * half;
+    const float4 c4 = *reinterpret_cast<const float4 *>(oth + m0);
+    float ex = 0.0f;   // the fifth x-neighbour: left of the group (p = 0) or right of it (p = 1)
+    if (p == 0) { if (q4 > 0) ex = oth[m0 - 1]; }
+    else { if (4 * q4 + 4 < hx) ex = oth[m0 + 4]; }
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 jm = j > 0 ? *reinterpret_cast<const float4 *>(oth + m0 - hx) : zero4;
+    const float4 jp = j < ny - 1 ? *reinterpret_cast<const float4 *>(oth + m0 + hx) : zero4;
+    const float4 km = k > 0 ? *reinterpret_cast<const float4 *>(oth + m0 - hxy) : zero4;
+    const float4 kp = k < nz - 1 ? *reinterpret_cast<const float4 *>(oth + m0 + hxy) : zero4;
+    const float dyz = rmul(dyj, dzk);
+    const float cv[4] = {c4.x, c4.y, c4.z, c4.w};
+    const float bv[4] = {bb.x, bb.y, bb.z, bb.w}, dv[4] = {dd.x, dd.y, dd.z, dd.w};
+    const float jmv[4] = {jm.x, jm.y, jm.z, jm.w}, jpv[4] = {jp.x, jp.y, jp.z, jp.w};
+    const float kmv[4] = {km.x, km.y, km.z, km.w}, kpv[4] = {kp.x, kp.y, kp.z, kp.w};
+    const float dxv[4] = {dx4.x, dx4.y, dx4.z, dx4.w};
+    const float rlv[4] = {rl4.x, rl4.y, rl4.z, rl4.w}, rrv[4] = {rr4.x, rr4.y, rr4.z, rr4.w};
+    float out[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const int i = 2 * (4 * q4 + e) + p;
+        const float xl = p == 0 ? (e == 0 ? ex : cv[e - 1]) : cv[e];
+        const float xr = p == 0 ? cv[e] : (e == 3 ? ex : cv[e + 1]);
+        const float dxi = dxv[e];
+        const float dxz = rmul(dxi, dzk), dxy = rmul(dxi, dyj);
+        float o = 0.0f, f;
+        if (i > 0) { f = rmul(dyz, rlv[e]); o = rfma(f, xl, o); }
+        if (i < nx - 1) { f = rmul(dyz, rrv[e]); o = rfma(f, xr, o); }
+        if (j > 0) { f = rmul(dxz, ryj); o = rfma(f, jmv[e], o); }
+        if (j < ny - 1) { f = rmul(dxz, ryj1); o = rfma(f, jpv[e], o); }
+        if (k > 0) { f = rmul(dxy, rzk); o = rfma(f, kmv[e], o); }
+        if (k < nz - 1) { f = rmul(dxy, rzk1); o = rfma(f, kpv[e], o); }
+        out[e] = rmul(radd(bv[e], o), dv[e]);
+    }
+    *reinterpret_cast<float4 *>(x + (size_t)color * half + m0) = make_float4(out[0], out[1], out[2], out[3]);
+}
+
 // The half sweep of k_rbgs4 marching along k (not the first, zero-initial
 // one): a block of 32 x 8 threads owns 128 cells of its colour in each of 8
 // rows of every plane of a chunk of jz planes.  The other colour's plane k
@@ -914,9 +977,21 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
                     return;
                 }
             }
-            const int planes = (long long)L.nx * L.ny * L.nz >= RB4_PLANES_CELLS ? RB4_PLANES : 1;
-            dim3 g4p(g4.x, g4.y, (unsigned)((L.nz + planes - 1) / planes));
-            launch_k(pdl, k_rbgs4, g4p, B38, s, L, color, zero_init, planes, b, invd, x);
+            if ((long long)L.nx * L.ny * L.nz >= RB4_PLANES_CELLS) {
+                launch_k(pdl, k_rbgs4,
+                         dim3(g4.x, g4.y, (unsigned)((L.nz + RB4_PLANES - 1) / RB4_PLANES)), B38, s, L, color, zero_init,
+                         RB4_PLANES, b, invd, x);
+                return;
+            }
+            // short rows share a warp: as few threads along x as cover the row
+            dim3 bs(32, 8, 1);
+            while ((int)bs.x >= L.nx / 4 && bs.x > 2) {
+                bs.x >>= 1;
+                bs.y <<= 1;
+            }
+            while ((int)bs.y >= 2 * L.ny && bs.x * bs.y > 32) bs.y >>= 1;
+            const dim3 g((L.nx / 8 + bs.x - 1) / bs.x, (L.ny + bs.y - 1) / bs.y, (unsigned)L.nz);
+            launch_k(pdl, k_rbgs4s, g, bs, s, L, color, zero_init, b, invd, x);
             return;
         }
     }

@@ -73,7 +73,7 @@ __global__ void k_pack_input(long long n, const float *__restrict__ in3, bf16 *_
 }
 
 // 2x2x2 average; g = coarse grid, C/8 channel blocks
-__global__ void k_pool(G3 g, int ncb, const bf16 *__restrict__ in, bf16 *__restrict__ out)
+__global__ void k_pool(G3 g, int ncb, const bf16 *in, bf16 *out)
 {
     pdl_trigger();
     pdl_wait();
@@ -103,8 +103,8 @@ __device__ __forceinline__ long long parent(long long v, const G3 &f)
 }
 
 // s = relu(up(c) + a) on the fine grid f
-__global__ void k_up_add_relu(G3 f, int ncb, const bf16 *__restrict__ c, const bf16 *__restrict__ a,
-                              bf16 *__restrict__ s)
+__global__ void k_up_add_relu(G3 f, int ncb, const bf16 *c, const bf16 *a,
+                              bf16 *s)
 {
     pdl_trigger();
     pdl_wait();
@@ -122,7 +122,7 @@ __global__ void k_up_add_relu(G3 f, int ncb, const bf16 *__restrict__ c, const b
 }
 
 // adjoint of the nearest upsampling: sum over the 8 children; g = coarse grid
-__global__ void k_down_sum(G3 g, int ncb, const bf16 *__restrict__ d, bf16 *__restrict__ out)
+__global__ void k_down_sum(G3 g, int ncb, const bf16 *d, bf16 *out)
 {
     pdl_trigger();
     pdl_wait();
@@ -144,8 +144,8 @@ __global__ void k_down_sum(G3 g, int ncb, const bf16 *__restrict__ d, bf16 *__re
 }
 
 // dz = (dzs + up(dp) / 8) * (a > 0) on the fine grid f
-__global__ void k_combine(G3 f, int ncb, const bf16 *__restrict__ dzs, const bf16 *__restrict__ dp,
-                          const bf16 *__restrict__ a, bf16 *__restrict__ dz)
+__global__ void k_combine(G3 f, int ncb, const bf16 *dzs, const bf16 *dp,
+                          const bf16 *a, bf16 *dz)
 {
     pdl_trigger();
     pdl_wait();
@@ -194,7 +194,7 @@ __device__ __forceinline__ void block_add(const float (&acc)[NV], float *const (
 }
 
 // per-channel sums over voxels (bias gradients): grid (blocks, ncb), 256 threads
-__global__ void k_chan_sum(long long n, const bf16 *__restrict__ d, float *__restrict__ g)
+__global__ void k_chan_sum(long long n, const bf16 *d, float *g)
 {
     pdl_trigger();
     pdl_wait();
