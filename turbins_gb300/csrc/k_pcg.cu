@@ -14,12 +14,6 @@ constexpr int NP = 4096;   // blocks of the grid-stride reductions
 constexpr int BS = 256;
 constexpr int VB = 4;      // blocks of a reduction that a block of its launch stands for
 
-__device__ __forceinline__ double warp_sum(double v)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 __device__ __forceinline__ void block_store(double v, double *dst)
 {
     __shared__ double sm[32];
@@ -33,64 +27,6 @@ __device__ __forceinline__ void block_store(double v, double *dst)
         if (lt == 0) *dst = r;
     }
     __syncthreads();
-}
-
-// Sums of the blocks' partials by the block that finishes last: it adds them
-// as one block of 1024 threads would (thread t takes partials t, t + 1024, ..,
-// then a shuffle tree per warp and one over the warps), whatever its own
-// size, so the sums do not depend on which block it is.  Partials
-// [nblk, nper) are those of blocks that would have no elements: zeros, which
-// adding leaves out.  nval values, value v's partials at part + v * stride.
-// A launch for the sums cost 6 us at every size; this costs one round trip.
-__device__ __forceinline__ bool last_block(unsigned *count, unsigned nblk)
-{
-    __shared__ bool last;
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        __threadfence();
-        last = atomicAdd(count, 1u) == nblk - 1;
-        if (last) {
-            *count = 0u;   // ready for the next launch
-            __threadfence();
-        }
-    }
-    __syncthreads();
-    return last;
-}
-
-template <int NVAL>
-__device__ __forceinline__ void sum_parts(const double *part, long long stride, int nblk, double *dst)
-{
-    __shared__ double sm[NVAL][1024];
-    const int lt = threadIdx.y * blockDim.x + threadIdx.x, lane = lt & 31;
-    // the 1024 threads' sums, four per thread of this block of 256
-#pragma unroll
-    for (int v = 0; v < NVAL; v++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            double acc = 0.0;
-            for (int t = q * 256 + lt; t < nblk; t += 1024) acc += __ldcg(part + v * stride + t);
-            sm[v][q * 256 + lt] = acc;
-        }
-    __syncthreads();
-    // the trees of the 32 warps, each pair added once: warp w's entries stay
-    // at w * 32 .. while their number halves (distances 16, 8, 4, 2, 1)
-    if (lt < 128) {
-        for (int d = 16; d >= 1; d >>= 1) {
-            for (int v = 0; v < NVAL; v++)
-                for (int t = lt; t < 32 * d; t += 128) {
-                    const int at = (t / d) * 32 + (t & (d - 1));
-                    sm[v][at] += sm[v][at + d];
-                }
-            asm volatile("bar.sync 2, 128;" ::: "memory");
-        }
-    }
-    if (lt < 32) {
-#pragma unroll
-        for (int v = 0; v < NVAL; v++) {
-            const double r = warp_sum(sm[v][lane * 32]);
-            if (lt == 0) dst[v] = r;
-        }
-    }
 }
 
 // block_store of NV values of a 256-thread block to dst + n * stride

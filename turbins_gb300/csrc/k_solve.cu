@@ -18,19 +18,35 @@ namespace {
 constexpr int HBX = 32, HBY = 8, KC = 4;   // 32x8 threads over (i, j), KC planes per thread
 constexpr int KCJ = 2;                      // planes per thread of the FP32 Jacobi sweep
 
-__device__ __forceinline__ double block_sum(double v)
+// the n partials of one sum, added by the last of `blocks` blocks (of one or
+// two launches that share the counter) into *dst
+struct SumTo {
+    int n;
+    unsigned blocks, *count;
+    double *dst;
+};
+__device__ __forceinline__ void sum_to(const double *part, const SumTo &to)
 {
-    __shared__ double sm[32];
-    int lt = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((lt & 31) == 0) sm[lt >> 5] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (lt < 32) {
-        r = (lt < (nt >> 5)) ? sm[lt] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    }
-    return r;   // valid in thread (0, 0)
+    if (last_block(to.count, to.blocks)) sum_parts<1>(part, 0, to.n, to.dst);
+}
+
+// FP64 <-> FP32 without the conversion instructions, which run on the FP64
+// pipe (two lanes per SM and clock on GB300): normal results are shifted and
+// rounded to nearest even on the integer pipe, the others converted
+__device__ __forceinline__ float to_f32(double v)
+{
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v), e = hi >> 20 & 0x7ffu;
+    if (e - 897u > 1150u - 897u) return (float)v;
+    unsigned f = (e - 896u) << 23 | (hi & 0xfffffu) << 3 | lo >> 29;
+    const unsigned rest = lo & 0x1fffffffu;
+    f += rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
+    return __uint_as_float(f | (hi & 0x80000000u));
+}
+__device__ __forceinline__ double to_f64(float v)
+{
+    const unsigned u = __float_as_uint(v), e = u >> 23 & 0xffu;
+    if (e - 1u > 253u) return (double)v;
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
 }
 
 __device__ __forceinline__ long long part_index()
@@ -115,7 +131,7 @@ __global__ void k_ib_apply(IbDev ib, const double *__restrict__ x, double *__res
 // one Jacobi sweep xn = x + (b - A x)/diag, partial sums of |b - A x|^2
 __global__ void k_helm_jacobi(Dims d, HelmTab h, const uint8_t *__restrict__ st, double a_dt,
                               const double *__restrict__ b, const double *__restrict__ x,
-                              double *__restrict__ xn, double *__restrict__ part)
+                              double *__restrict__ xn, double *__restrict__ part, const SumTo to)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     double r2 = 0.0;
@@ -136,10 +152,11 @@ __global__ void k_helm_jacobi(Dims d, HelmTab h, const uint8_t *__restrict__ st,
     double bs[1];
     block_sum256<1>({r2}, bs);
     if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs[0];
+    sum_to(part, to);
 }
 
 __global__ void k_ib_jacobi(IbDev ib, const double *__restrict__ b, const double *__restrict__ x,
-                            double *__restrict__ xn, double *__restrict__ part)
+                            double *__restrict__ xn, double *__restrict__ part, long long part0, const SumTo to)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     double r2 = 0.0;
@@ -154,76 +171,140 @@ __global__ void k_ib_jacobi(IbDev ib, const double *__restrict__ b, const double
     }
     double bs[1];
     block_sum256<1>({r2}, bs);
-    if (threadIdx.x == 0) part[blockIdx.x] = bs[0];
-}
-
-__global__ void k_sum_final(long long n, const double *__restrict__ part, double *__restrict__ out)
-{
-    double v = 0.0;
-    for (long long t = threadIdx.x; t < n; t += blockDim.x) v += part[t];
-    double s = block_sum(v);
-    if (threadIdx.x == 0) *out = s;
+    if (threadIdx.x == 0) part[part0 + blockIdx.x] = bs[0];
+    sum_to(part, to);
 }
 
 // ---- mixed-precision defect correction -----------------------------------
-// xn = x + e over the whole field (FP64 accumulation of the FP32 correction)
-__global__ void k_add_corr(long long n, const double *__restrict__ x, const float *__restrict__ e,
-                           double *__restrict__ xn)
+// x += e over the whole field (FP64 accumulation of the FP32 correction of a
+// single sweep)
+__global__ void k_add_corr(long long n, double *__restrict__ x, const float *__restrict__ e)
 {
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
-        xn[p] = x[p] + (double)e[p];
+        x[p] = x[p] + (double)e[p];
 }
 
-// r = b - A x in FP64, rounded to FP32 for the inner solve; |r|^2 partials.
-// The FP64 pipe bounds this kernel, so the row is accumulated as
-// -(diag x - b + sum a_nb x_nb) (no separate subtraction) and apz[k] + 1/dt
-// is formed once per plane of the block: nine FP64 operations per point
-__global__ void k_helm_resid64(Dims d, HelmTab h, const uint8_t *__restrict__ st, double a_dt,
-                               const double *__restrict__ b, const double *__restrict__ x,
-                               float *__restrict__ rf, double *__restrict__ part)
+// r = b - A x in FP64, rounded to FP32 for the inner solve; |r|^2; and the
+// inner solve's first sweep, e = r / diag (from e = 0), whose FP32 work is free
+// here.  The FP64 pipe bounds this kernel on large grids, so the row is
+// accumulated as -(diag x - b + sum a_nb x_nb) (no separate subtraction),
+// apz[k] + 1/dt is formed once per plane of the block and r is rounded on the
+// integer pipe: nine FP64 operations per point.  On small grids (G = 0)
+// latency does: the KC planes' loads are all in flight before the first row is
+// formed (98 registers; on large grids fewer warps then cost more than the
+// latency: 975 us against 715 at 513x257x257).  The last block adds the
+// partial sums.
+struct ResidRow {
+    double axy, aw, ae, as, an;
+    float afx, afy;
+};
+__device__ __forceinline__ void resid_store(const HelmTab &h, const HelmTabF &hf, const ResidRow &w, double a_dt, double zdt, int s,
+                                            int k, double xc, double bc, double xw, double xe, double xs, double xn, double xb,
+                                            double xf, float *rf, float *e0, double &r2)
 {
+    const bool stn = is_stencil(h.q, s);
+    double r;
+    if (!stn) {
+        r = bc - (h.ap_solid + a_dt) * xc;
+    } else {
+        double acc = fma(w.axy + zdt, xc, -bc);
+        acc = fma(w.aw, xw, acc);
+        acc = fma(w.ae, xe, acc);
+        acc = fma(w.as, xs, acc);
+        acc = fma(w.an, xn, acc);
+        acc = fma(h.ab[k], xb, acc);
+        acc = fma(h.af[k], xf, acc);
+        r = -acc;
+    }
+    const float rv = to_f32(r), a_dtf = (float)a_dt;
+    const float dg = stn ? __fadd_rn(__fadd_rn(__fadd_rn(w.afx, w.afy), hf.apz[k]), a_dtf) : __fadd_rn(hf.ap_solid, a_dtf);
+    *rf = rv;
+    *e0 = __fmul_rn(rv, __frcp_rn(dg));
+    r2 = fma(r, r, r2);
+}
+
+// G: groups of KC planes a block marches, G partial sums (those of G blocks of
+// one group); 0: one group with AHEAD loads
+template <int G>
+__global__ void __launch_bounds__(HBX *HBY, G ? 4 : 2) k_helm_resid64(Dims d, HelmTab h, HelmTabF hf, const uint8_t *__restrict__ st, double a_dt,
+                               const double *__restrict__ b, const double *__restrict__ x,
+                               float *__restrict__ rf, float *__restrict__ e0, double *__restrict__ part, const SumTo to)
+{
+    constexpr int NG = G ? G : 1;
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    __shared__ double zdt[KC];
+    const int k0 = blockIdx.z * KC * NG;
+    __shared__ double zdt[KC * NG];
     {
-        int t = threadIdx.y * blockDim.x + threadIdx.x, k = blockIdx.z * KC + t;
-        if (t < KC) zdt[t] = k < d.NZ ? h.apz[k] + a_dt : 0.0;
+        int t = threadIdx.y * blockDim.x + threadIdx.x, k = k0 + t;
+        if (t < KC * NG) zdt[t] = k < d.NZ ? h.apz[k] + a_dt : 0.0;
     }
     __syncthreads();
-    double r2 = 0.0;
+    double r2[NG] = {};
     pdl_trigger();   // the immersed rows' kernel (disjoint points) may start at once
     if (i < d.NX && j < d.NY) {
-        const double axy = h.apx[i] + h.apy[j];
-        for (int kk = 0; kk < KC; kk++) {
-            int k = blockIdx.z * KC + kk;
-            if (k >= d.NZ) break;
-            long long p = d.at(i, j, k);
-            int s = st[p];
-            if (s == T_IMMERSED) continue;
-            double r;
-            if (!is_stencil(h.q, s)) {
-                r = b[p] - (h.ap_solid + a_dt) * x[p];
-            } else {
-                Nb o = nb_of(d, i, j, k);
-                double acc = fma(axy + zdt[kk], x[p], -b[p]);
-                acc = fma(h.aw[i], x[p + o.w], acc);
-                acc = fma(h.ae[i], x[p + o.e], acc);
-                acc = fma(h.as[j], x[p + o.s], acc);
-                acc = fma(h.an[j], x[p + o.n], acc);
-                acc = fma(h.ab[k], x[p + o.b], acc);
-                acc = fma(h.af[k], x[p + o.f], acc);
-                r = -acc;
+        const long long pj = d.at(i, j, 0);
+        const int ow = i > 0 ? -1 : 0, oe = i < d.NX - 1 ? 1 : 0;
+        const int os = j > 0 ? -(int)d.PX : 0, on = j < d.NY - 1 ? (int)d.PX : 0;
+        const ResidRow w{h.apx[i] + h.apy[j], h.aw[i], h.ae[i], h.as[j], h.an[j], hf.apx[i], hf.apy[j]};
+        if (G == 0) {
+            // planes past the last are the last one again, not stored; so is the
+            // neighbour beyond an end plane (its coefficient is zero)
+            double xc[KC + 2], xw[KC], xe[KC], xs[KC], xn[KC], bc[KC];
+            int sv[KC];
+            xc[0] = x[pj + max(k0 - 1, 0) * d.plane];
+#pragma unroll
+            for (int kk = 0; kk < KC; kk++) {
+                const long long p = pj + min(k0 + kk, d.NZ - 1) * d.plane;
+                sv[kk] = st[p];
+                xc[kk + 1] = x[p];
+                xw[kk] = x[p + ow];
+                xe[kk] = x[p + oe];
+                xs[kk] = x[p + os];
+                xn[kk] = x[p + on];
+                bc[kk] = b[p];
             }
-            rf[p] = (float)r;
-            r2 = fma(r, r, r2);
+            xc[KC + 1] = x[pj + min(k0 + KC, d.NZ - 1) * d.plane];
+#pragma unroll
+            for (int kk = 0; kk < KC; kk++) {
+                const int k = k0 + kk;
+                const long long p = pj + k * d.plane;
+                if (k < d.NZ && sv[kk] != T_IMMERSED)
+                    resid_store(h, hf, w, a_dt, zdt[kk], sv[kk], k, xc[kk + 1], bc[kk], xw[kk], xe[kk], xs[kk], xn[kk], xc[kk],
+                                xc[kk + 2], rf + p, e0 + p, r2[0]);
+            }
+        } else {
+            long long p = pj + k0 * d.plane;
+            double xc = x[p], xb = k0 > 0 ? x[p - d.plane] : xc;
+#pragma unroll
+            for (int g = 0; g < NG; g++) {
+                for (int kk = 0; kk < KC; kk++, p += d.plane) {
+                    const int k = k0 + g * KC + kk;
+                    if (k >= d.NZ) break;
+                    const double xf = k < d.NZ - 1 ? x[p + d.plane] : xc;
+                    const int s = st[p];
+                    if (s != T_IMMERSED)
+                        resid_store(h, hf, w, a_dt, zdt[g * KC + kk], s, k, xc, b[p], x[p + ow], x[p + oe], x[p + os], x[p + on],
+                                    xb, xf, rf + p, e0 + p, r2[g]);
+                    xb = xc;
+                    xc = xf;
+                }
+            }
         }
     }
-    double bs[1];
-    block_sum256<1>({r2}, bs);
-    if (threadIdx.x == 0 && threadIdx.y == 0) part[part_index()] = bs[0];
+    double bs[NG];
+    block_sum256<NG>(r2, bs);
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            const int bz = blockIdx.z * NG + g;
+            if (bz * KC < d.NZ) part[((long long)bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = bs[g];
+        }
+    sum_to(part, to);
 }
 
-__global__ void k_ib_resid64(IbDev ib, const double *__restrict__ b, const double *__restrict__ x,
-                             float *__restrict__ rf, double *__restrict__ part)
+__global__ void k_ib_resid64(IbDev ib, IbDevF ibf, const double *__restrict__ b, const double *__restrict__ x,
+                             float *__restrict__ rf, float *__restrict__ e0, double *__restrict__ part, long long part0,
+                             const SumTo to)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     double r2 = 0.0;
@@ -234,27 +315,34 @@ __global__ void k_ib_resid64(IbDev ib, const double *__restrict__ b, const doubl
         for (int g = 0; g < c; g++) acc += ib.val[t * 8 + g] * x[ib.col[t * 8 + g]];
         double r = b[im] - acc;
         rf[im] = (float)r;
+        e0[im] = (float)r * __frcp_rn(ibf.diag[t]);
         r2 = r * r;
     }
     double bs[1];
     block_sum256<1>({r2}, bs);
-    if (threadIdx.x == 0) part[blockIdx.x] = bs[0];
+    if (threadIdx.x == 0) part[part0 + blockIdx.x] = bs[0];
+    sum_to(part, to);
     pdl_wait();   // as in k_ib_jac32: end after the stencil residual
 }
 
-// inner FP32 Jacobi sweep on A e = r (first sweep from e = 0), four points
-// of a row per thread: e, r, status and the j+-1 / k+-1 neighbours are
-// 16-byte (4-byte for status) loads, the x tables are padded to the pitch.
-// Immersed points are left to k_ib_jac32 (not written here, so the two
-// kernels may overlap); pad columns (i >= NX) are not written.
+// inner FP32 Jacobi sweep on A e = r (after the first, which the residual
+// does), four points of a row per thread: e, r, status and the j+-1 / k+-1
+// neighbours are 16-byte (4-byte for status) loads, the x tables are padded to
+// the pitch.  The last sweep (LAST) adds its result to x instead of storing
+// it: 25 bytes per point where the sweep and the addition moved 33.  Immersed
+// points are left to k_ib_jac32 (not written here, so the two kernels may
+// overlap); pad columns (i >= NX) are not written.  e and
+// x, which kernels just before write, are not __restrict__: nothing reads them
+// before pdl_wait.
 // four blocks of 32 x 8 per SM (64 registers): measured 17 % faster at
 // 513x257x257 than the three that 76 registers allow
+template <bool LAST>
 __global__ void __launch_bounds__(HBX *HBY, 4) k_helm_jac32v(Dims d, HelmTabF h, const uint8_t *__restrict__ st, float a_dt,
-                              const float *__restrict__ r, const float *__restrict__ e, float *__restrict__ en,
-                              int first)
+                              const float *__restrict__ r, const float *e, float *en, double *x)
 {
-    pdl_trigger();   // the immersed rows' kernel may start at once
     const int i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), j = blockIdx.y * blockDim.y + threadIdx.y;
+    pdl_wait();
+    pdl_trigger();   // the immersed rows' kernel, which reads e too, may start
     if (i0 >= d.NX || j >= d.NY) return;
     const float4 apx = *reinterpret_cast<const float4 *>(h.apx + i0);
     const float4 aw = *reinterpret_cast<const float4 *>(h.aw + i0);
@@ -273,44 +361,49 @@ __global__ void __launch_bounds__(HBX *HBY, 4) k_helm_jac32v(Dims d, HelmTabF h,
         const float rv[4] = {r4.x, r4.y, r4.z, r4.w};
         const float apzk = h.apz[k], abk = h.ab[k], afk = h.af[k];
         float out[4];
-        if (first) {
+        const float4 e4 = *reinterpret_cast<const float4 *>(e + p);
+        const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
+        const float xw = i0 > 0 ? e[p - 1] : ev[0];
+        const float xe = i0 + 4 < d.NX ? e[p + 4] : ev[3];
+        const float4 s_ = j > 0 ? *reinterpret_cast<const float4 *>(e + p - d.PX) : e4;
+        const float4 n_ = j < d.NY - 1 ? *reinterpret_cast<const float4 *>(e + p + d.PX) : e4;
+        const float4 b_ = k > 0 ? *reinterpret_cast<const float4 *>(e + p - d.plane) : e4;
+        const float4 f_ = k < d.NZ - 1 ? *reinterpret_cast<const float4 *>(e + p + d.plane) : e4;
+        const float sv_[4] = {s_.x, s_.y, s_.z, s_.w}, nv_[4] = {n_.x, n_.y, n_.z, n_.w};
+        const float bv_[4] = {b_.x, b_.y, b_.z, b_.w}, fv_[4] = {f_.x, f_.y, f_.z, f_.w};
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const bool stn = is_stencil(h.q, sv[t]);
-                const float dg = stn ? __fadd_rn(__fadd_rn(__fadd_rn(apxv[t], apyj), apzk), a_dt)
-                                     : __fadd_rn(h.ap_solid, a_dt);
-                out[t] = __fmul_rn(rv[t], __frcp_rn(dg));
+        for (int t = 0; t < 4; t++) {
+            const bool stn = is_stencil(h.q, sv[t]);
+            const float dg = stn ? __fadd_rn(__fadd_rn(__fadd_rn(apxv[t], apyj), apzk), a_dt)
+                                 : __fadd_rn(h.ap_solid, a_dt);
+            float acc = __fmul_rn(dg, ev[t]);
+            if (stn) {
+                acc = __fmaf_rn(awv[t], t == 0 ? xw : ev[t - 1], acc);
+                acc = __fmaf_rn(aev[t], t == 3 ? xe : ev[t + 1], acc);
+                acc = __fmaf_rn(asj, sv_[t], acc);
+                acc = __fmaf_rn(anj, nv_[t], acc);
+                acc = __fmaf_rn(abk, bv_[t], acc);
+                acc = __fmaf_rn(afk, fv_[t], acc);
             }
-        } else {
-            const float4 e4 = *reinterpret_cast<const float4 *>(e + p);
-            const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
-            const float xw = i0 > 0 ? e[p - 1] : ev[0];
-            const float xe = i0 + 4 < d.NX ? e[p + 4] : ev[3];
-            const float4 s_ = j > 0 ? *reinterpret_cast<const float4 *>(e + p - d.PX) : e4;
-            const float4 n_ = j < d.NY - 1 ? *reinterpret_cast<const float4 *>(e + p + d.PX) : e4;
-            const float4 b_ = k > 0 ? *reinterpret_cast<const float4 *>(e + p - d.plane) : e4;
-            const float4 f_ = k < d.NZ - 1 ? *reinterpret_cast<const float4 *>(e + p + d.plane) : e4;
-            const float sv_[4] = {s_.x, s_.y, s_.z, s_.w}, nv_[4] = {n_.x, n_.y, n_.z, n_.w};
-            const float bv_[4] = {b_.x, b_.y, b_.z, b_.w}, fv_[4] = {f_.x, f_.y, f_.z, f_.w};
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const bool stn = is_stencil(h.q, sv[t]);
-                const float dg = stn ? __fadd_rn(__fadd_rn(__fadd_rn(apxv[t], apyj), apzk), a_dt)
-                                     : __fadd_rn(h.ap_solid, a_dt);
-                float acc = __fmul_rn(dg, ev[t]);
-                if (stn) {
-                    acc = __fmaf_rn(awv[t], t == 0 ? xw : ev[t - 1], acc);
-                    acc = __fmaf_rn(aev[t], t == 3 ? xe : ev[t + 1], acc);
-                    acc = __fmaf_rn(asj, sv_[t], acc);
-                    acc = __fmaf_rn(anj, nv_[t], acc);
-                    acc = __fmaf_rn(abk, bv_[t], acc);
-                    acc = __fmaf_rn(afk, fv_[t], acc);
-                }
-                out[t] = __fmaf_rn(__fadd_rn(rv[t], -acc), __frcp_rn(dg), ev[t]);
-            }
+            out[t] = __fmaf_rn(__fadd_rn(rv[t], -acc), __frcp_rn(dg), ev[t]);
         }
         const bool ib4 = sv[0] == T_IMMERSED || sv[1] == T_IMMERSED || sv[2] == T_IMMERSED || sv[3] == T_IMMERSED;
-        if (nvalid == 4 && !ib4) {
+        const bool all = nvalid == 4 && !ib4;
+        if (LAST) {
+            if (all) {
+                double2 *xp = reinterpret_cast<double2 *>(x + p);
+                double2 lo = xp[0], hi = xp[1];
+                lo.x += to_f64(out[0]);
+                lo.y += to_f64(out[1]);
+                hi.x += to_f64(out[2]);
+                hi.y += to_f64(out[3]);
+                xp[0] = lo;
+                xp[1] = hi;
+            } else {
+                for (int t = 0; t < nvalid; t++)
+                    if (sv[t] != T_IMMERSED) x[p + t] += (double)out[t];
+            }
+        } else if (all) {
             *reinterpret_cast<float4 *>(en + p) = make_float4(out[0], out[1], out[2], out[3]);
         } else {
             for (int t = 0; t < nvalid; t++)
@@ -438,54 +531,22 @@ __global__ void __launch_bounds__(HBX *HBY, 3) k_helm_jac32z(Dims d, HelmTabF h,
     }
 }
 
-__global__ void k_helm_jac32(Dims d, HelmTabF h, const uint8_t *__restrict__ st, float a_dt,
-                             const float *__restrict__ r, const float *__restrict__ e, float *__restrict__ en,
-                             int first)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= d.NX || j >= d.NY) return;
-    for (int kk = 0; kk < KC; kk++) {
-        int k = blockIdx.z * KC + kk;
-        if (k >= d.NZ) break;
-        long long p = d.at(i, j, k);
-        int s = st[p];
-        if (s == T_IMMERSED) continue;
-        bool stencil = is_stencil(h.q, s);
-        float dg = stencil ? (h.apx[i] + h.apy[j] + h.apz[k] + a_dt) : (h.ap_solid + a_dt);
-        float inv = __frcp_rn(dg);
-        if (first) { en[p] = r[p] * inv; continue; }
-        float acc = dg * e[p];
-        if (stencil) {
-            Nb o = nb_of(d, i, j, k);
-            acc = fmaf(h.aw[i], e[p + o.w], acc);
-            acc = fmaf(h.ae[i], e[p + o.e], acc);
-            acc = fmaf(h.as[j], e[p + o.s], acc);
-            acc = fmaf(h.an[j], e[p + o.n], acc);
-            acc = fmaf(h.ab[k], e[p + o.b], acc);
-            acc = fmaf(h.af[k], e[p + o.f], acc);
-        }
-        en[p] = fmaf(r[p] - acc, inv, e[p]);
-    }
-}
-
 __global__ void k_ib_jac32(IbDevF ib, const float *__restrict__ r, const float *__restrict__ e,
-                           float *__restrict__ en, int first)
+                           float *__restrict__ en, double *__restrict__ x)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < ib.n) {
         long long im = ib.im[t];
         float inv = __frcp_rn(ib.diag[t]);
-        if (first) {
-            en[im] = r[im] * inv;
-        } else {
-            float acc = ib.diag[t] * e[im];
-            int c = ib.cnt[t];
-            for (int g = 0; g < c; g++) acc += ib.val[t * 8 + g] * e[ib.col[t * 8 + g]];
-            en[im] = fmaf(r[im] - acc, inv, e[im]);
-        }
+        float acc = ib.diag[t] * e[im];
+        int c = ib.cnt[t];
+        for (int g = 0; g < c; g++) acc += ib.val[t * 8 + g] * e[ib.col[t * 8 + g]];
+        const float v = fmaf(r[im] - acc, inv, e[im]);
+        if (x) x[im] += (double)v;
+        else en[im] = v;
     }
     // launched as a programmatic dependent of the stencil sweep (which
-    // writes the other points of en): end only after it has completed, so
+    // writes the other points): end only after it has completed, so
     // that the kernels after this one see both
     pdl_wait();
 }
@@ -498,14 +559,15 @@ inline dim3 hgrid(const Dims &d)
 
 constexpr int NPART = 1024;
 
-__global__ void k_norm2(long long n, const double *__restrict__ x, double *__restrict__ part)
+__global__ void k_norm2(long long n, long long stride, const double *__restrict__ x, double *__restrict__ part, const SumTo to)
 {
     double v = 0.0;
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
         v += x[p] * x[p];
     double s[1];
     block_sum256<1>({v}, s);
     if (threadIdx.x == 0) part[blockIdx.x] = s[0];
+    sum_to(part, to);
 }
 
 }  // namespace
@@ -516,8 +578,6 @@ long long helm_parts(const Dims &d)
     return (long long)g.x * g.y * g.z;
 }
 
-long long norm_parts() { return NPART; }
-
 void launch_helm_apply(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
                        const double *x, double *y, const IbDev &ib)
 {
@@ -525,30 +585,30 @@ void launch_helm_apply(cudaStream_t s, const Dims &d, const HelmTab &h, const ui
     if (ib.n > 0) k_ib_apply<<<(ib.n + 255) / 256, 256, 0, s>>>(ib, x, y);
 }
 
-// part must hold helm_parts(d) + (ib.n+255)/256 entries
+// part must hold helm_parts(d) + (ib.n+255)/256 entries; |r|^2 goes to *dst
 void launch_helm_jacobi(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
                         const double *b, const double *x, double *xn, const IbDev &ib, double *part,
-                        long long nparts)
+                        unsigned *count, double *dst)
 {
-    k_helm_jacobi<<<hgrid(d), dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, b, x, xn, part);
-    if (ib.n > 0) k_ib_jacobi<<<(ib.n + 255) / 256, 256, 0, s>>>(ib, b, x, xn, part + nparts);
+    const long long hp = helm_parts(d);
+    const unsigned nib = (unsigned)((ib.n + 255) / 256);
+    const SumTo to{(int)(hp + nib), (unsigned)hp + nib, count, dst};
+    k_helm_jacobi<<<hgrid(d), dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, b, x, xn, part, to);
+    if (ib.n > 0) k_ib_jacobi<<<nib, 256, 0, s>>>(ib, b, x, xn, part, hp, to);
 }
 
-void launch_sum_final(cudaStream_t s, long long nparts, const double *part, double *out)
+// |x|^2 to *dst
+void launch_norm2(cudaStream_t s, long long n, const double *x, double *part, unsigned *count, double *dst)
 {
-    k_sum_final<<<1, 1024, 0, s>>>(nparts, part, out);
+    // blocks without elements would add zeros
+    const long long want = (n + 255) / 256;
+    const int nb = (int)(want < NPART ? (want > 0 ? want : 1) : NPART);
+    k_norm2<<<nb, 256, 0, s>>>(n, (long long)NPART * 256, x, part, SumTo{nb, (unsigned)nb, count, dst});
 }
 
-void launch_norm2(cudaStream_t s, long long n, const double *x, double *part, long long nparts, double *out)
+void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e)
 {
-    (void)nparts;
-    k_norm2<<<NPART, 256, 0, s>>>(n, x, part);
-    k_sum_final<<<1, 1024, 0, s>>>(NPART, part, out);
-}
-
-void launch_add_corr(cudaStream_t s, long long n, const double *x, const float *e, double *xn)
-{
-    k_add_corr<<<1216, 256, 0, s>>>(n, x, e, xn);
+    k_add_corr<<<1216, 256, 0, s>>>(n, x, e);
 }
 
 // a launch with the programmatic stream serialisation attribute: the kernel
@@ -570,30 +630,43 @@ static void launch_pdl(void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... arg
     cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
-                         const double *b, const double *x, float *rf, const IbDev &ib, double *part,
-                         long long nparts)
+// |r|^2 goes to *dst, the first sweep's result to e0
+void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
+                         const double *b, const double *x, float *rf, float *e0, const IbDev &ib, const IbDevF &ibf,
+                         double *part, unsigned *count, double *dst)
 {
-    k_helm_resid64<<<hgrid(d), dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, b, x, rf, part);
-    if (ib.n > 0) launch_pdl(k_ib_resid64, dim3((ib.n + 255) / 256), dim3(256), s, ib, b, x, rf, part + nparts);
+    const long long hp = helm_parts(d);
+    const unsigned nib = (unsigned)((ib.n + 255) / 256);
+    // groups per block: as many as leave about seven blocks per SM
+    const int g = hp >= 4096 ? 4 : hp >= 2048 ? 2 : hp > 2 * 152 ? 1 : 0;
+    dim3 gr = hgrid(d);
+    if (g) gr.z = (gr.z + g - 1) / g;
+    const SumTo to{(int)(hp + nib), gr.x * gr.y * gr.z + nib, count, dst};
+    const auto k = g == 4 ? k_helm_resid64<4> : g == 2 ? k_helm_resid64<2> : g == 1 ? k_helm_resid64<1> : k_helm_resid64<0>;
+    k<<<gr, dim3(HBX, HBY), 0, s>>>(d, h, hf, st, a_dt, b, x, rf, e0, part, to);
+    if (ib.n > 0) launch_pdl(k_ib_resid64, dim3(nib), dim3(256), s, ib, ibf, b, x, rf, e0, part, hp, to);
 }
 
-// marching 1: the FP32 Jacobi sweeps after the first march along k through
-// shared-memory plane tiles (k_helm_jac32z); 0: k_helm_jac32v throughout
+// The sweep after the first ones: from e to en, or (x given) added to x.
+// alone: the kernel ahead of it on the stream is not a sweep.  marching 1: the
+// sweeps but the last march along k through shared-memory plane tiles
+// (k_helm_jac32z); 0: k_helm_jac32v throughout
 void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, float a_dt,
-                       const float *r, const float *e, float *en, const IbDevF &ib, int first, int marching)
+                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching)
 {
     dim3 g((unsigned)((d.NX + 4 * HBX - 1) / (4 * HBX)), (unsigned)((d.NY + HBY - 1) / HBY),
            (unsigned)((d.NZ + KCJ - 1) / KCJ));
-    if (!first && marching) {
+    if (!x && marching) {
         dim3 gz((unsigned)((d.NX + 4 * HBX - 1) / (4 * HBX)), (unsigned)((d.NY + HBY - 1) / HBY),
                 (unsigned)((d.NZ + JZ - 1) / JZ));
         k_helm_jac32z<<<gz, dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, r, e, en);
         // k_helm_jac32z writes placeholders at immersed points: the immersed
         // rows go after it in plain stream order
-        if (ib.n > 0) k_ib_jac32<<<(ib.n + 255) / 256, 256, 0, s>>>(ib, r, e, en, first);
+        if (ib.n > 0) k_ib_jac32<<<(ib.n + 255) / 256, 256, 0, s>>>(ib, r, e, en, x);
         return;
     }
-    k_helm_jac32v<<<g, dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, r, e, en, first);
-    if (ib.n > 0) launch_pdl(k_ib_jac32, dim3((ib.n + 255) / 256), dim3(256), s, ib, r, e, en, first);
+    const auto k = x ? k_helm_jac32v<true> : k_helm_jac32v<false>;
+    if (alone || marching) k<<<g, dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, r, e, en, x);
+    else launch_pdl(k, g, dim3(HBX, HBY), s, d, h, st, a_dt, r, e, en, x);
+    if (ib.n > 0) launch_pdl(k_ib_jac32, dim3((ib.n + 255) / 256), dim3(256), s, ib, r, e, en, x);
 }

@@ -102,7 +102,7 @@ struct DevBuf {
 // and the row's result.
 constexpr double ENO_X_BYTES = 24.0, ENO_YZ_BYTES = 32.0;
 constexpr double HELM_JACOBI_BYTES = 25.0, HELM_RESID64_BYTES = 21.0;
-constexpr double HELM_JAC32_FIRST_BYTES = 9.0, HELM_JAC32_BYTES = 13.0;
+constexpr double HELM_JAC32_BYTES = 13.0;
 constexpr double IB_ROW_BYTES = 8.0 + 4.0 + 8.0 * (4.0 + 8.0 + 8.0) + 8.0 + 8.0;
 
 struct turb_ctx {
@@ -160,6 +160,7 @@ struct turb_ctx {
     cudaGraphExec_t g_pcg[2] = {nullptr, nullptr};
     cudaGraphExec_t g_inner[3 + TURB_MAXCONC] = {nullptr};
     int g_inner_n[3 + TURB_MAXCONC] = {0};
+    double *g_inner_x[3 + TURB_MAXCONC] = {nullptr};
     int use_graphs = 1;
     // red-black Gauss-Seidel sweeps before / after the coarse correction per
     // level (0 = the finest) and pressure mode, set in turb_create
@@ -2377,6 +2378,9 @@ static double diag_term(turb_ctx *c, int sys, double dt)
     return a;
 }
 
+// |b|^2 and |r|^2 of a Helmholtz solve, written by the kernels to page-locked memory
+constexpr int HS_B = 4, HS_R = 5;
+
 static int helm_solve_fp64(turb_ctx *c, int q, int ic, int fx, int fb, double dt, int *iters)
 {
     const Dims &d = c->d;
@@ -2384,24 +2388,17 @@ static int helm_solve_fp64(turb_ctx *c, int q, int ic, int fx, int fb, double dt
     const IbDev &ib = c->ib[q];
     double a_dt = diag_term(c, q < 3 ? q : 3 + ic, dt);
     double *b = c->fld[fb];
-    launch_norm2(c->s, d.n, b, c->part, norm_parts(), c->dscal);
-    int rc = fetch_scalars(c, 1);
-    if (rc) return rc;
-    double nb = std::sqrt(c->hscal[0]);
-    long long hp = helm_parts(d);
-    long long np = hp + (ib.n > 0 ? (ib.n + 255) / 256 : 0);
+    launch_norm2(c->s, d.n, b, c->part, c->count, c->hscal + HS_B);
     int it = 0;
-    c->launches += 2;
+    c->launches += 1;
     for (;;) {
         double *x = c->fld[fx];
         int ph = prof_begin(c, TURB_PROF_JACOBI);
-        launch_helm_jacobi(c->s, d, h, c->st[q], a_dt, b, x, c->jtmp, ib, c->part, hp);
+        launch_helm_jacobi(c->s, d, h, c->st[q], a_dt, b, x, c->jtmp, ib, c->part, c->count, c->hscal + HS_R);
         prof_end(c, ph, 1, HELM_JACOBI_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
-        launch_sum_final(c->s, np, c->part, c->dscal);
-        c->launches += 2 + (ib.n > 0);
-        rc = fetch_scalars(c, 1);
-        if (rc) return rc;
-        double nr = std::sqrt(c->hscal[0]);
+        c->launches += 1 + (ib.n > 0);
+        TURB_CHECK(cudaStreamSynchronize(c->s));
+        double nb = std::sqrt(c->hscal[HS_B]), nr = std::sqrt(c->hscal[HS_R]);
         if (!std::isfinite(nr)) { if (iters) *iters = it; return TURB_ERR_NAN; }
         if (nr <= c->prm.vel_rtol * nb) break;
         if (it >= c->prm.vel_maxit) { if (iters) *iters = it; return TURB_ERR_NOT_CONVERGED; }
@@ -2414,8 +2411,9 @@ static int helm_solve_fp64(turb_ctx *c, int q, int ic, int fx, int fb, double dt
 }
 
 // FP64 defect correction with FP32 inner Jacobi sweeps: every outer step
-// forms x <- x + e and r = b - A x in FP64 (the convergence test is on this
-// FP64 residual), then approximately solves A e = r with hinner FP32 sweeps.
+// forms r = b - A x in FP64 (the convergence test is on this FP64 residual)
+// and the first of hinner FP32 sweeps on A e = r, then runs the others, the
+// last of which adds e to x.
 static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double dt, int *iters)
 {
     const Dims &d = c->d;
@@ -2424,30 +2422,18 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
     const IbDev &ib = c->ib[q];
     const IbDevF &ibf = c->ibf[q];
     double a_dt = diag_term(c, q < 3 ? q : 3 + ic, dt);
-    double *b = c->fld[fb];
-    launch_norm2(c->s, d.n, b, c->part, norm_parts(), c->dscal);
-    int rc = fetch_scalars(c, 1);
-    if (rc) return rc;
-    double nb = std::sqrt(c->hscal[0]);
-    long long hp = helm_parts(d);
-    long long np = hp + (ib.n > 0 ? (ib.n + 255) / 256 : 0);
+    double *b = c->fld[fb], *x = c->fld[fx];
+    launch_norm2(c->s, d.n, b, c->part, c->count, c->hscal + HS_B);
     int it = 0;
-    c->launches += 2;
-    float *e = c->he0, *en = c->he1;
+    c->launches += 1;
     for (;;) {
-        if (it > 0) {
-            launch_add_corr(c->s, d.n, c->fld[fx], e, c->jtmp);   // x <- x + e
-            std::swap(c->fld[fx], c->jtmp);
-            c->launches += 1;
-        }
         int ph = prof_begin(c, TURB_PROF_JACOBI);
-        launch_helm_resid64(c->s, d, h, c->st[q], a_dt, b, c->fld[fx], c->hrf, ib, c->part, hp);
+        launch_helm_resid64(c->s, d, h, hf, c->st[q], a_dt, b, x, c->hrf, c->he0, ib, ibf, c->part, c->count,
+                            c->hscal + HS_R);
         prof_end(c, ph, 1, HELM_RESID64_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
-        launch_sum_final(c->s, np, c->part, c->dscal);
-        c->launches += 2 + (ib.n > 0);
-        rc = fetch_scalars(c, 1);
-        if (rc) return rc;
-        double nr = std::sqrt(c->hscal[0]);
+        c->launches += 1 + (ib.n > 0);
+        TURB_CHECK(cudaStreamSynchronize(c->s));
+        double nb = std::sqrt(c->hscal[HS_B]), nr = std::sqrt(c->hscal[HS_R]);
         if (!std::isfinite(nr)) { if (iters) *iters = it; return TURB_ERR_NAN; }
         if (nr <= c->prm.vel_rtol * nb) break;
         if (it >= c->prm.vel_maxit) { if (iters) *iters = it; return TURB_ERR_NOT_CONVERGED; }
@@ -2455,27 +2441,35 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
         int gi = q < 3 ? q : 3 + ic;
         auto sweeps = [&]() {
             float *ea = c->he0, *eb = c->he1;
-            for (int t = 0; t < c->hinner; t++) {
-                launch_helm_jac32(c->s, d, hf, c->st[q], (float)a_dt, c->hrf, ea, eb, ibf, t == 0,
-                                  c->kvariant & TURB_KV_MARCHING);
+            for (int t = 1; t < c->hinner; t++) {
+                launch_helm_jac32(c->s, d, hf, c->st[q], (float)a_dt, c->hrf, ea, eb, t == c->hinner - 1 ? x : nullptr, ibf,
+                                  t == 1, c->kvariant & TURB_KV_MARCHING);
                 std::swap(ea, eb);
             }
         };
-        if (c->use_graphs) {
-            if (c->g_inner[gi] && c->g_inner_n[gi] != c->hinner) { cudaGraphExecDestroy(c->g_inner[gi]); c->g_inner[gi] = nullptr; }
-            if (!c->g_inner[gi]) { int rc2 = capture(c, &c->g_inner[gi], sweeps); if (rc2) return rc2; c->g_inner_n[gi] = c->hinner; }
+        if (c->hinner == 1) {
+            launch_add_corr(c->s, d.n, x, c->he0);
+            c->launches += 1;
+        } else if (c->use_graphs) {
+            // a graph holds the number of sweeps and the address of x (an FP64 solve swaps it)
+            if (c->g_inner[gi] && (c->g_inner_n[gi] != c->hinner || c->g_inner_x[gi] != x)) {
+                cudaGraphExecDestroy(c->g_inner[gi]);
+                c->g_inner[gi] = nullptr;
+            }
+            if (!c->g_inner[gi]) {
+                int rc2 = capture(c, &c->g_inner[gi], sweeps);
+                if (rc2) return rc2;
+                c->g_inner_n[gi] = c->hinner;
+                c->g_inner_x[gi] = x;
+            }
             TURB_CHECK(cudaGraphLaunch(c->g_inner[gi], c->s));
         } else {
             sweeps();
         }
-        // the sweeps start from he0 and alternate; the result is in he0 after
-        // an even number of sweeps
-        e = (c->hinner % 2 == 0) ? c->he0 : c->he1;
-        en = (e == c->he0) ? c->he1 : c->he0;
-        prof_end(c, ph, c->hinner,
-                 (HELM_JAC32_FIRST_BYTES + HELM_JAC32_BYTES * (c->hinner - 1)) * ((double)d.NX * d.NY * d.NZ) +
+        prof_end(c, ph, c->hinner - 1,
+                 (HELM_JAC32_BYTES * (c->hinner - 1) + 12.0) * ((double)d.NX * d.NY * d.NZ) +
                      IB_ROW_BYTES * 0.5 * ibf.n * c->hinner);
-        c->launches += c->hinner * (1 + (ib.n > 0));
+        c->launches += (c->hinner - 1) * (1 + (ib.n > 0));
         it++;
     }
     if (iters) *iters = it;

@@ -66,14 +66,12 @@ void launch_helm_apply(cudaStream_t s, const Dims &d, const HelmTab &h, const ui
                        const double *x, double *y, const IbDev &ib);
 void launch_helm_jacobi(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
                         const double *b, const double *x, double *xn, const IbDev &ib, double *part,
-                        long long nparts);
+                        unsigned *count, double *dst);
 long long helm_parts(const Dims &d);
-void launch_add_corr(cudaStream_t s, long long n, const double *x, const float *e, double *xn);
-void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
-                         const double *b, const double *x, float *rf, const IbDev &ib, double *part,
-                         long long nparts);
+void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e);
+void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
+                         const double *b, const double *x, float *rf, float *e0, const IbDev &ib, const IbDevF &ibf,
+                         double *part, unsigned *count, double *dst);
 void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, float a_dt,
-                       const float *r, const float *e, float *en, const IbDevF &ib, int first, int marching);
-void launch_sum_final(cudaStream_t s, long long nparts, const double *part, double *out);
-void launch_norm2(cudaStream_t s, long long n, const double *x, double *part, long long nparts, double *out);
-long long norm_parts();
+                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching);
+void launch_norm2(cudaStream_t s, long long n, const double *x, double *part, unsigned *count, double *dst);
