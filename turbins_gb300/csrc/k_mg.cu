@@ -131,6 +131,120 @@ __global__ void k_rbgs(MgDevLevel Ld, int color, int zero_init, const T *__restr
     rb_cell<T>(L, zero_init, b, invd, x, i, j, k);
 }
 
+// ---- FP64 kernels of the large levels, marching planes of k -------------------
+// Of a cell's FP64 operations (17 of a half sweep, 29 of a residual) most form
+// its coefficients, which along k change only where dz or the face distances
+// do.  A thread keeps those of its columns and forms them again when a plane's
+// differ from those two planes (half sweep) or one plane (residual) before, so
+// uniform planes cost eight or nine; the values and their order are s_row's.
+template <typename T>
+struct ColCoef {
+    T f[6];
+    __device__ __forceinline__ void form(const LevelT<T> &L, int i, int j, int k)
+    {
+        const T dy = L.dy[j], dz = L.dz[k], dx = L.dx[i];
+        const T dyz = rmul(dy, dz), dxz = rmul(dx, dz), dxy = rmul(dx, dy);
+        f[0] = i > 0 ? rmul(dyz, L.rfx[i]) : T(0);
+        f[1] = i < L.nx - 1 ? rmul(dyz, L.rfx[i + 1]) : T(0);
+        f[2] = j > 0 ? rmul(dxz, L.rfy[j]) : T(0);
+        f[3] = j < L.ny - 1 ? rmul(dxz, L.rfy[j + 1]) : T(0);
+        f[4] = k > 0 ? rmul(dxy, L.rfz[k]) : T(0);
+        f[5] = k < L.nz - 1 ? rmul(dxy, L.rfz[k + 1]) : T(0);
+    }
+};
+// plane k's coefficients are not plane k - s's
+template <typename T>
+__device__ __forceinline__ bool planes_differ(const LevelT<T> &L, int k, int s)
+{
+    if (k - s <= 0 || k >= L.nz - 1) return true;
+    return L.dz[k] != L.dz[k - s] || L.rfz[k] != L.rfz[k - s] || L.rfz[k + 1] != L.rfz[k + 1 - s];
+}
+
+// The half sweep: a thread alternates between the columns i = 2 m, 2 m + 1.
+// Two planes are loaded before either is stored (the cells read are of the
+// colour that is not written; x and b are not __restrict__, so nothing is read
+// before pdl_wait).
+template <typename T>
+__global__ void __launch_bounds__(256, 3) k_rbgs_col(MgDevLevel Ld, int color, int planes, const T *b, const T *__restrict__ invd, T *x)
+{
+    pdl_trigger();
+    pdl_wait();
+    const LevelT<T> L = lev_of<T>(Ld);
+    const int m = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const int k0 = blockIdx.z * planes, k1 = min(k0 + planes, L.nz);
+    if (j >= L.ny || 2 * m >= L.nx) return;
+    const int p0 = (j + k0 + color) & 1;   // the first plane's cell is i = 2 m + p0
+    const long long nxy = (long long)L.nx * L.ny;
+    ColCoef<T> f[2];
+    for (int k2 = k0; k2 < k1; k2 += 2) {
+        T xv[2][6], bv[2], iv[2];
+        long long at[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int k = min(k2 + c, L.nz - 1), i = 2 * m + (k2 + c < L.nz ? p0 ^ c : p0);   // a plane past the last is not stored
+            const long long n = ((long long)k * L.ny + j) * L.nx + i;
+            at[c] = L.at(n, i, j, k);
+            bv[c] = b[at[c]];
+            iv[c] = invd[at[c]];
+            // an absent neighbour has a zero coefficient and the value of another cell of its colour
+            const int iw = i > 0 ? -1 : 1, ie = i < L.nx - 1 ? 1 : -1;
+            xv[c][0] = x[L.at(n + iw, i + iw, j, k)];
+            xv[c][1] = x[L.at(n + ie, i + ie, j, k)];
+            xv[c][2] = j > 0 ? x[L.at(n - L.nx, i, j - 1, k)] : xv[c][0];
+            xv[c][3] = j < L.ny - 1 ? x[L.at(n + L.nx, i, j + 1, k)] : xv[c][0];
+            xv[c][4] = k > 0 ? x[L.at(n - nxy, i, j, k - 1)] : xv[c][0];
+            xv[c][5] = k < L.nz - 1 ? x[L.at(n + nxy, i, j, k + 1)] : xv[c][0];
+        }
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int k = k2 + c;
+            if (k >= k1) break;
+            if (k2 == k0 || planes_differ(L, k, 2)) f[c].form(L, 2 * m + (p0 ^ c), j, k);
+            T o = rfma(f[c].f[0], xv[c][0], T(0));
+#pragma unroll
+            for (int e = 1; e < 6; e++) o = rfma(f[c].f[e], xv[c][e], o);
+            x[at[c]] = rmul(radd(bv[c], o), iv[c]);
+        }
+    }
+}
+
+// the residual r = b - S x (r in natural order) of a column of cells
+template <typename T>
+__global__ void __launch_bounds__(256, 4) k_resid_col(MgDevLevel Ld, int planes, const T *b, const T *x, T *r)
+{
+    pdl_trigger();
+    pdl_wait();
+    const LevelT<T> L = lev_of<T>(Ld);
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const int k0 = blockIdx.z * planes, k1 = min(k0 + planes, L.nz);
+    if (i >= L.nx || j >= L.ny) return;
+    const long long nxy = (long long)L.nx * L.ny;
+    ColCoef<T> f;
+    T dg = 0;
+    long long n = ((long long)k0 * L.ny + j) * L.nx + i;
+    T xc = x[L.at(n, i, j, k0)], xb = k0 > 0 ? x[L.at(n - nxy, i, j, k0 - 1)] : xc;
+    for (int k = k0; k < k1; k++, n += nxy) {
+        const T bc = b[L.at(n, i, j, k)];
+        const T xw = i > 0 ? x[L.at(n - 1, i - 1, j, k)] : xc, xe = i < L.nx - 1 ? x[L.at(n + 1, i + 1, j, k)] : xc;
+        const T xs = j > 0 ? x[L.at(n - L.nx, i, j - 1, k)] : xc, xn = j < L.ny - 1 ? x[L.at(n + L.nx, i, j + 1, k)] : xc;
+        const T xf = k < L.nz - 1 ? x[L.at(n + nxy, i, j, k + 1)] : xc;
+        if (k == k0 || planes_differ(L, k, 1)) {
+            f.form(L, i, j, k);
+            dg = radd(radd(radd(radd(radd(f.f[0], f.f[1]), f.f[2]), f.f[3]), f.f[4]), f.f[5]);
+            if (i == L.nx - 1 && j == L.ny - 1 && k == L.nz - 1) dg = radd(dg, L.pin);
+        }
+        T o = rfma(f.f[0], xw, T(0));
+        o = rfma(f.f[1], xe, o);
+        o = rfma(f.f[2], xs, o);
+        o = rfma(f.f[3], xn, o);
+        o = rfma(f.f[4], xb, o);
+        o = rfma(f.f[5], xf, o);
+        r[n] = radd(bc, -rfma(dg, xc, -o));
+        xb = xc;
+        xc = xf;
+    }
+}
+
 // The same half sweep on colour-split FP32 storage, four cells of one row per
 // thread (nx a multiple of 8) in each of `planes` planes (2 on the large
 // levels, 1 on the small ones, whose launches are latency-bound and need
@@ -516,6 +630,19 @@ __device__ __forceinline__ void prolong_cell(const MgDevLevel &Lf, const MgDevLe
 {
     long long c = ((long long)k * Lf.ny + j) * Lf.nx + i;
     int Ix[2] = {Lf.tx.I0[i], Lf.tx.I1[i]}, Iy[2] = {Lf.ty.I0[j], Lf.ty.I1[j]}, Iz[2] = {Lf.tz.I0[k], Lf.tz.I1[k]};
+    if (Lc.nx == Lf.nx) {   // the upper x weights are 0, the lower 1: half the terms, the same sum
+        T acc = 0;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int J = Iy[e & 1], K = Iz[e >> 1];
+            const T v = xc[lev_at(Lc, ((long long)K * Lc.ny + J) * Lc.nx + i, i, J, K)];
+            acc = mg_fma(mg_mul(e & 2 ? pw1_of<T>(Lf.tz)[k] : pw0_of<T>(Lf.tz)[k], e & 1 ? pw1_of<T>(Lf.ty)[j] : pw0_of<T>(Lf.ty)[j]),
+                         v, acc);
+        }
+        const long long o = lev_at(Lf, c, i, j, k);
+        xf[o] = radd(xf[o], acc);
+        return;
+    }
     T val[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
@@ -947,6 +1074,16 @@ const dim3 B38(32, 8, 1);
 
 }  // namespace
 
+// planes a block of the marching FP64 kernels takes of a launch of g blocks,
+// one per plane: the most (up to 8) that leave two blocks per SM, 0 where two
+// planes leave fewer
+static int col_planes(dim3 g)
+{
+    int planes = 8;
+    while (planes > 2 && (long long)g.x * g.y * ((g.z + planes - 1) / planes) < 2 * 152) planes >>= 1;
+    return (long long)g.x * g.y * ((g.z + planes - 1) / planes) >= 2 * 152 ? planes : 0;
+}
+
 template <typename T>
 void mg_setup_invdiag(cudaStream_t s, const MgDevLevel &L, T *invd)
 {
@@ -995,6 +1132,15 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
             return;
         }
     }
+    if constexpr (sizeof(T) == 8) {
+        dim3 g = g3(L.nx >> 1, L.ny, L.nz);
+        const int planes = col_planes(g);
+        if (!zero_init && L.nx % 2 == 0 && planes) {
+            g.z = (g.z + planes - 1) / planes;
+            launch_k(pdl, k_rbgs_col<T>, g, B38, s, L, color, planes, b, invd, x);
+            return;
+        }
+    }
     launch_k(pdl, k_rbgs<T>, g3((L.nx + 1) >> 1, L.ny, L.nz), B38, s, L, color, zero_init, b, invd, x);
 }
 
@@ -1005,6 +1151,15 @@ void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r
         if (L.split && L.nx % 8 == 0) {
             dim3 g8((unsigned)((L.nx / 8 + 31) / 32), (unsigned)((L.ny + 7) / 8), (unsigned)L.nz);
             launch_k(pdl, k_resid8, g8, B38, s, L, b, x, r);
+            return;
+        }
+    }
+    if constexpr (sizeof(T) == 8) {
+        const int planes = col_planes(g3(L.nx, L.ny, L.nz));
+        if (planes) {
+            dim3 g = g3(L.nx, L.ny, L.nz);
+            g.z = (g.z + planes - 1) / planes;
+            launch_k(pdl, k_resid_col<T>, g, B38, s, L, planes, b, x, r);
             return;
         }
     }
