@@ -54,7 +54,8 @@ def test_umma_swizzle128_mn_row_shift(shift):
 
 
 @pytest.mark.parametrize("X,Y,Z,cin,cout", [(16, 1, 1, 16, 16), (8, 2, 3, 32, 32), (64, 7, 9, 16, 16), (62, 8, 21, 16, 32),
-                                            (128, 5, 3, 16, 16), (256, 3, 2, 32, 32), (160, 4, 5, 32, 16)])
+                                            (128, 5, 3, 16, 16), (256, 3, 2, 32, 32), (160, 4, 5, 32, 16),
+                                            (128, 64, 100, 16, 16)])
 def test_wgrad_tiles(X, Y, Z, cin, cout):
     from turbins_gb300 import build
     build.build()

@@ -61,11 +61,11 @@ const char *conv_last_error();
 // writes anything the others do, pdl_wait; the first kernel of a pass is an
 // ordinary launch, so what was written before the pass is visible to all
 template <typename... P, typename... A>
-inline void net_launch(void (*k)(P...), int gx, int gy, int threads, uint32_t smem, cudaStream_t s, A... args)
+inline void net_launch(void (*k)(P...), dim3 grid, dim3 block, uint32_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
-    cfg.blockDim = dim3((unsigned)threads);
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -74,4 +74,9 @@ inline void net_launch(void (*k)(P...), int gx, int gy, int threads, uint32_t sm
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+template <typename... P, typename... A>
+inline void net_launch(void (*k)(P...), int gx, int gy, int threads, uint32_t smem, cudaStream_t s, A... args)
+{
+    net_launch(k, dim3((unsigned)gx, (unsigned)gy), dim3((unsigned)threads), smem, s, args...);
 }
