@@ -82,6 +82,24 @@ __device__ __forceinline__ void sum_parts(const double *part, long long stride, 
 {
     __shared__ double sm[NVAL][1024];
     const int lt = threadIdx.y * blockDim.x + threadIdx.x, lane = lt & 31;
+    if (nblk <= 256) {
+        // one partial per thread of the first eight of the 32 warps: their
+        // shuffle trees and one over the warps, a barrier instead of seven
+#pragma unroll
+        for (int v = 0; v < NVAL; v++) {
+            const double r = warp_sum(lt < nblk ? __ldcg(part + v * stride + lt) : 0.0);
+            if (lane == 0) sm[v][lt >> 5] = r;
+        }
+        __syncthreads();
+        if (lt < 32) {
+#pragma unroll
+            for (int v = 0; v < NVAL; v++) {
+                const double r = warp_sum(lane < 8 ? sm[v][lane] : 0.0);
+                if (lt == 0) dst[v] = r;
+            }
+        }
+        return;
+    }
     // the 1024 threads' sums, four per thread of this block of 256
 #pragma unroll
     for (int v = 0; v < NVAL; v++)
