@@ -1,0 +1,73 @@
+"""Kernels that start before the one ahead of them has ended (those that call
+pdl_wait) read what it writes only after the wait.
+
+A load through a kernel argument declared __restrict__ does not have that
+order: the declaration promises that nothing else writes the data while the
+kernel runs, so the compiler may move the load above the wait, whose memory
+clobber covers only data that others can reach.  Such a kernel may therefore
+declare __restrict__ only on what is written before every kernel that can still
+run beside it: the tables listed in SETTLED, per kernel where the reason is
+its own.  The order cannot be observed by running the kernels (the present
+code generation may keep it), so the declarations are read.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "turbins_gb300", "csrc")
+FILES = ["k_pcg.cu"]
+
+# const tables formed when a context is created
+SETTLED = {"*": {"invd", "ainv", "st"}}
+
+
+def kernels(path):
+    """(name, parameters, body) of every __global__ function of a file"""
+    src = open(path).read()
+    src = re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", src, flags=re.S))
+
+    def close(at, pair):
+        depth = 0
+        for n in range(at, len(src)):
+            depth += (src[n] == pair[0]) - (src[n] == pair[1])
+            if depth == 0:
+                return n
+        raise AssertionError("unbalanced %s in %s" % (pair, path))
+
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__)?", src):
+        at = m.end()
+        if src[at] == "(":
+            at = close(at, "()") + 1
+        op = src.index("(", at)
+        cp = close(op, "()")
+        ob = src.index("{", cp)
+        yield src[at:op].strip(), src[op + 1:cp], src[ob:close(ob, "{}") + 1]
+
+
+def unsettled(name, params):
+    """arguments of a kernel whose loads may pass its wait"""
+    bad = []
+    for p in params.split(","):
+        m = re.search(r"__restrict__\s*(\w+)", p)
+        if m and not (("const" in p and m.group(1) in SETTLED["*"]) or m.group(1) in SETTLED.get(name, ())):
+            bad.append(m.group(1))
+    return bad
+
+
+def test_the_reader_finds_a_planted_mistake(tmp_path):
+    f = tmp_path / "k.cu"
+    f.write_text("template <int G>\n__global__ void __launch_bounds__(256, G ? 4 : 2) k_a(L l, const double *__restrict__ p, const\n"
+                 " float *__restrict__ invd, double *q) // pdl\n{ pdl_wait(); { q[0] = p[0]; } }\n"
+                 "__global__ void k_b(const double *__restrict__ p) { /* pdl_wait */ }\n")
+    ks = list(kernels(str(f)))
+    assert [k[0] for k in ks] == ["k_a", "k_b"]
+    assert unsettled(*ks[0][:2]) == ["p"]
+    assert "pdl_wait" in ks[0][2] and "pdl_wait" not in ks[1][2]
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_no_restrict_on_what_the_kernel_ahead_writes(name):
+    early = [k for k in kernels(os.path.join(CSRC, name)) if "pdl_wait" in k[2]]
+    assert early
+    assert {k[0]: unsettled(k[0], k[1]) for k in early if unsettled(k[0], k[1])} == {}

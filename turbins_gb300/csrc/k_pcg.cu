@@ -99,9 +99,10 @@ __device__ __forceinline__ void s_planes(const MgDevLevel &L, SPlane *sp, int k0
 // column.  A block of G groups forms the column's coefficients (eight FP64
 // operations) once for 4 G cells and reads the cells above and below as the
 // march reaches them; each group's sum is stored apart, so the partials are
-// those of blocks of one group.
+// those of blocks of one group.  x is not __restrict__: k_apply starts before
+// the kernel that writes it has ended.
 template <int G, typename F>
-__device__ __forceinline__ void s_march(const MgDevLevel &L, const double *__restrict__ x, F f)
+__device__ __forceinline__ void s_march(const MgDevLevel &L, const double *x, F f)
 {
     __shared__ SPlane sp[KC * G];
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -182,10 +183,13 @@ __global__ void k_resid(MgDevLevel L, const double *__restrict__ bw, const doubl
     if (count && last_block(count, gridDim.x * gridDim.y * gridDim.z)) sum_parts<1>(part, 0, nparts, dst);
 }
 
+// The kernels of a CG step start before the one ahead of them has ended, so
+// the vectors they read are not __restrict__: through such a pointer the
+// compiler may load what that kernel is still writing before pdl_wait.
+
 // q = S p with partial p.q per group of planes, then alpha = rz / p.q
 template <int G>
-__global__ void k_apply(MgDevLevel L, const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part,
-                        int nparts, PcgScal *sc, unsigned *count)
+__global__ void k_apply(MgDevLevel L, const double *p, double *q, double *part, int nparts, PcgScal *sc, unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
@@ -244,8 +248,8 @@ __global__ void k_dot(long long n, int nvb, const double *__restrict__ a, const 
 }
 
 // rz = r.z and zr_old = z.r_old, then beta (0 on a restart)
-__global__ void __launch_bounds__(BS, 4) k_dot2(long long n, int nvb, const double *__restrict__ r, const double *__restrict__ z,
-                       const double *__restrict__ ro, double *__restrict__ part, PcgScal *sc, int restart, unsigned *count)
+__global__ void __launch_bounds__(BS, 4) k_dot2(long long n, int nvb, const double *r, const double *z, const double *ro,
+                                                   double *part, PcgScal *sc, int restart, unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
@@ -283,8 +287,7 @@ __global__ void k_reduce(const double *__restrict__ part, int nvals, int nper, d
     }
 }
 
-__global__ void k_pupdate(long long n, int nvb, const double *__restrict__ z, double *__restrict__ p, const PcgScal *sc,
-                          int first)
+__global__ void k_pupdate(long long n, int nvb, const double *z, double *p, const PcgScal *sc, int first)
 {
     pdl_trigger();
     pdl_wait();
@@ -308,9 +311,9 @@ __global__ void k_pupdate(long long n, int nvb, const double *__restrict__ z, do
 }
 
 // x += alpha p, r_old = r, r -= alpha q and |r|^2
-__global__ void __launch_bounds__(BS, 3) k_xrupdate(long long n, int nvb, double *__restrict__ x, double *__restrict__ r,
-                           double *__restrict__ ro, const double *__restrict__ p, const double *__restrict__ q,
-                           PcgScal *sc, double *__restrict__ part, double *host_rr, unsigned *count)
+__global__ void __launch_bounds__(BS, 3) k_xrupdate(long long n, int nvb, double *x, double *r, double *ro, const double *p,
+                                                       const double *q, PcgScal *sc, double *part, double *host_rr,
+                                                       unsigned *count)
 {
     pdl_trigger();
     pdl_wait();
