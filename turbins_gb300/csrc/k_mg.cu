@@ -12,6 +12,11 @@
 // directions whose mean spacing is more than twice the finest, and a dense
 // inverse on the coarsest (<= 64 cells) level.  The V-cycle is templated on
 // its precision: FP64 (plain method) or FP32 inside the FP64 CG (mixed).
+//
+// The cycle's kernels start before the one ahead of them has ended (pdl_wait),
+// so their arguments are __restrict__ only where set-up wrote the data (1/diag,
+// the coarsest level's inverse): through such a pointer the compiler may load
+// what the kernel ahead is still writing before the wait.
 #include "turb_internal.cuh"
 #include "turb_kernels.cuh"
 #include "turb_mg.cuh"
@@ -118,8 +123,7 @@ __device__ __forceinline__ void rb_cell(const LevelT<T> &L, int zero_init, const
 }
 
 template <typename T>
-__global__ void k_rbgs(MgDevLevel Ld, int color, int zero_init, const T *__restrict__ b, const T *__restrict__ invd,
-                       T *__restrict__ x)
+__global__ void k_rbgs(MgDevLevel Ld, int color, int zero_init, const T *b, const T *__restrict__ invd, T *x)
 {
     pdl_trigger();
     pdl_wait();
@@ -259,8 +263,8 @@ __global__ void __launch_bounds__(256, 4) k_resid_col(MgDevLevel Ld, int planes,
 // per cell is s_row's, operation for operation.
 constexpr int RB4_PLANES = 2;                    // planes per thread on the large levels
 constexpr long long RB4_PLANES_CELLS = 1ll << 22;   // levels of at least this many cells
-__global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, int planes, const float *__restrict__ b,
-                        const float *__restrict__ invd, float *__restrict__ x)
+__global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, int planes, const float *b,
+                        const float *__restrict__ invd, float *x)
 {
     pdl_trigger();
     pdl_wait();
@@ -396,8 +400,8 @@ __global__ void __launch_bounds__(256) k_rbgs4s(MgDevLevel Ld, int color, int ze
 // in registers, loaded one plane ahead.  Each cell's arithmetic is k_rbgs4's,
 // operation for operation, so the results are the same bits.
 constexpr int RTX = 4 * 32 + 2;
-__global__ void __launch_bounds__(256, 3) k_rbgs4z(MgDevLevel Ld, int color, int jz, const float *__restrict__ b,
-                                                   const float *__restrict__ invd, float *__restrict__ x)
+__global__ void __launch_bounds__(256, 3) k_rbgs4z(MgDevLevel Ld, int color, int jz, const float *b,
+                                                   const float *__restrict__ invd, float *x)
 {
     pdl_trigger();
     pdl_wait();
@@ -503,7 +507,7 @@ __device__ __forceinline__ void resid_cell(const LevelT<T> &L, const T *__restri
 }
 
 template <typename T>
-__global__ void k_resid(MgDevLevel Ld, const T *__restrict__ b, const T *__restrict__ x, T *__restrict__ r)
+__global__ void k_resid(MgDevLevel Ld, const T *b, const T *x, T *r)
 {
     pdl_trigger();
     pdl_wait();
@@ -518,8 +522,7 @@ __global__ void k_resid(MgDevLevel Ld, const T *__restrict__ b, const T *__restr
 // live at index m0+e of colour halves c0 = (j+k)&1 and c0^1, so every x and
 // b access is a float4 (two scalars for the row ends); r is written in the
 // natural order the restriction reads.  Per cell the arithmetic is s_row's.
-__global__ void __launch_bounds__(256, 4) k_resid8(MgDevLevel Ld, const float *__restrict__ b, const float *__restrict__ x,
-                                                   float *__restrict__ r)
+__global__ void __launch_bounds__(256, 4) k_resid8(MgDevLevel Ld, const float *b, const float *x, float *r)
 {
     pdl_trigger();
     pdl_wait();
@@ -659,7 +662,7 @@ __device__ __forceinline__ void prolong_cell(const MgDevLevel &Lf, const MgDevLe
 }
 
 template <typename T>
-__global__ void k_restrict(MgDevLevel Lf, MgDevLevel Lc, const T *__restrict__ rf, T *__restrict__ bc)
+__global__ void k_restrict(MgDevLevel Lf, MgDevLevel Lc, const T *rf, T *bc)
 {
     pdl_trigger();
     pdl_wait();
@@ -669,7 +672,7 @@ __global__ void k_restrict(MgDevLevel Lf, MgDevLevel Lc, const T *__restrict__ r
 }
 
 template <typename T>
-__global__ void k_prolong(MgDevLevel Lf, MgDevLevel Lc, const T *__restrict__ xc, T *__restrict__ xf)
+__global__ void k_prolong(MgDevLevel Lf, MgDevLevel Lc, const T *xc, T *xf)
 {
     pdl_trigger();
     pdl_wait();
@@ -713,7 +716,7 @@ __device__ __forceinline__ void st8(const MgDevLevel &L, float *a, int i0, int j
 // restriction where x is not coarsened (cx = 0: identity in x), eight cells
 // of a coarse row per thread; r is natural, b of the coarse level in its
 // storage order
-__global__ void k_restrict_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *__restrict__ rf, float *__restrict__ bc)
+__global__ void k_restrict_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *rf, float *bc)
 {
     pdl_trigger();
     pdl_wait();
@@ -747,7 +750,7 @@ __global__ void k_restrict_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *__rest
 }
 
 // prolongation where x is not coarsened, eight cells of a fine row per thread
-__global__ void k_prolong_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *__restrict__ xc, float *__restrict__ xf)
+__global__ void k_prolong_yz8(MgDevLevel Lf, MgDevLevel Lc, const float *xc, float *xf)
 {
     pdl_trigger();
     pdl_wait();
@@ -783,7 +786,7 @@ __device__ __forceinline__ void coarse_row(int n, const double *__restrict__ ain
 }
 
 template <typename T>
-__global__ void k_coarse(int n, const double *__restrict__ ainv, const T *__restrict__ b, T *__restrict__ x)
+__global__ void k_coarse(int n, const double *__restrict__ ainv, const T *b, T *x)
 {
     pdl_trigger();
     pdl_wait();
@@ -991,7 +994,7 @@ __global__ void k_to_float_lev(MgDevLevel L, const double *__restrict__ a, float
     long long c = ((long long)k * L.ny + j) * L.nx + i;
     b[lev_at(L, c, i, j, k)] = (float)a[c];
 }
-__global__ void k_to_double_lev(MgDevLevel L, const float *__restrict__ a, double *__restrict__ b)
+__global__ void k_to_double_lev(MgDevLevel L, const float *a, double *b)
 {
     pdl_trigger();
     pdl_wait();
@@ -1025,7 +1028,7 @@ __global__ void k_to_float_lev8(MgDevLevel L, const double *__restrict__ a, floa
         *reinterpret_cast<float4 *>(b + c0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
 }
-__global__ void k_to_double_lev8(MgDevLevel L, const float *__restrict__ a, double *__restrict__ b)
+__global__ void k_to_double_lev8(MgDevLevel L, const float *a, double *b)
 {
     pdl_trigger();
     pdl_wait();
