@@ -220,7 +220,8 @@ __global__ void k_add_corr(long long n, double *__restrict__ x, const float *__r
 // latency does: the KC planes' loads are all in flight before the first row is
 // formed (98 registers; on large grids fewer warps then cost more than the
 // latency: 975 us against 715 at 513x257x257).  The last block adds the
-// partial sums.
+// partial sums.  adt: 1/dt for the sweeps, whose captured graphs outlive a
+// time step of one length.
 struct ResidRow {
     double axy, aw, ae, as, an;
     float afx, afy;
@@ -255,7 +256,8 @@ __device__ __forceinline__ void resid_store(const HelmTab &h, const HelmTabF &hf
 template <int G>
 __global__ void __launch_bounds__(HBX *HBY, G ? 4 : 2) k_helm_resid64(Dims d, HelmTab h, HelmTabF hf, const uint8_t *__restrict__ st, double a_dt,
                                const double *__restrict__ b, const double *__restrict__ x,
-                               float *__restrict__ rf, float *__restrict__ e0, double *__restrict__ part, const SumTo to)
+                               float *__restrict__ rf, float *__restrict__ e0, float *__restrict__ adt, double *__restrict__ part,
+                               const SumTo to)
 {
     constexpr int NG = G ? G : 1;
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(HBX *HBY, G ? 4 : 2) k_helm_resid64(Dims d, He
     {
         int t = threadIdx.y * blockDim.x + threadIdx.x, k = k0 + t;
         if (t < KC * NG) zdt[t] = k < d.NZ ? h.apz[k] + a_dt : 0.0;
+        if (t == 0 && part_index() == 0) *adt = (float)a_dt;   // for the sweeps
     }
     __syncthreads();
     double r2[NG] = {};
@@ -364,13 +367,14 @@ __global__ void k_ib_resid64(IbDev ib, IbDevF ibf, const double *__restrict__ b,
 // four blocks of 32 x 8 per SM (64 registers): measured 17 % faster at
 // 513x257x257 than the three that 76 registers allow
 template <bool LAST>
-__global__ void __launch_bounds__(HBX *HBY, 4) k_helm_jac32v(Dims d, HelmTabF h, const uint8_t *__restrict__ st, float a_dt,
+__global__ void __launch_bounds__(HBX *HBY, 4) k_helm_jac32v(Dims d, HelmTabF h, const uint8_t *__restrict__ st, const float *adt,
                               const float *__restrict__ r, const float *e, float *en, double *x)
 {
     const int i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), j = blockIdx.y * blockDim.y + threadIdx.y;
     pdl_wait();
     pdl_trigger();   // the immersed rows' kernel, which reads e too, may start
     if (i0 >= d.NX || j >= d.NY) return;
+    const float a_dt = *adt;
     const float4 apx = *reinterpret_cast<const float4 *>(h.apx + i0);
     const float4 aw = *reinterpret_cast<const float4 *>(h.aw + i0);
     const float4 ae = *reinterpret_cast<const float4 *>(h.ae + i0);
@@ -451,10 +455,11 @@ __global__ void __launch_bounds__(HBX *HBY, 4) k_helm_jac32v(Dims d, HelmTabF h,
 constexpr int JZ = 16;                 // planes per block
 constexpr int JTX = 4 * HBX + 2;       // tile row: 128 points and two halo columns
 __global__ void __launch_bounds__(HBX *HBY, 3) k_helm_jac32z(Dims d, HelmTabF h, const uint8_t *__restrict__ st,
-                                                          float a_dt, const float *__restrict__ r,
+                                                          const float *__restrict__ adt, const float *__restrict__ r,
                                                           const float *__restrict__ e, float *__restrict__ en)
 {
     __shared__ float tile[HBY + 2][JTX];
+    const float a_dt = *adt;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int i0 = 4 * (blockIdx.x * HBX + tx), j = blockIdx.y * HBY + ty;
     const int k0 = blockIdx.z * JZ, k1 = min(k0 + JZ, d.NZ);
@@ -658,10 +663,10 @@ static void launch_pdl(void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... arg
     cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-// |r|^2 goes to *dst, the first sweep's result to e0
+// |r|^2 goes to *dst, the first sweep's result to e0, 1/dt for the others to *adt
 void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
-                         const double *b, const double *x, float *rf, float *e0, const IbDev &ib, const IbDevF &ibf,
-                         double *part, unsigned *count, double *dst)
+                         const double *b, const double *x, float *rf, float *e0, float *adt, const IbDev &ib,
+                         const IbDevF &ibf, double *part, unsigned *count, double *dst)
 {
     const long long hp = helm_parts(d);
     const unsigned nib = (unsigned)((ib.n + 255) / 256);
@@ -671,7 +676,7 @@ void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const 
     if (g) gr.z = (gr.z + g - 1) / g;
     const SumTo to{(int)(hp + nib), gr.x * gr.y * gr.z + nib, count, dst};
     const auto k = g == 4 ? k_helm_resid64<4> : g == 2 ? k_helm_resid64<2> : g == 1 ? k_helm_resid64<1> : k_helm_resid64<0>;
-    k<<<gr, dim3(HBX, HBY), 0, s>>>(d, h, hf, st, a_dt, b, x, rf, e0, part, to);
+    k<<<gr, dim3(HBX, HBY), 0, s>>>(d, h, hf, st, a_dt, b, x, rf, e0, adt, part, to);
     if (ib.n > 0) launch_pdl(k_ib_resid64, dim3(nib), dim3(256), s, ib, ibf, b, x, rf, e0, part, hp, to);
 }
 
@@ -679,7 +684,7 @@ void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const 
 // alone: the kernel ahead of it on the stream is not a sweep.  marching 1: the
 // sweeps but the last march along k through shared-memory plane tiles
 // (k_helm_jac32z); 0: k_helm_jac32v throughout
-void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, float a_dt,
+void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, const float *adt,
                        const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching)
 {
     dim3 g((unsigned)((d.NX + 4 * HBX - 1) / (4 * HBX)), (unsigned)((d.NY + HBY - 1) / HBY),
@@ -687,14 +692,14 @@ void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const u
     if (!x && marching) {
         dim3 gz((unsigned)((d.NX + 4 * HBX - 1) / (4 * HBX)), (unsigned)((d.NY + HBY - 1) / HBY),
                 (unsigned)((d.NZ + JZ - 1) / JZ));
-        k_helm_jac32z<<<gz, dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, r, e, en);
+        k_helm_jac32z<<<gz, dim3(HBX, HBY), 0, s>>>(d, h, st, adt, r, e, en);
         // k_helm_jac32z writes placeholders at immersed points: the immersed
         // rows go after it in plain stream order
         if (ib.n > 0) k_ib_jac32<<<(ib.n + 255) / 256, 256, 0, s>>>(ib, r, e, en, x);
         return;
     }
     const auto k = x ? k_helm_jac32v<true> : k_helm_jac32v<false>;
-    if (alone || marching) k<<<g, dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, r, e, en, x);
-    else launch_pdl(k, g, dim3(HBX, HBY), s, d, h, st, a_dt, r, e, en, x);
+    if (alone || marching) k<<<g, dim3(HBX, HBY), 0, s>>>(d, h, st, adt, r, e, en, x);
+    else launch_pdl(k, g, dim3(HBX, HBY), s, d, h, st, adt, r, e, en, x);
     if (ib.n > 0) launch_pdl(k_ib_jac32, dim3((ib.n + 255) / 256), dim3(256), s, ib, r, e, en, x);
 }

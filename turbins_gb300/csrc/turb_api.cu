@@ -127,6 +127,7 @@ struct turb_ctx {
     HelmTabF helmf[3], helmf_c[TURB_MAXCONC];
     IbDevF ibf[4];
     float *hrf = nullptr, *he0 = nullptr, *he1 = nullptr;   // defect-correction buffers
+    float *hadt = nullptr;                                  // 1/dt of the correction in flight
     int hmode = TURB_HMODE_MIXED;
     // the 1/dt term of each Helmholtz diagonal (u, v, w, c_0..) and the dt it
     // was last updated for (0: not yet)
@@ -1165,6 +1166,7 @@ int turb_create(const turb_grid_desc *g, const turb_params *p, turb_ctx **out)
     c->hrf = m.alloc<float>(d.n);
     c->he0 = m.alloc<float>(d.n);
     c->he1 = m.alloc<float>(d.n);
+    c->hadt = m.alloc<float>(1);
     {
         double a_dEta = 1.0 / c->dEta, a_dXi = 1.0 / c->dXi, a_dPhi = 1.0 / c->dPhi;
         std::vector<double> cx(d.NX), cy(d.NY), cz(d.NZ), cyv(d.NY), czw(d.NZ);
@@ -2432,8 +2434,8 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
     c->launches += 1;
     for (;;) {
         int ph = prof_begin(c, TURB_PROF_JACOBI);
-        launch_helm_resid64(c->s, d, h, hf, c->st[q], a_dt, b, x, c->hrf, c->he0, ib, ibf, c->part, c->count,
-                            c->hscal + HS_R);
+        launch_helm_resid64(c->s, d, h, hf, c->st[q], a_dt, b, x, c->hrf, c->he0, c->hadt, ib, ibf, c->part,
+                            c->count, c->hscal + HS_R);
         prof_end(c, ph, 1, HELM_RESID64_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
         c->launches += 1 + (ib.n > 0);
         TURB_CHECK(cudaStreamSynchronize(c->s));
@@ -2446,7 +2448,7 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
         auto sweeps = [&]() {
             float *ea = c->he0, *eb = c->he1;
             for (int t = 1; t < c->hinner; t++) {
-                launch_helm_jac32(c->s, d, hf, c->st[q], (float)a_dt, c->hrf, ea, eb, t == c->hinner - 1 ? x : nullptr, ibf,
+                launch_helm_jac32(c->s, d, hf, c->st[q], c->hadt, c->hrf, ea, eb, t == c->hinner - 1 ? x : nullptr, ibf,
                                   t == 1, c->kvariant & TURB_KV_MARCHING);
                 std::swap(ea, eb);
             }
@@ -2455,7 +2457,9 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
             launch_add_corr(c->s, d.n, x, c->he0);
             c->launches += 1;
         } else if (c->use_graphs) {
-            // a graph holds the number of sweeps and the address of x (an FP64 solve swaps it)
+            // a graph holds the number of sweeps and the address of x (an FP64
+            // solve swaps it); 1/dt, which changes with every step of a
+            // run that sets its own dt, it reads where the residual puts it
             if (c->g_inner[gi] && (c->g_inner_n[gi] != c->hinner || c->g_inner_x[gi] != x)) {
                 cudaGraphExecDestroy(c->g_inner[gi]);
                 c->g_inner[gi] = nullptr;
