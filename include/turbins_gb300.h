@@ -230,6 +230,14 @@ int turb_set_mg_coarse_sweeps(turb_ctx *ctx, int from_level, int npre, int npost
  * shared memory where they fit, else a single block (by default only from
  * 4096 cells on); results are bit-identical */
 int turb_set_mg_tail(turb_ctx *ctx, long long max_cells);
+/* forms of the V-cycle's kernels that the rules may choose, so that each can
+ * be compared with the others (the results are the same bits): low_blocks, the
+ * most blocks of the shared-memory cluster (16, the default; 8 is the form
+ * for a device that cannot hold 16, 1 a single block; 0: not used, the
+ * single-block launch over global memory takes its place); fp64_columns, 1
+ * (default): the FP64 half sweeps and residuals of the large levels march
+ * along k with kept coefficients, 0: a thread per cell */
+int turb_set_mg_forms(turb_ctx *ctx, int low_blocks, int fp64_columns);
 /* with TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level of at most
  * max_cells cells (default 131072; 0: never) runs as one thread-block
  * cluster launch, the levels from the single-block tail's on in block 0 of

@@ -319,8 +319,12 @@ class Context:
         _check(self.lib.turb_set_mg_sweeps(self.ctx, npre, npost), "set_mg_sweeps")
 
     def set_mg_tail(self, max_cells):
-        """turb_set_mg_tail: single-block V-cycle below max_cells cells (0: off)"""
+        """turb_set_mg_tail: the V-cycle in one launch below max_cells cells (0: off)"""
         _check(self.lib.turb_set_mg_tail(self.ctx, C.c_longlong(int(max_cells))), "set_mg_tail")
+
+    def set_mg_forms(self, low_blocks=16, fp64_columns=True):
+        """turb_set_mg_forms: which forms of the V-cycle's kernels may be chosen"""
+        _check(self.lib.turb_set_mg_forms(self.ctx, int(low_blocks), int(bool(fp64_columns))), "set_mg_forms")
 
     def set_mg_cluster(self, max_cells):
         """turb_set_mg_cluster: one-cluster V-cycle below max_cells cells (0: off), with KV_CLUSTER_VCYCLE"""

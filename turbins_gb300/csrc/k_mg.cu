@@ -1100,10 +1100,11 @@ void mg_setup_invdiag(cudaStream_t s, const MgDevLevel &L, T *invd)
 // one red-black half sweep of level L: the vectorised kernel where the
 // level is colour-split FP32 with nx a multiple of 8
 // marching: half sweeps after the first of a cycle march along k (k_rbgs4z)
-// on the levels large enough to fill the GPU with them
+// on the levels large enough to fill the GPU with them; columns: the same for
+// the FP64 levels (k_rbgs_col)
 template <typename T>
 void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, const T *b, const T *invd, T *x,
-             int marching, int pdl)
+             int marching, int columns, int pdl)
 {
     if constexpr (sizeof(T) == 4) {
         if (L.split && L.nx % 8 == 0) {
@@ -1141,7 +1142,7 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
     if constexpr (sizeof(T) == 8) {
         dim3 g = g3(L.nx >> 1, L.ny, L.nz);
         const int planes = col_planes(g);
-        if (!zero_init && L.nx % 2 == 0 && planes) {
+        if (columns && !zero_init && L.nx % 2 == 0 && planes) {
             g.z = (g.z + planes - 1) / planes;
             launch_k(pdl, k_rbgs_col<T>, g, B38, s, L, color, planes, b, invd, x);
             return;
@@ -1151,7 +1152,7 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
 }
 
 template <typename T>
-void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r, int pdl)
+void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r, int columns, int pdl)
 {
     if constexpr (sizeof(T) == 4) {
         if (L.split && L.nx % 8 == 0) {
@@ -1162,7 +1163,7 @@ void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r
     }
     if constexpr (sizeof(T) == 8) {
         const int planes = col_planes(g3(L.nx, L.ny, L.nz));
-        if (planes) {
+        if (columns && planes) {
             dim3 g = g3(L.nx, L.ny, L.nz);
             g.z = (g.z + planes - 1) / planes;
             launch_k(pdl, k_resid_col<T>, g, B38, s, L, planes, b, x, r);
@@ -1245,10 +1246,10 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
     for (int it = pre_done; it < npre; it++) {
         // the first colour-0 half sweep takes x = 0 (it reads no neighbours);
         // every colour-1 point is then rewritten from colour-0 values only
-        rb_half<T>(s, L, 0, it == 0, H.b[l], H.invd[l], H.x[l], H.marching, H.pdl);
-        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.pdl);
+        rb_half<T>(s, L, 0, it == 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
+        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
     }
-    resid_lev<T>(s, L, H.b[l], H.x[l], H.r[l], H.pdl);
+    resid_lev<T>(s, L, H.b[l], H.x[l], H.r[l], H.columns, H.pdl);
     const MgDevLevel &C = H.lev[l + 1];
     bool yz8 = false;
     if constexpr (sizeof(T) == 4) yz8 = L.cx == 0 && L.nx % 8 == 0 && C.nx == L.nx;
@@ -1267,8 +1268,8 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
         for (int f = 0; f < post_done / 2; f++) mg_tb_sweeps(s, *H.tb, f & 1, 1, 0, H.pdl);
     }
     for (int it = post_done; it < npost; it++) {
-        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.pdl);
-        rb_half<T>(s, L, 0, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.pdl);
+        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
+        rb_half<T>(s, L, 0, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
     }
 }
 

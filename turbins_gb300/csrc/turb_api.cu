@@ -180,6 +180,7 @@ struct turb_ctx {
     // shared-memory plane tiles, ENO y / z lines walked in segments
     int kvariant = TURB_KV_ENO_SEGMENTS | TURB_KV_PDL;
     long long mg_tail_cells = -1;   // turb_set_mg_tail (-1: the default rule of place_tail)
+    int low_held[2] = {0, 0};       // blocks of k_vcycle_low's cluster that the device holds, FP64 and FP32
     long long mg_cluster_cells = 1 << 17;   // TURB_KV_CLUSTER_VCYCLE from the first level of at most this many cells
     // TURB_KV_SWEEP_PAIRS: the finest FP32 level's two-sweeps-per-pass smoother
     RbTbPlan tbplan;
@@ -928,8 +929,8 @@ int build_mg(turb_ctx *c)
     c->count = c->mem.alloc<unsigned>(4);
     c->H64.cluster_ctas = mg_cluster_ctas<double>();
     c->H32.cluster_ctas = mg_cluster_ctas<float>();
-    c->H64.low_ctas = mg_low_ctas<double>();
-    c->H32.low_ctas = mg_low_ctas<float>();
+    c->low_held[0] = c->H64.low_ctas = mg_low_ctas<double>();
+    c->low_held[1] = c->H32.low_ctas = mg_low_ctas<float>();
     set_cluster_from(c);
     place_tail(c);
     set_tb(c);
@@ -1769,6 +1770,19 @@ int turb_set_mg_cluster(turb_ctx *c, long long max_cells)
     place_tail(c);
     for (int m = 0; m < 2; m++)
         if (c->g_mg[m]) { cudaGraphExecDestroy(c->g_mg[m]); c->g_mg[m] = nullptr; }
+    return TURB_OK;
+}
+
+int turb_set_mg_forms(turb_ctx *c, int low_blocks, int fp64_columns)
+{
+    if (!c || (low_blocks != 0 && low_blocks != 1 && low_blocks != 8 && low_blocks != 16) || fp64_columns < 0 || fp64_columns > 1)
+        return TURB_ERR_ARG;
+    c->H64.low_ctas = std::min(c->low_held[0], low_blocks);
+    c->H32.low_ctas = std::min(c->low_held[1], low_blocks);
+    c->H64.columns = fp64_columns;
+    place_tail(c);
+    for (auto &g : c->g_mg)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     return TURB_OK;
 }
 

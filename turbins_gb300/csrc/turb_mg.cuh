@@ -86,6 +86,9 @@ struct MgHier {
     int low_ctas = 0;   // blocks of k_vcycle_low's cluster (mg_low_ctas; 0: not used)
     // 1: FP32 half sweeps after the first of a cycle march along k (k_rbgs4z)
     int marching = 0;
+    // 1: FP64 half sweeps and residuals of large levels march along k
+    // (k_rbgs_col, k_resid_col); 0: k_rbgs, k_resid throughout
+    int columns = 1;
     // 1: the V-cycle's kernels use programmatic dependent launch
     int pdl = 1;
     // from this level on (-1: never) the V-cycle runs as one launch of one
