@@ -175,9 +175,10 @@ int turb_reset_pressure_history(turb_ctx *ctx);
  * through shared-memory plane tiles (else one point, four cells, per thread);
  * TURB_KV_ENO_SEGMENTS, every y / z ENO line is walked in segments of about
  * 64 nodes by separate threads (else one thread per line); TURB_KV_PDL,
- * the V-cycle's kernels are launched with programmatic dependent launch, so
- * that each may be scheduled while the one before it drains (else plain
- * stream order); TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level
+ * the kernels of the V-cycle, the conjugate-gradient step, the Helmholtz
+ * solves and the network that the context runs are launched with
+ * programmatic dependent launch, so that each may be scheduled while the one
+ * before it drains (else plain stream order); TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level
  * of at most turb_set_mg_cluster cells down runs as one launch of one
  * thread-block cluster (16 blocks of 1024 threads, or 8 where 16 do not fit),
  * its phases separated by the hardware cluster barrier; TURB_KV_SWEEP_PAIRS,
@@ -190,7 +191,7 @@ int turb_reset_pressure_history(turb_ctx *ctx);
  * 512x256x256). */
 #define TURB_KV_MARCHING 1
 #define TURB_KV_ENO_SEGMENTS 2
-#define TURB_KV_PDL 4   /* V-cycle kernels with programmatic dependent launch */
+#define TURB_KV_PDL 4   /* the solvers' kernels with programmatic dependent launch */
 #define TURB_KV_CLUSTER_VCYCLE 8   /* coarse V-cycle levels in one thread-block cluster */
 #define TURB_KV_SWEEP_PAIRS 16    /* finest FP32 level: two sweeps per pass */
 int turb_set_sweep_kernels(turb_ctx *ctx, int variants);

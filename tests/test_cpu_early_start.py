@@ -82,3 +82,17 @@ def test_no_restrict_on_what_the_kernel_ahead_writes(name):
     early = [k for k in kernels(os.path.join(CSRC, name)) if "pdl_wait" in k[2]]
     assert early
     assert {k[0]: unsettled(k[0], k[1]) for k in early if unsettled(k[0], k[1])} == {}
+
+
+def test_every_early_launch_follows_the_switch():
+    """TURB_KV_PDL off means plain stream order for every kernel (a race is
+    looked for that way): the launch attribute is set in one helper and the two
+    cluster launches, each under a flag, and every call hands a flag on."""
+    src = {f: open(os.path.join(CSRC, f)).read() for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))}
+    where = {f: s.count("cudaLaunchAttributeProgrammaticStreamSerialization") for f, s in src.items()}
+    assert {f: n for f, n in where.items() if n} == {"turb_internal.cuh": 1, "k_mg.cu": 1, "k_mglow.cu": 1}
+    assert "cfg.numAttrs = early ? 1 : 0;" in src["turb_internal.cuh"]
+    assert "cfg.numAttrs = H.pdl ? 2 : 1;" in src["k_mg.cu"]
+    assert re.search(r"if \(pdl\) \{\s*at\[n\]\.id = cudaLaunchAttributeProgrammaticStreamSerialization", src["k_mglow.cu"])
+    flags = [m.group(1) for s in src.values() for m in re.finditer(r"\b(?:launch_early|launch_k|net_launch|launch_pairs)\(([^,]+),", s)]
+    assert set(flags) <= {"pdl", "early", "H.pdl", "n->pdl", "int early", "int pdl"} and len(flags) > 40

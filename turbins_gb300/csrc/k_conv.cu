@@ -1179,7 +1179,7 @@ void conv_pack_weights(cudaStream_t s, const float *W, int cin, int cout, const 
 namespace {
 
 template <int CIN, int COUT, int ZRING>
-int launch_rows(cudaStream_t s, RowArgs r, int nsm)
+int launch_rows(cudaStream_t s, RowArgs r, int nsm, int pdl)
 {
     constexpr uint32_t smem = rows_smem(CIN, COUT);
     static int lim = dyn_smem_limit((const void *)k_conv_rows<CIN, COUT, ZRING>);
@@ -1191,21 +1191,21 @@ int launch_rows(cudaStream_t s, RowArgs r, int nsm)
     r.rch = 32;
     while ((r.rch > 4 && lines / r.rch < 2LL * most) || (r.rch > 1 && lines / r.rch < most)) r.rch >>= 1;
     r.nitems = r.ntx * ((r.R + r.rch - 1) / r.rch);
-    net_launch(k_conv_rows<CIN, COUT, ZRING>, most < r.nitems ? most : r.nitems, 1, 288, smem, s, r);
+    net_launch(pdl, k_conv_rows<CIN, COUT, ZRING>, most < r.nitems ? most : r.nitems, 1, 288, smem, s, r);
     return launch_error("k_conv_rows");
 }
 
 template <int ZRING>
-int launch_rows(cudaStream_t s, const RowArgs &r, int cin, int cout, int nsm)
+int launch_rows(cudaStream_t s, const RowArgs &r, int cin, int cout, int nsm, int pdl)
 {
-    if (cin == 16) return cout == 16 ? launch_rows<16, 16, ZRING>(s, r, nsm) : launch_rows<16, 32, ZRING>(s, r, nsm);
-    return cout == 16 ? launch_rows<32, 16, ZRING>(s, r, nsm) : launch_rows<32, 32, ZRING>(s, r, nsm);
+    if (cin == 16) return cout == 16 ? launch_rows<16, 16, ZRING>(s, r, nsm, pdl) : launch_rows<16, 32, ZRING>(s, r, nsm, pdl);
+    return cout == 16 ? launch_rows<32, 16, ZRING>(s, r, nsm, pdl) : launch_rows<32, 32, ZRING>(s, r, nsm, pdl);
 }
 
 }  // namespace
 
 int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int cout, const bf16 *wpk,
-              const ConvEpi &e, int *err, int nsm)
+              const ConvEpi &e, int *err, int nsm, int pdl)
 {
     if (cin % 16 || cout % 16 || cout > 128 || cin > 128) { snprintf(g_conv_err, sizeof(g_conv_err), "conv channels"); return 1; }
     const ConvPlan p = conv_plan(X, Y, Z, cin, cout);
@@ -1218,7 +1218,7 @@ int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int 
         r.Q = p.zring ? Y : Z; r.qs = p.zring ? X : X * Y;
         r.ntx = (int)(((long long)r.Q * r.W + 127) / 128);
         r.in = in; r.wpk = wpk; r.epi = epi; r.err = err;
-        return p.zring ? launch_rows<1>(s, r, cin, cout, nsm) : launch_rows<0>(s, r, cin, cout, nsm);
+        return p.zring ? launch_rows<1>(s, r, cin, cout, nsm, pdl) : launch_rows<0>(s, r, cin, cout, nsm, pdl);
     }
     WideArgs a{};
     a.X = X; a.Y = Y; a.Z = Z; a.W = X + 2;
@@ -1235,14 +1235,14 @@ int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int 
     if (a.stages > WSTAGES) a.stages = WSTAGES;
     if (a.stages <= WLAG) { snprintf(g_conv_err, sizeof(g_conv_err), "conv needs %u B of shared memory a stage", a.stride); return 1; }
     const int nwork = a.ntiles * a.nsplit;
-    net_launch(k_conv_wide, nsm < nwork ? nsm : nwork, 1, 288, (uint32_t)a.stages * a.stride + 1024u, s, a);
+    net_launch(pdl, k_conv_wide, nsm < nwork ? nsm : nwork, 1, 288, (uint32_t)a.stages * a.stride + 1024u, s, a);
     return launch_error("k_conv_wide");
 }
 
 namespace {
 
 template <int CIN, int COUT>
-int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm)
+int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm, int pdl)
 {
     constexpr uint32_t smem = WRS * wgr_stage(CIN, COUT) + 1024u;
     static int lim = dyn_smem_limit((const void *)k_wgrad_rows<CIN, COUT>);
@@ -1250,14 +1250,14 @@ int launch_wgrad_rows(cudaStream_t s, WgRowArgs r, int nsm)
     r.nsteps = r.ntx * ((r.R + WgR<CIN>::RA - 1) / WgR<CIN>::RA);
     r.ndx = r.nsteps > 20 * nsm ? 1 : 3;
     const int ng = 3 / r.ndx, per = nsm / ng < r.nsteps ? nsm / ng : r.nsteps;
-    net_launch(k_wgrad_rows<CIN, COUT>, ng * (per > 0 ? per : 1), 1, 288, smem, s, r);
+    net_launch(pdl, k_wgrad_rows<CIN, COUT>, ng * (per > 0 ? per : 1), 1, 288, smem, s, r);
     return launch_error("k_wgrad_rows");
 }
 
 }  // namespace
 
 int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int Z, int cin, int cout, float *dw,
-                int *err, int nsm)
+                int *err, int nsm, int pdl)
 {
     if (cin % 16 || cout % 16 || cout > 128 || cin > 128) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad channels"); return 1; }
     WgArgs a{};
@@ -1274,8 +1274,8 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
         r.cstep = X * Y * Z;
         r.ntx = (int)(((long long)r.Q * r.W + 127) / 128);
         r.x = x; r.dy = dy; r.dw = dw; r.err = err;
-        if (cin == 16) return cout == 16 ? launch_wgrad_rows<16, 16>(s, r, nsm) : launch_wgrad_rows<16, 32>(s, r, nsm);
-        return cout == 16 ? launch_wgrad_rows<32, 16>(s, r, nsm) : launch_wgrad_rows<32, 32>(s, r, nsm);
+        if (cin == 16) return cout == 16 ? launch_wgrad_rows<16, 16>(s, r, nsm, pdl) : launch_wgrad_rows<16, 32>(s, r, nsm, pdl);
+        return cout == 16 ? launch_wgrad_rows<32, 16>(s, r, nsm, pdl) : launch_wgrad_rows<32, 32>(s, r, nsm, pdl);
     }
     a.X = X; a.Y = Y; a.Z = Z; a.cin = cin; a.cout = cout;
     a.G = 128 / cin; a.ngroups = (27 + a.G - 1) / a.G;
@@ -1297,7 +1297,7 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
     a.nsplit = want < 1 ? 1 : want;
     if (a.nsplit > a.ntiles) a.nsplit = a.ntiles;
     a.dw = dw; a.err = err;
-    net_launch(k_wgrad, a.ngroups * a.nsplit, 1, 192, smem, s, mx, md, a);
+    net_launch(pdl, k_wgrad, a.ngroups * a.nsplit, 1, 192, smem, s, mx, md, a);
     return launch_error("k_wgrad");
 }
 

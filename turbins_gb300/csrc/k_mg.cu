@@ -1053,27 +1053,12 @@ __global__ void k_to_double_lev8(MgDevLevel L, const float *a, double *b)
 
 inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
-// a V-cycle kernel launch; pdl: with the programmatic stream serialisation
-// attribute (the kernels start with pdl_trigger / pdl_wait), so that a small
-// level's launches overlap the drain of the kernel before them
-template <typename... P, typename... A>
-void launch_k(int pdl, void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... args)
+// a V-cycle kernel launch (the kernels start with pdl_trigger / pdl_wait, so that
+// with pdl a small level's launches overlap the drain of the kernel before them)
+template <typename K, typename... A>
+void launch_k(int pdl, K k, dim3 g, dim3 b, cudaStream_t s, A... args)
 {
-    if (!pdl) {
-        k<<<g, b, 0, s>>>(args...);
-        return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, args...);
+    launch_early(pdl, k, g, b, 0u, s, args...);
 }
 inline dim3 g3(int nx, int ny, int nz) { return dim3((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz); }
 const dim3 B38(32, 8, 1);

@@ -406,6 +406,7 @@ struct Rng {
 
 struct TurbNet {
     int nx, ny, nz, train, nsm;
+    int pdl = 1;   // its kernels use programmatic dependent launch
     int X[4], Y[4], Z[4];
     long long V[4];
     long long nparam = 0, woff[NL], boff[NL], hw_off, hb_off;
@@ -458,7 +459,7 @@ int conv(TurbNet *n, cudaStream_t s, int l, const bf16 *in, const ConvEpi &e)
 {
     const LayerDef &d = DEFS[l];
     int lv = d.lev;
-    int rc = conv3_fwd(s, in, n->X[lv], n->Y[lv], n->Z[lv], d.cin, d.cout, n->wf[l], e, n->err, n->nsm);
+    int rc = conv3_fwd(s, in, n->X[lv], n->Y[lv], n->Z[lv], d.cin, d.cout, n->wf[l], e, n->err, n->nsm, n->pdl);
     return rc ? turb_set_error_text(conv_last_error()) : TURB_OK;
 }
 // data gradient of layer l: dy (cout ch) -> dx (cin ch), masked by `mask`
@@ -469,30 +470,30 @@ int dgrad(TurbNet *n, cudaStream_t s, int l, const bf16 *dy, const bf16 *mask, b
     ConvEpi e;
     e.mask = mask;
     e.out = dx;
-    int rc = conv3_fwd(s, dy, n->X[lv], n->Y[lv], n->Z[lv], d.cout, d.cin, n->wd[l], e, n->err, n->nsm);
+    int rc = conv3_fwd(s, dy, n->X[lv], n->Y[lv], n->Z[lv], d.cout, d.cin, n->wd[l], e, n->err, n->nsm, n->pdl);
     return rc ? turb_set_error_text(conv_last_error()) : TURB_OK;
 }
 int wgrad(TurbNet *n, cudaStream_t s, int l, const bf16 *x, const bf16 *dy)
 {
     const LayerDef &d = DEFS[l];
     int lv = d.lev;
-    int rc = conv3_wgrad(s, x, dy, n->X[lv], n->Y[lv], n->Z[lv], d.cin, d.cout, n->G + n->woff[l], n->err, n->nsm);
+    int rc = conv3_wgrad(s, x, dy, n->X[lv], n->Y[lv], n->Z[lv], d.cin, d.cout, n->G + n->woff[l], n->err, n->nsm, n->pdl);
     if (rc) return turb_set_error_text(conv_last_error());
     // four voxels per thread, about two blocks per SM over all channel blocks
     const int want = nblk((n->V[lv] + 3) / 4), most = 2 * n->nsm * 8 / d.cout;
-    net_launch(k_chan_sum, want < most ? want : most > 1 ? most : 1, d.cout / 8, 256, 0, s, n->V[lv], dy, n->G + n->boff[l]);
+    net_launch(n->pdl, k_chan_sum, want < most ? want : most > 1 ? most : 1, d.cout / 8, 256, 0, s, n->V[lv], dy, n->G + n->boff[l]);
     return TURB_OK;
 }
 G3 g3(const TurbNet *n, int l) { return G3{n->X[l], n->Y[l], n->Z[l]}; }
 
 // a kernel over the voxel pairs (pair_of) of ncb channel blocks of f
 template <typename K, typename... A>
-void launch_pairs(K k, const G3 &f, int ncb, cudaStream_t s, A... args)
+void launch_pairs(int pdl, K k, const G3 &f, int ncb, cudaStream_t s, A... args)
 {
     unsigned bx = 128;
     while (bx > 8 && (int)bx >= f.X) bx >>= 1;
     const unsigned by = 256 / bx;
-    net_launch(k, dim3((unsigned)(f.Z * ncb), ((unsigned)f.Y + by - 1) / by, ((unsigned)f.X / 2 + bx - 1) / bx), dim3(bx, by), 0u, s, f,
+    launch_early(pdl, k, dim3((unsigned)(f.Z * ncb), ((unsigned)f.Y + by - 1) / by, ((unsigned)f.X / 2 + bx - 1) / bx), dim3(bx, by), 0u, s, f,
                args...);
 }
 
@@ -521,13 +522,13 @@ int forward(TurbNet *n, cudaStream_t s, const float *in3, float *hout)
     e.relu = 1;
     e.bias = P + n->boff[0]; e.out = n->a0;
     NCHK(conv(n, s, 0, n->x0, e));
-    net_launch(k_pool, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->a0, n->p0);
+    net_launch(n->pdl, k_pool, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->a0, n->p0);
     e.bias = P + n->boff[1]; e.out = n->a1;
     NCHK(conv(n, s, 1, n->p0, e));
-    net_launch(k_pool, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->a1, n->p1);
+    net_launch(n->pdl, k_pool, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->a1, n->p1);
     e.bias = P + n->boff[2]; e.out = n->a2;
     NCHK(conv(n, s, 2, n->p1, e));
-    net_launch(k_pool, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->a2, n->p2);
+    net_launch(n->pdl, k_pool, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->a2, n->p2);
     e.bias = P + n->boff[3]; e.out = n->a3;
     NCHK(conv(n, s, 3, n->p2, e));
     e.bias = P + n->boff[4]; e.out = n->b3;
@@ -535,17 +536,17 @@ int forward(TurbNet *n, cudaStream_t s, const float *in3, float *hout)
     ConvEpi u;
     u.bias = P + n->boff[5]; u.out = n->c2;
     NCHK(conv(n, s, 5, n->b3, u));
-    launch_pairs(k_up_add_relu, g3(n, 2), 8, s, n->c2, n->a2, n->s2);
+    launch_pairs(n->pdl, k_up_add_relu, g3(n, 2), 8, s, n->c2, n->a2, n->s2);
     e.bias = P + n->boff[6]; e.out = n->b2;
     NCHK(conv(n, s, 6, n->s2, e));
     u.bias = P + n->boff[7]; u.out = n->c1;
     NCHK(conv(n, s, 7, n->b2, u));
-    launch_pairs(k_up_add_relu, g3(n, 1), 4, s, n->c1, n->a1, n->s1);
+    launch_pairs(n->pdl, k_up_add_relu, g3(n, 1), 4, s, n->c1, n->a1, n->s1);
     e.bias = P + n->boff[8]; e.out = n->b1;
     NCHK(conv(n, s, 8, n->s1, e));
     u.bias = P + n->boff[9]; u.out = n->c0;
     NCHK(conv(n, s, 9, n->b1, u));
-    launch_pairs(k_up_add_relu, g3(n, 0), 2, s, n->c0, n->a0, n->s0);
+    launch_pairs(n->pdl, k_up_add_relu, g3(n, 0), 2, s, n->c0, n->a0, n->s0);
     ConvEpi h;
     h.relu = 1;
     h.bias = P + n->boff[10];
@@ -564,30 +565,30 @@ int backward(TurbNet *n, cudaStream_t s, const float *gout)
                                                                            n->dz0b, n->G + n->hw_off, n->G + n->hb_off);
     NCHK(wgrad(n, s, 10, n->s0, n->dz0b));
     NCHK(dgrad(n, s, 10, n->dz0b, n->s0, n->dzs0));
-    net_launch(k_down_sum, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->dzs0, n->dc0);
+    net_launch(n->pdl, k_down_sum, nblk(n->V[1] * 2), 1, 256, 0, s, g3(n, 1), 2, n->dzs0, n->dc0);
     NCHK(wgrad(n, s, 9, n->b1, n->dc0));
     NCHK(dgrad(n, s, 9, n->dc0, n->b1, n->dz1b));
     NCHK(wgrad(n, s, 8, n->s1, n->dz1b));
     NCHK(dgrad(n, s, 8, n->dz1b, n->s1, n->dzs1));
-    net_launch(k_down_sum, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->dzs1, n->dc1);
+    net_launch(n->pdl, k_down_sum, nblk(n->V[2] * 4), 1, 256, 0, s, g3(n, 2), 4, n->dzs1, n->dc1);
     NCHK(wgrad(n, s, 7, n->b2, n->dc1));
     NCHK(dgrad(n, s, 7, n->dc1, n->b2, n->dz2b));
     NCHK(wgrad(n, s, 6, n->s2, n->dz2b));
     NCHK(dgrad(n, s, 6, n->dz2b, n->s2, n->dzs2));
-    net_launch(k_down_sum, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->dzs2, n->dc2);
+    net_launch(n->pdl, k_down_sum, nblk(n->V[3] * 8), 1, 256, 0, s, g3(n, 3), 8, n->dzs2, n->dc2);
     NCHK(wgrad(n, s, 5, n->b3, n->dc2));
     NCHK(dgrad(n, s, 5, n->dc2, n->b3, n->dz3b));
     NCHK(wgrad(n, s, 4, n->a3, n->dz3b));
     NCHK(dgrad(n, s, 4, n->dz3b, n->a3, n->dz3));
     NCHK(wgrad(n, s, 3, n->p2, n->dz3));
     NCHK(dgrad(n, s, 3, n->dz3, nullptr, n->dp2));
-    launch_pairs(k_combine, g3(n, 2), 8, s, n->dzs2, n->dp2, n->a2, n->dz2);
+    launch_pairs(n->pdl, k_combine, g3(n, 2), 8, s, n->dzs2, n->dp2, n->a2, n->dz2);
     NCHK(wgrad(n, s, 2, n->p1, n->dz2));
     NCHK(dgrad(n, s, 2, n->dz2, nullptr, n->dp1));
-    launch_pairs(k_combine, g3(n, 1), 4, s, n->dzs1, n->dp1, n->a1, n->dz1);
+    launch_pairs(n->pdl, k_combine, g3(n, 1), 4, s, n->dzs1, n->dp1, n->a1, n->dz1);
     NCHK(wgrad(n, s, 1, n->p0, n->dz1));
     NCHK(dgrad(n, s, 1, n->dz1, nullptr, n->dp0));
-    launch_pairs(k_combine, g3(n, 0), 2, s, n->dzs0, n->dp0, n->a0, n->dz0);
+    launch_pairs(n->pdl, k_combine, g3(n, 0), 2, s, n->dzs0, n->dp0, n->a0, n->dz0);
     NCHK(wgrad(n, s, 0, n->x0, n->dz0));
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
 }
@@ -648,12 +649,12 @@ int loss(TurbNet *n, cudaStream_t s, const MgDevLevel &L0, const double *invd, c
     pcg_resid(s, L0, n->r64, n->x64, n->rr, n->part, nullptr, nullptr);
     pcg_reduce(s, n->part, 1, n->sc + 2, np);
     if (want_grad) {
-        pcg_apply(s, L0, n->rr, n->q64, n->part, nullptr, nullptr);
+        pcg_apply(s, L0, n->rr, n->q64, n->part, nullptr, nullptr, n->pdl);
         k_loss_grad<<<nblk(V), 256, 0, s>>>(V, n->q64, invd, n->gout);
         if (n->wr != 1.0) k_scale_f<<<nblk(V), 256, 0, s>>>(V, (float)n->wr, n->gout);
     }
     k_energy_in<<<nblk(V), 256, 0, s>>>(V, n->hout, snap + 3 * V, invd, n->x64);
-    pcg_apply(s, L0, n->x64, n->q64, n->part, nullptr, nullptr);
+    pcg_apply(s, L0, n->x64, n->q64, n->part, nullptr, nullptr, n->pdl);
     pcg_reduce(s, n->part, 1, n->sc + 3, np);
     if (want_grad && n->we != 0.0) k_grad_add<<<nblk(V), 256, 0, s>>>(V, n->we, e0, n->q64, invd, n->gout);
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
@@ -678,9 +679,10 @@ int snaps_dims(const TurbSnaps *s, int *nx, int *ny, int *nz)
 }
 
 int net_guess(TurbNet *n, cudaStream_t st, const MgDevLevel &L0, const double *invd, const double *r1,
-              const double *bw, const double *p1, const double *p2, const double *base, double *out)
+              const double *bw, const double *p1, const double *p2, const double *base, double *out, int pdl)
 {
     if (!n || !same_grid(n, L0)) return TURB_ERR_ARG;
+    n->pdl = pdl;
     if (ensure_parts(&n->part, &n->nparts, L0)) return TURB_ERR_ALLOC;
     long long V = n->V[0];
     input_norms(st, V, r1, bw, p1, p2, n->part, n->sc);
@@ -707,7 +709,7 @@ int net_snapshot(TurbSnaps *sn, cudaStream_t st, const MgDevLevel &L0, const dou
 }
 
 int net_snapshot_finish(TurbSnaps *sn, cudaStream_t st, const MgDevLevel &L0, const double *invd, const double *p,
-                        int converged)
+                        int converged, int pdl)
 {
     if (!sn || sn->pending < 0) return TURB_OK;
     int k = sn->pending;
@@ -722,15 +724,16 @@ int net_snapshot_finish(TurbSnaps *sn, cudaStream_t st, const MgDevLevel &L0, co
     float *t = sn->data + (long long)k * SNAP_CH * V + 3 * V;
     k_target<<<nblk(V), 256, 0, st>>>(V, p, sn->base, invd, sn->sc, t);
     k_t64<<<nblk(V), 256, 0, st>>>(V, t, invd, sn->x64);
-    pcg_apply(st, L0, sn->x64, sn->q64, sn->part, nullptr, nullptr);
+    pcg_apply(st, L0, sn->x64, sn->q64, sn->part, nullptr, nullptr, pdl);
     pcg_reduce(st, sn->part, 1, sn->e0 + k, pcg_stencil_parts(L0));
     return cudaGetLastError() == cudaSuccess ? TURB_OK : TURB_ERR_CUDA;
 }
 
 int net_train(TurbNet *n, cudaStream_t st, const MgDevLevel &L0, const double *invd, TurbSnaps *sn, int steps,
-              float lr, unsigned long long seed, double *mean_loss)
+              float lr, unsigned long long seed, double *mean_loss, int pdl)
 {
     if (!n || !sn || !n->train || !same_grid(n, L0) || sn->n < 1 || steps < 1) return TURB_ERR_ARG;
+    n->pdl = pdl;
     if (ensure_parts(&n->part, &n->nparts, L0)) return TURB_ERR_ALLOC;
     Rng rng{seed};
     double *hbuf = nullptr;
@@ -764,9 +767,10 @@ int net_train(TurbNet *n, cudaStream_t st, const MgDevLevel &L0, const double *i
 }
 
 int net_eval(TurbNet *n, cudaStream_t st, const MgDevLevel &L0, const double *invd, TurbSnaps *sn, int first,
-             int count, double *mean_res, double *mean_energy)
+             int count, double *mean_res, double *mean_energy, int pdl)
 {
     if (!n || !sn || !same_grid(n, L0) || first < 0 || count < 1 || first + count > sn->n) return TURB_ERR_ARG;
+    n->pdl = pdl;
     if (ensure_parts(&n->part, &n->nparts, L0)) return TURB_ERR_ALLOC;
     if (!n->x64) {   // inference nets get the loss buffers on first use
         n->x64 = n->alloc<double>(n->V[0]); n->r64 = n->alloc<double>(n->V[0]);
@@ -926,6 +930,7 @@ int turb_net_forward(turb_net *h, const float *in3, float *out, void *stream)
     TurbNet *n = reinterpret_cast<TurbNet *>(h);
     if (!n || !in3 || !out) return TURB_ERR_ARG;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    n->pdl = 1;
     NCHK(forward(n, s, in3, out));
     return read_err(n, s);
 }
@@ -935,6 +940,7 @@ int turb_net_backward(turb_net *h, const float *gout, void *stream)
     TurbNet *n = reinterpret_cast<TurbNet *>(h);
     if (!n || !n->train || !gout) return TURB_ERR_ARG;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    n->pdl = 1;
     NCHK(backward(n, s, gout));
     return read_err(n, s);
 }
@@ -1048,8 +1054,8 @@ int turb_conv3_test(int X, int Y, int Z, int cin, int cout, const void *in, cons
     e.bias = dgrad_mode ? nullptr : bias;
     e.relu = relu;
     e.out = reinterpret_cast<bf16 *>(out);
-    int rc = dgrad_mode ? conv3_fwd(s, reinterpret_cast<const bf16 *>(in), X, Y, Z, cout, cin, wd, e, err, nsm)
-                        : conv3_fwd(s, reinterpret_cast<const bf16 *>(in), X, Y, Z, cin, cout, wf, e, err, nsm);
+    int rc = dgrad_mode ? conv3_fwd(s, reinterpret_cast<const bf16 *>(in), X, Y, Z, cout, cin, wd, e, err, nsm, 1)
+                        : conv3_fwd(s, reinterpret_cast<const bf16 *>(in), X, Y, Z, cin, cout, wf, e, err, nsm, 1);
     int h = 0;
     cudaError_t ce = cudaStreamSynchronize(s);
     if (ce == cudaSuccess) ce = cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost);
@@ -1071,7 +1077,7 @@ int turb_conv3_wgrad_test(int X, int Y, int Z, int cin, int cout, const void *x,
     cudaMemsetAsync(err, 0, sizeof(int), s);
     cudaMemsetAsync(dw, 0, 27ull * cin * cout * sizeof(float), s);
     int rc = conv3_wgrad(s, reinterpret_cast<const bf16 *>(x), reinterpret_cast<const bf16 *>(dy), X, Y, Z, cin, cout,
-                         dw, err, nsm);
+                         dw, err, nsm, 1);
     int h = 0;
     cudaError_t ce = cudaStreamSynchronize(s);
     if (ce == cudaSuccess) ce = cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost);

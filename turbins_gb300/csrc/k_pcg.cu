@@ -498,22 +498,6 @@ int pcg_nparts() { return NP; }
 // blocks of the grid-stride kernels: NP, or as many as have elements
 static unsigned nblk(long long n) { return (unsigned)std::min<long long>(NP, (n + BS - 1) / BS); }
 
-// a launch with the programmatic stream serialisation attribute
-template <typename... P, typename... A>
-static void launch_pdl(void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 static dim3 g3k(const MgDevLevel &L)
 {
     return dim3((unsigned)((L.nx + 31) / 32), (unsigned)((L.ny + 7) / 8), (unsigned)((L.nz + KC - 1) / KC));
@@ -568,13 +552,13 @@ void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const dou
 }
 
 void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc,
-               unsigned *count)
+               unsigned *count, int pdl)
 {
     const int np = pcg_stencil_parts(L0), g = groups(L0);
     const dim3 gr = g3g(L0, g), b(32, 8);
-    if (g == 4) launch_pdl(k_apply<4>, gr, b, s, L0, p, q, part, np, sc, count);
-    else if (g == 2) launch_pdl(k_apply<2>, gr, b, s, L0, p, q, part, np, sc, count);
-    else launch_pdl(k_apply<1>, gr, b, s, L0, p, q, part, np, sc, count);
+    if (g == 4) launch_early(pdl, k_apply<4>, gr, b, 0u, s, L0, p, q, part, np, sc, count);
+    else if (g == 2) launch_early(pdl, k_apply<2>, gr, b, 0u, s, L0, p, q, part, np, sc, count);
+    else launch_early(pdl, k_apply<1>, gr, b, 0u, s, L0, p, q, part, np, sc, count);
 }
 
 void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part, double *dst, unsigned *count)
@@ -584,23 +568,23 @@ void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, doub
 }
 
 void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part,
-              PcgScal *sc, int restart, unsigned *count)
+              PcgScal *sc, int restart, unsigned *count, int pdl)
 {
     const unsigned nb = nblk(n);
-    launch_pdl(k_dot2, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, r, z, rold, part, sc, restart, count);
+    launch_early(pdl, k_dot2, dim3((nb + VB - 1) / VB), dim3(BS), 0u, s, n, (int)nb, r, z, rold, part, sc, restart, count);
 }
 
-void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first)
+void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first, int pdl)
 {
     const unsigned nb = nblk(n);
-    launch_pdl(k_pupdate, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, z, p, sc, first);
+    launch_early(pdl, k_pupdate, dim3((nb + VB - 1) / VB), dim3(BS), 0u, s, n, (int)nb, z, p, sc, first);
 }
 
 void pcg_xrupdate(cudaStream_t s, long long n, double *x, double *r, double *rold, const double *p,
-                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count)
+                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count, int pdl)
 {
     const unsigned nb = nblk(n);
-    launch_pdl(k_xrupdate, dim3((nb + VB - 1) / VB), dim3(BS), s, n, (int)nb, x, r, rold, p, q, sc, part, host_rr, count);
+    launch_early(pdl, k_xrupdate, dim3((nb + VB - 1) / VB), dim3(BS), 0u, s, n, (int)nb, x, r, rold, p, q, sc, part, host_rr, count);
 }
 
 void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper)

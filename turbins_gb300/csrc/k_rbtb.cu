@@ -406,15 +406,5 @@ void mg_tb_sweeps(cudaStream_t s, const RbTbPlan &p, int in, int c0, int zero_in
     a.tiles_x = p.tiles_x;
     a.ntiles = p.ntiles;
     a.err = p.err;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p.grid);
-    cfg.blockDim = dim3(TB_THREADS);
-    cfg.dynamicSmemBytes = mg_tb_smem();
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, k_rbgs_tb, p.mx[in], a);
+    launch_early(pdl, k_rbgs_tb, dim3((unsigned)p.grid), dim3(TB_THREADS), (unsigned)mg_tb_smem(), s, p.mx[in], a);
 }

@@ -644,29 +644,10 @@ void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e)
     k_add_corr<<<1216, 256, 0, s>>>(n, x, e);
 }
 
-// a launch with the programmatic stream serialisation attribute: the kernel
-// may start while the one before it on the stream runs (the immersed rows'
-// kernels are written for that: they read nothing the stencil kernel writes,
-// write only immersed points, and end with pdl_wait)
-template <typename... P, typename... A>
-static void launch_pdl(void (*k)(P...), dim3 g, dim3 b, cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 // |r|^2 goes to *dst, the first sweep's result to e0, 1/dt for the others to *adt
 void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
                          const double *b, const double *x, float *rf, float *e0, float *adt, const IbDev &ib,
-                         const IbDevF &ibf, double *part, unsigned *count, double *dst)
+                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int pdl)
 {
     const long long hp = helm_parts(d);
     const unsigned nib = (unsigned)((ib.n + 255) / 256);
@@ -677,7 +658,9 @@ void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const 
     const SumTo to{(int)(hp + nib), gr.x * gr.y * gr.z + nib, count, dst};
     const auto k = g == 4 ? k_helm_resid64<4> : g == 2 ? k_helm_resid64<2> : g == 1 ? k_helm_resid64<1> : k_helm_resid64<0>;
     k<<<gr, dim3(HBX, HBY), 0, s>>>(d, h, hf, st, a_dt, b, x, rf, e0, adt, part, to);
-    if (ib.n > 0) launch_pdl(k_ib_resid64, dim3(nib), dim3(256), s, ib, ibf, b, x, rf, e0, part, hp, to);
+    // the immersed rows beside it: they read nothing that it writes, write
+    // only immersed points and end with pdl_wait
+    if (ib.n > 0) launch_early(pdl, k_ib_resid64, dim3(nib), dim3(256), 0u, s, ib, ibf, b, x, rf, e0, part, hp, to);
 }
 
 // The sweep after the first ones: from e to en, or (x given) added to x.
@@ -685,7 +668,8 @@ void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const 
 // sweeps but the last march along k through shared-memory plane tiles
 // (k_helm_jac32z); 0: k_helm_jac32v throughout
 void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, const float *adt,
-                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching)
+                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching,
+                       int pdl)
 {
     dim3 g((unsigned)((d.NX + 4 * HBX - 1) / (4 * HBX)), (unsigned)((d.NY + HBY - 1) / HBY),
            (unsigned)((d.NZ + KCJ - 1) / KCJ));
@@ -700,6 +684,6 @@ void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const u
     }
     const auto k = x ? k_helm_jac32v<true> : k_helm_jac32v<false>;
     if (alone || marching) k<<<g, dim3(HBX, HBY), 0, s>>>(d, h, st, adt, r, e, en, x);
-    else launch_pdl(k, g, dim3(HBX, HBY), s, d, h, st, adt, r, e, en, x);
-    if (ib.n > 0) launch_pdl(k_ib_jac32, dim3((ib.n + 255) / 256), dim3(256), s, ib, r, e, en, x);
+    else launch_early(pdl, k, g, dim3(HBX, HBY), 0u, s, d, h, st, adt, r, e, en, x);
+    if (ib.n > 0) launch_early(pdl, k_ib_jac32, dim3((ib.n + 255) / 256), dim3(256), 0u, s, ib, r, e, en, x);
 }

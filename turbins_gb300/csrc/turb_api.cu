@@ -1377,6 +1377,8 @@ int turb_set_sweep_kernels(turb_ctx *c, int variants)
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         for (auto &g : c->g_mg)
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+        for (auto &g : c->g_pcg)
+            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
     c->kvariant = variants;
     c->H64.marching = (variants & TURB_KV_MARCHING) ? 1 : 0;
@@ -1466,7 +1468,7 @@ int turb_net_train(turb_net *net, turb_ctx *c, turb_snaps *snaps, int steps, flo
 {
     if (!c || !net || !snaps) return TURB_ERR_ARG;
     return net_train(reinterpret_cast<TurbNet *>(net), c->s, c->H64.lev[0], c->H64.invd[0],
-                     reinterpret_cast<TurbSnaps *>(snaps), steps, lr, seed, mean_loss);
+                     reinterpret_cast<TurbSnaps *>(snaps), steps, lr, seed, mean_loss, c->H32.pdl);
 }
 
 int turb_net_eval(turb_net *net, turb_ctx *c, turb_snaps *snaps, int first, int count, double *mean_residual,
@@ -1474,7 +1476,7 @@ int turb_net_eval(turb_net *net, turb_ctx *c, turb_snaps *snaps, int first, int 
 {
     if (!c || !net || !snaps) return TURB_ERR_ARG;
     return net_eval(reinterpret_cast<TurbNet *>(net), c->s, c->H64.lev[0], c->H64.invd[0],
-                    reinterpret_cast<TurbSnaps *>(snaps), first, count, mean_residual, mean_energy);
+                    reinterpret_cast<TurbSnaps *>(snaps), first, count, mean_residual, mean_energy, c->H32.pdl);
 }
 
 int turb_pressure_guess_ratio(turb_ctx *c, double *geo_mean)
@@ -2449,7 +2451,7 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
     for (;;) {
         int ph = prof_begin(c, TURB_PROF_JACOBI);
         launch_helm_resid64(c->s, d, h, hf, c->st[q], a_dt, b, x, c->hrf, c->he0, c->hadt, ib, ibf, c->part,
-                            c->count, c->hscal + HS_R);
+                            c->count, c->hscal + HS_R, c->H32.pdl);
         prof_end(c, ph, 1, HELM_RESID64_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
         c->launches += 1 + (ib.n > 0);
         TURB_CHECK(cudaStreamSynchronize(c->s));
@@ -2463,7 +2465,7 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
             float *ea = c->he0, *eb = c->he1;
             for (int t = 1; t < c->hinner; t++) {
                 launch_helm_jac32(c->s, d, hf, c->st[q], c->hadt, c->hrf, ea, eb, t == c->hinner - 1 ? x : nullptr, ibf,
-                                  t == 1, c->kvariant & TURB_KV_MARCHING);
+                                  t == 1, c->kvariant & TURB_KV_MARCHING, c->H32.pdl);
                 std::swap(ea, eb);
             }
         };
@@ -2689,7 +2691,7 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             // candidate = previous pressure + network correction of its residual
             ph = prof_begin(c, TURB_PROF_NET);
             int rc = net_guess(c->net, s, L0, c->H64.invd[0], c->pr, c->pbw, c->ph[st][0], c->ph[st][1], c->px,
-                               c->pz);
+                               c->pz, c->H32.pdl);
             if (rc) return rc;
             c->launches += NET_GUESS_LAUNCHES;
             ok = 1;
@@ -2788,10 +2790,10 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
             }
         };
         auto cgstep = [&](int rs) {
-            pcg_dot2(s, n0, c->pr, c->pz, c->pro, c->part, sc, rs, c->count);   // r.z, z.r_old, beta
-            pcg_pupdate(s, n0, c->pz, c->pp, sc, rs);
-            pcg_apply(s, L0, c->pp, c->pq, c->part, sc, c->count);               // q = S p, p.q, alpha
-            pcg_xrupdate(s, n0, c->px, c->pr, c->pro, c->pp, c->pq, sc, c->part, c->hscal + 1, c->count);
+            pcg_dot2(s, n0, c->pr, c->pz, c->pro, c->part, sc, rs, c->count, c->H32.pdl);   // r.z, z.r_old, beta
+            pcg_pupdate(s, n0, c->pz, c->pp, sc, rs, c->H32.pdl);
+            pcg_apply(s, L0, c->pp, c->pq, c->part, sc, c->count, c->H32.pdl);   // q = S p, p.q, alpha
+            pcg_xrupdate(s, n0, c->px, c->pr, c->pro, c->pp, c->pq, sc, c->part, c->hscal + 1, c->count, c->H32.pdl);
         };
         const int nmg = vl + (pm ? 2 : 0), ncg = 4;
         auto precondition = [&]() -> int {
@@ -2857,7 +2859,7 @@ int turb_Pressure_solve(turb_ctx *c, int *iters, double *relres)
     pcg_scatter(s, d, L0, c->px, c->fld[TURB_F_PHI]);
     c->launches += 1;
     if (c->snaps) {
-        int rc = net_snapshot_finish(c->snaps, s, L0, c->H64.invd[0], c->px, status == TURB_OK);
+        int rc = net_snapshot_finish(c->snaps, s, L0, c->H64.invd[0], c->px, status == TURB_OK, c->H32.pdl);
         if (rc) return rc;
     }
     // the per-stage history of converged pressures (what the extrapolated and

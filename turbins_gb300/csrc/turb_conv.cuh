@@ -11,6 +11,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "turb_internal.cuh"
+
 typedef __nv_bfloat16 bf16;
 
 // which kernel runs one convolution on one grid, and its weight layout
@@ -49,34 +51,19 @@ inline long long conv_pack_elems(int cin, int cout)
 }
 
 int conv3_fwd(cudaStream_t s, const bf16 *in, int X, int Y, int Z, int cin, int cout, const bf16 *wpk,
-              const ConvEpi &e, int *err, int nsm);
+              const ConvEpi &e, int *err, int nsm, int pdl);
 int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int Z, int cin, int cout, float *dw,
-                int *err, int nsm);
+                int *err, int nsm, int pdl);
 int conv_selftest_umma(int mn_major, int swap, unsigned long long *mismatches);
 const char *conv_last_error();
 
-// Launches a network kernel as a programmatic dependent of the one before it
-// on the stream: its set-up (barriers, TMEM, resident weights) overlaps that
-// kernel's tail.  Every such kernel calls pdl_trigger and, before it reads or
-// writes anything the others do, pdl_wait; the first kernel of a pass is an
-// ordinary launch, so what was written before the pass is visible to all
-template <typename... P, typename... A>
-inline void net_launch(void (*k)(P...), dim3 grid, dim3 block, uint32_t smem, cudaStream_t s, A... args)
+// A network kernel starts while the one before it on the stream drains (pdl):
+// its set-up (barriers, TMEM, resident weights) overlaps that kernel's tail.
+// Every such kernel calls pdl_trigger and, before it reads or writes anything
+// the others do, pdl_wait; the first kernel of a pass is an ordinary launch,
+// so what was written before the pass is visible to all
+template <typename K, typename... A>
+inline void net_launch(int pdl, K k, int gx, int gy, int threads, uint32_t smem, cudaStream_t s, A... args)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, P(args)...);
-}
-template <typename... P, typename... A>
-inline void net_launch(void (*k)(P...), int gx, int gy, int threads, uint32_t smem, cudaStream_t s, A... args)
-{
-    net_launch(k, dim3((unsigned)gx, (unsigned)gy), dim3((unsigned)threads), smem, s, args...);
+    launch_early(pdl, k, dim3((unsigned)gx, (unsigned)gy), dim3((unsigned)threads), smem, s, args...);
 }

@@ -174,6 +174,24 @@ __device__ __forceinline__ double turb_warp_maxbits(double v)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A launch; early: with that attribute.  A failure stays in the runtime's last
+// error, which the callers' check_launch, launch_error or cudaGetLastError read.
+template <typename... P, typename... A>
+inline void launch_early(int early, void (*k)(P...), dim3 grid, dim3 block, unsigned smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 #define TURB_CHECK(x)                                                          \
     do {                                                                       \
         cudaError_t e_ = (x);                                                  \

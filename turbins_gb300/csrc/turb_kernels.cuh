@@ -71,7 +71,8 @@ long long helm_parts(const Dims &d);
 void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e);
 void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
                          const double *b, const double *x, float *rf, float *e0, float *adt, const IbDev &ib,
-                         const IbDevF &ibf, double *part, unsigned *count, double *dst);
+                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int pdl);
 void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, const float *adt,
-                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching);
+                       const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching,
+                       int pdl);
 void launch_norm2(cudaStream_t s, long long n, const double *x, double *part, unsigned *count, double *dst);

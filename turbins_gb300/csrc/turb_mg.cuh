@@ -89,7 +89,7 @@ struct MgHier {
     // 1: FP64 half sweeps and residuals of large levels march along k
     // (k_rbgs_col, k_resid_col); 0: k_rbgs, k_resid throughout
     int columns = 1;
-    // 1: the V-cycle's kernels use programmatic dependent launch
+    // 1: the kernels of the V-cycle and of the CG step use programmatic dependent launch
     int pdl = 1;
     // from this level on (-1: never) the V-cycle runs as one launch of one
     // thread-block cluster of cluster_ctas blocks (k_vcycle_cluster)
@@ -169,18 +169,20 @@ void pcg_scatter(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const doub
 // The sums of these end in the launch itself (the last block adds the
 // partials; count: a zero word the launch leaves zero): |r|^2, p.q and alpha,
 // a.b, r.z, z.r_old and beta, |r|^2 (also to the page-locked *host_rr).  With
-// count null, pcg_resid and pcg_apply leave the partials for pcg_reduce
+// count null, pcg_resid and pcg_apply leave the partials for pcg_reduce.  pdl:
+// the kernel may be scheduled while the one ahead of it drains
 void pcg_resid(cudaStream_t s, const MgDevLevel &L0, const double *bw, const double *x, double *r, double *part,
                double *dst, unsigned *count);
-void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc, unsigned *count);
+void pcg_apply(cudaStream_t s, const MgDevLevel &L0, const double *p, double *q, double *part, PcgScal *sc,
+               unsigned *count, int pdl);
 void pcg_dot(cudaStream_t s, long long n, const double *a, const double *b, double *part, double *dst, unsigned *count);
 void pcg_dot2(cudaStream_t s, long long n, const double *r, const double *z, const double *rold, double *part,
-              PcgScal *sc, int restart, unsigned *count);
+              PcgScal *sc, int restart, unsigned *count, int pdl);
 int pcg_stencil_parts(const MgDevLevel &L);
 void pcg_reduce(cudaStream_t s, const double *part, int nvals, double *dst, int nper = 0);
-void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first);
+void pcg_pupdate(cudaStream_t s, long long n, const double *z, double *p, const PcgScal *sc, int first, int pdl);
 void pcg_xrupdate(cudaStream_t s, long long n, double *x, double *r, double *rold, const double *p,
-                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count);
+                  const double *q, PcgScal *sc, double *part, double *host_rr, unsigned *count, int pdl);
 void pcg_to_float(cudaStream_t s, long long n, const double *a, float *b);
 void pcg_to_double(cudaStream_t s, long long n, const float *a, double *b);
 // the same into / out of a level's storage order (colour-split or not)
