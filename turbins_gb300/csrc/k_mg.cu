@@ -1068,11 +1068,11 @@ const dim3 B38(32, 8, 1);
 // planes a block of the marching FP64 kernels takes of a launch of g blocks,
 // one per plane: the most (up to 8) that leave two blocks per SM, 0 where two
 // planes leave fewer
-static int col_planes(dim3 g)
+static int col_planes(dim3 g, int nsm)
 {
     int planes = 8;
-    while (planes > 2 && (long long)g.x * g.y * ((g.z + planes - 1) / planes) < 2 * 152) planes >>= 1;
-    return (long long)g.x * g.y * ((g.z + planes - 1) / planes) >= 2 * 152 ? planes : 0;
+    while (planes > 2 && (long long)g.x * g.y * ((g.z + planes - 1) / planes) < 2 * nsm) planes >>= 1;
+    return (long long)g.x * g.y * ((g.z + planes - 1) / planes) >= 2 * nsm ? planes : 0;
 }
 
 template <typename T>
@@ -1081,26 +1081,27 @@ void mg_setup_invdiag(cudaStream_t s, const MgDevLevel &L, T *invd)
     k_invdiag<T><<<1024, 256, 0, s>>>(L, invd);
 }
 
-// One V-cycle from level l: input b[l], output x[l] (x starts at zero).
-// one red-black half sweep of level L: the vectorised kernel where the
-// level is colour-split FP32 with nx a multiple of 8
-// marching: half sweeps after the first of a cycle march along k (k_rbgs4z)
-// on the levels large enough to fill the GPU with them; columns: the same for
-// the FP64 levels (k_rbgs_col)
+// One red-black half sweep of level l: the vectorised kernel where the level
+// is colour-split FP32 with nx a multiple of 8.  H.marching: half sweeps after
+// the first of a cycle march along k (k_rbgs4z) on the levels large enough to
+// fill the GPU with them; H.columns: the same for the FP64 levels (k_rbgs_col)
 template <typename T>
-void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, const T *b, const T *invd, T *x,
-             int marching, int columns, int pdl)
+void rb_half(cudaStream_t s, const MgHier<T> &H, int l, int color, int zero_init)
 {
+    const MgDevLevel &L = H.lev[l];
+    const T *b = H.b[l], *invd = H.invd[l];
+    T *x = H.x[l];
+    const int pdl = H.pdl;
     if constexpr (sizeof(T) == 4) {
         if (L.split && L.nx % 8 == 0) {
             dim3 g4((unsigned)((L.nx / 8 + 31) / 32), (unsigned)((L.ny + 7) / 8), (unsigned)L.nz);
-            if (marching && !zero_init) {
+            if (H.marching && !zero_init) {
                 // planes per block: the most (up to 16) that still gives two
                 // waves of three blocks on every SM
                 long long bxy = (long long)g4.x * g4.y;
                 int jz = 16;
-                while (jz > 2 && bxy * ((L.nz + jz - 1) / jz) < 2 * 3 * 152) jz >>= 1;
-                if (bxy * ((L.nz + jz - 1) / jz) >= 152) {
+                while (jz > 2 && bxy * ((L.nz + jz - 1) / jz) < 2 * 3 * H.nsm) jz >>= 1;
+                if (bxy * ((L.nz + jz - 1) / jz) >= H.nsm) {
                     dim3 gz(g4.x, g4.y, (unsigned)((L.nz + jz - 1) / jz));
                     launch_k(pdl, k_rbgs4z, gz, B38, s, L, color, jz, b, invd, x);
                     return;
@@ -1126,8 +1127,8 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
     }
     if constexpr (sizeof(T) == 8) {
         dim3 g = g3(L.nx >> 1, L.ny, L.nz);
-        const int planes = col_planes(g);
-        if (columns && !zero_init && L.nx % 2 == 0 && planes) {
+        const int planes = col_planes(g, H.nsm);
+        if (H.columns && !zero_init && L.nx % 2 == 0 && planes) {
             g.z = (g.z + planes - 1) / planes;
             launch_k(pdl, k_rbgs_col<T>, g, B38, s, L, color, planes, b, invd, x);
             return;
@@ -1137,8 +1138,12 @@ void rb_half(cudaStream_t s, const MgDevLevel &L, int color, int zero_init, cons
 }
 
 template <typename T>
-void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r, int columns, int pdl)
+void resid_lev(cudaStream_t s, const MgHier<T> &H, int l)
 {
+    const MgDevLevel &L = H.lev[l];
+    const T *b = H.b[l], *x = H.x[l];
+    T *r = H.r[l];
+    const int pdl = H.pdl;
     if constexpr (sizeof(T) == 4) {
         if (L.split && L.nx % 8 == 0) {
             dim3 g8((unsigned)((L.nx / 8 + 31) / 32), (unsigned)((L.ny + 7) / 8), (unsigned)L.nz);
@@ -1147,8 +1152,8 @@ void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r
         }
     }
     if constexpr (sizeof(T) == 8) {
-        const int planes = col_planes(g3(L.nx, L.ny, L.nz));
-        if (columns && planes) {
+        const int planes = col_planes(g3(L.nx, L.ny, L.nz), H.nsm);
+        if (H.columns && planes) {
             dim3 g = g3(L.nx, L.ny, L.nz);
             g.z = (g.z + planes - 1) / planes;
             launch_k(pdl, k_resid_col<T>, g, B38, s, L, planes, b, x, r);
@@ -1158,6 +1163,7 @@ void resid_lev(cudaStream_t s, const MgDevLevel &L, const T *b, const T *x, T *r
     launch_k(pdl, k_resid<T>, g3(L.nx, L.ny, L.nz), B38, s, L, b, x, r);
 }
 
+// One V-cycle from level l: input b[l], output x[l] (x starts at zero).
 template <typename T>
 void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const int *post)
 {
@@ -1231,10 +1237,10 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
     for (int it = pre_done; it < npre; it++) {
         // the first colour-0 half sweep takes x = 0 (it reads no neighbours);
         // every colour-1 point is then rewritten from colour-0 values only
-        rb_half<T>(s, L, 0, it == 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
-        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
+        rb_half<T>(s, H, l, 0, it == 0);
+        rb_half<T>(s, H, l, 1, 0);
     }
-    resid_lev<T>(s, L, H.b[l], H.x[l], H.r[l], H.columns, H.pdl);
+    resid_lev<T>(s, H, l);
     const MgDevLevel &C = H.lev[l + 1];
     bool yz8 = false;
     if constexpr (sizeof(T) == 4) yz8 = L.cx == 0 && L.nx % 8 == 0 && C.nx == L.nx;
@@ -1253,8 +1259,8 @@ void mg_vcycle(cudaStream_t s, const MgHier<T> &H, int l, const int *pre, const 
         for (int f = 0; f < post_done / 2; f++) mg_tb_sweeps(s, *H.tb, f & 1, 1, 0, H.pdl);
     }
     for (int it = post_done; it < npost; it++) {
-        rb_half<T>(s, L, 1, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
-        rb_half<T>(s, L, 0, 0, H.b[l], H.invd[l], H.x[l], H.marching, H.columns, H.pdl);
+        rb_half<T>(s, H, l, 1, 0);
+        rb_half<T>(s, H, l, 0, 0);
     }
 }
 

@@ -620,12 +620,12 @@ void launch_helm_apply(cudaStream_t s, const Dims &d, const HelmTab &h, const ui
 // part must hold helm_parts(d) + (ib.n+255)/256 entries; |r|^2 goes to *dst
 void launch_helm_jacobi(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
                         const double *b, const double *x, double *xn, const IbDev &ib, double *part,
-                        unsigned *count, double *dst)
+                        unsigned *count, double *dst, int nsm)
 {
     const long long hp = helm_parts(d);
     const unsigned nib = (unsigned)((ib.n + 255) / 256);
     const SumTo to{(int)(hp + nib), (unsigned)hp + nib, count, dst};
-    const auto k = hp <= 2 * 152 ? k_helm_jacobi<true> : k_helm_jacobi<false>;
+    const auto k = hp <= 2 * nsm ? k_helm_jacobi<true> : k_helm_jacobi<false>;
     k<<<hgrid(d), dim3(HBX, HBY), 0, s>>>(d, h, st, a_dt, b, x, xn, part, to);
     if (ib.n > 0) k_ib_jacobi<<<nib, 256, 0, s>>>(ib, b, x, xn, part, hp, to);
 }
@@ -647,12 +647,12 @@ void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e)
 // |r|^2 goes to *dst, the first sweep's result to e0, 1/dt for the others to *adt
 void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
                          const double *b, const double *x, float *rf, float *e0, float *adt, const IbDev &ib,
-                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int pdl)
+                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int nsm, int pdl)
 {
     const long long hp = helm_parts(d);
     const unsigned nib = (unsigned)((ib.n + 255) / 256);
     // groups per block: as many as leave about seven blocks per SM
-    const int g = hp >= 4096 ? 4 : hp >= 2048 ? 2 : hp > 2 * 152 ? 1 : 0;
+    const int g = hp >= 4096 ? 4 : hp >= 2048 ? 2 : hp > 2 * nsm ? 1 : 0;
     dim3 gr = hgrid(d);
     if (g) gr.z = (gr.z + g - 1) / g;
     const SumTo to{(int)(hp + nib), gr.x * gr.y * gr.z + nib, count, dst};

@@ -179,6 +179,7 @@ struct turb_ctx {
     // kernel variants (TURB_KV_*): FP32 sweeps marching along k through
     // shared-memory plane tiles, ENO y / z lines walked in segments
     int kvariant = TURB_KV_ENO_SEGMENTS | TURB_KV_PDL;
+    int nsm = 1;                    // SMs of the device
     long long mg_tail_cells = -1;   // turb_set_mg_tail (-1: the default rule of place_tail)
     int low_held[2] = {0, 0};       // blocks of k_vcycle_low's cluster that the device holds, FP64 and FP32
     long long mg_cluster_cells = 1 << 17;   // TURB_KV_CLUSTER_VCYCLE from the first level of at most this many cells
@@ -929,6 +930,7 @@ int build_mg(turb_ctx *c)
     c->count = c->mem.alloc<unsigned>(4);
     c->H64.cluster_ctas = mg_cluster_ctas<double>();
     c->H32.cluster_ctas = mg_cluster_ctas<float>();
+    c->H64.nsm = c->H32.nsm = c->nsm;
     c->low_held[0] = c->H64.low_ctas = mg_low_ctas<double>();
     c->low_held[1] = c->H32.low_ctas = mg_low_ctas<float>();
     set_cluster_from(c);
@@ -1092,6 +1094,13 @@ int turb_create(const turb_grid_desc *g, const turb_params *p, turb_ctx **out)
     c->xu.assign(g->xu, g->xu + d.NX); c->yv.assign(g->yv, g->yv + d.NY); c->zw.assign(g->zw, g->zw + d.NZ);
     metrics(c);
     if (cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking) != cudaSuccess) { delete c; return TURB_ERR_CUDA; }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaStreamDestroy(c->s);
+        delete c;
+        return TURB_ERR_CUDA;
+    }
     DevBuf &m = c->mem;
     c->geo.xc = m.upload(c->xc); c->geo.yc = m.upload(c->yc); c->geo.zc = m.upload(c->zc);
     c->geo.xu = m.upload(c->xu); c->geo.yv = m.upload(c->yv); c->geo.zw = m.upload(c->zw);
@@ -2416,7 +2425,8 @@ static int helm_solve_fp64(turb_ctx *c, int q, int ic, int fx, int fb, double dt
     for (;;) {
         double *x = c->fld[fx];
         int ph = prof_begin(c, TURB_PROF_JACOBI);
-        launch_helm_jacobi(c->s, d, h, c->st[q], a_dt, b, x, c->jtmp, ib, c->part, c->count, c->hscal + HS_R);
+        launch_helm_jacobi(c->s, d, h, c->st[q], a_dt, b, x, c->jtmp, ib, c->part, c->count, c->hscal + HS_R,
+                           c->nsm);
         prof_end(c, ph, 1, HELM_JACOBI_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
         c->launches += 1 + (ib.n > 0);
         TURB_CHECK(cudaStreamSynchronize(c->s));
@@ -2451,7 +2461,7 @@ static int helm_solve_mixed(turb_ctx *c, int q, int ic, int fx, int fb, double d
     for (;;) {
         int ph = prof_begin(c, TURB_PROF_JACOBI);
         launch_helm_resid64(c->s, d, h, hf, c->st[q], a_dt, b, x, c->hrf, c->he0, c->hadt, ib, ibf, c->part,
-                            c->count, c->hscal + HS_R, c->H32.pdl);
+                            c->count, c->hscal + HS_R, c->nsm, c->H32.pdl);
         prof_end(c, ph, 1, HELM_RESID64_BYTES * ((double)d.NX * d.NY * d.NZ) + IB_ROW_BYTES * ib.n);
         c->launches += 1 + (ib.n > 0);
         TURB_CHECK(cudaStreamSynchronize(c->s));

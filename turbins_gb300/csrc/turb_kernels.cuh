@@ -66,12 +66,12 @@ void launch_helm_apply(cudaStream_t s, const Dims &d, const HelmTab &h, const ui
                        const double *x, double *y, const IbDev &ib);
 void launch_helm_jacobi(cudaStream_t s, const Dims &d, const HelmTab &h, const uint8_t *st, double a_dt,
                         const double *b, const double *x, double *xn, const IbDev &ib, double *part,
-                        unsigned *count, double *dst);
+                        unsigned *count, double *dst, int nsm);
 long long helm_parts(const Dims &d);
 void launch_add_corr(cudaStream_t s, long long n, double *x, const float *e);
 void launch_helm_resid64(cudaStream_t s, const Dims &d, const HelmTab &h, const HelmTabF &hf, const uint8_t *st, double a_dt,
                          const double *b, const double *x, float *rf, float *e0, float *adt, const IbDev &ib,
-                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int pdl);
+                         const IbDevF &ibf, double *part, unsigned *count, double *dst, int nsm, int pdl);
 void launch_helm_jac32(cudaStream_t s, const Dims &d, const HelmTabF &h, const uint8_t *st, const float *adt,
                        const float *r, const float *e, float *en, double *x, const IbDevF &ib, int alone, int marching,
                        int pdl);

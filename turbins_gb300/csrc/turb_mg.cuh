@@ -89,6 +89,7 @@ struct MgHier {
     // 1: FP64 half sweeps and residuals of large levels march along k
     // (k_rbgs_col, k_resid_col); 0: k_rbgs, k_resid throughout
     int columns = 1;
+    int nsm = 1;   // SMs of the device
     // 1: the kernels of the V-cycle and of the CG step use programmatic dependent launch
     int pdl = 1;
     // from this level on (-1: never) the V-cycle runs as one launch of one
