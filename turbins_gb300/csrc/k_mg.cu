@@ -253,17 +253,16 @@ __global__ void __launch_bounds__(256, 4) k_resid_col(MgDevLevel Ld, int planes,
 }
 
 // The same half sweep on colour-split FP32 storage, four cells of one row per
-// thread (nx a multiple of 8) in each of `planes` planes (2 on the large
-// levels, 1 on the small ones, whose launches are latency-bound and need
-// every thread they can get): the cells' own
-// b and invd, their x-neighbours (other colour, indices m-1+p .. m+p for row
+// thread (nx a multiple of 8) in each of RB4_PLANES planes (the large levels;
+// k_rbgs4s takes the small ones, whose launches are latency-bound and need
+// every thread they can get): the cells' own b and invd, their x-neighbours (other colour, indices m-1+p .. m+p for row
 // parity p) and the j+-1 / k+-1 neighbours are float4 loads, the x metric
 // tables come as float4 from their parity-split copies (dxp / rlp / rrp),
 // indices are 32-bit, and the row constants are loaded once.  The arithmetic
 // per cell is s_row's, operation for operation.
-constexpr int RB4_PLANES = 2;                    // planes per thread on the large levels
+constexpr int RB4_PLANES = 2;                    // planes per thread of k_rbgs4
 constexpr long long RB4_PLANES_CELLS = 1ll << 22;   // levels of at least this many cells
-__global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, int planes, const float *b,
+__global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, const float *b,
                         const float *__restrict__ invd, float *x)
 {
     pdl_trigger();
@@ -275,8 +274,8 @@ __global__ void k_rbgs4(MgDevLevel Ld, int color, int zero_init, int planes, con
     const float dyj = Ld.dyf[j], ryj = Ld.rfyf[j], ryj1 = Ld.rfyf[j + 1];
 #pragma unroll
     for (int g = 0; g < RB4_PLANES; g++) {
-        const int k = blockIdx.z * planes + g;
-        if (g >= planes || k >= nz) break;
+        const int k = blockIdx.z * RB4_PLANES + g;
+        if (k >= nz) break;
         const int p = (color + j + k) & 1;
         const int m0 = (k * ny + j) * hx + 4 * q4;
         const float4 bb = *reinterpret_cast<const float4 *>(b + (size_t)color * half + m0);
@@ -1051,8 +1050,6 @@ __global__ void k_to_double_lev8(MgDevLevel L, const float *a, double *b)
         *reinterpret_cast<double2 *>(b + c0 + 2 * t) = make_double2((double)v[2 * t], (double)v[2 * t + 1]);
 }
 
-inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
-
 // a V-cycle kernel launch (the kernels start with pdl_trigger / pdl_wait, so that
 // with pdl a small level's launches overlap the drain of the kernel before them)
 template <typename K, typename... A>
@@ -1109,8 +1106,8 @@ void rb_half(cudaStream_t s, const MgHier<T> &H, int l, int color, int zero_init
             }
             if ((long long)L.nx * L.ny * L.nz >= RB4_PLANES_CELLS) {
                 launch_k(pdl, k_rbgs4,
-                         dim3(g4.x, g4.y, (unsigned)((L.nz + RB4_PLANES - 1) / RB4_PLANES)), B38, s, L, color, zero_init,
-                         RB4_PLANES, b, invd, x);
+                         dim3(g4.x, g4.y, (unsigned)((L.nz + RB4_PLANES - 1) / RB4_PLANES)), B38, s, L, color, zero_init, b,
+                         invd, x);
                 return;
             }
             // short rows share a warp: as few threads along x as cover the row

@@ -165,7 +165,6 @@ __device__ __forceinline__ int cell_at(const MgDevLevel &L, int i, int row, int 
 // (indices in units of T from its base) and its cells
 template <typename T>
 struct Lev {
-    static constexpr int CPT = Low<T>::CPT;
     int nx, ny, hx, pitch, wsz, rpc, r0, nloc, xo, co, ro, io, dr, dm, rl0, m0;
 
     __device__ __forceinline__ void open(const LowLev<T> &v, int rank)
@@ -508,9 +507,12 @@ __device__ __forceinline__ void low_visit(const LowLev<T> &v, int rank, bool dow
 template <typename T>
 __global__ void __launch_bounds__(LOW_THREADS, 1) k_vcycle_low(const __grid_constant__ LowArgs<T> arg)
 {
-    __shared__ LowArgs<T> a;   // the functions below read it many times
-    for (int t = threadIdx.x; t < (int)(sizeof(a) / 4); t += LOW_THREADS)
-        reinterpret_cast<unsigned *>(&a)[t] = reinterpret_cast<const unsigned *>(&arg)[t];
+    // a copy that the functions below read many times, as words: shared
+    // variables cannot have the initialisers of LowArgs' members
+    __shared__ __align__(16) unsigned args_sm[sizeof(LowArgs<T>) / 4];
+    for (int t = threadIdx.x; t < (int)(sizeof(LowArgs<T>) / 4); t += LOW_THREADS)
+        args_sm[t] = reinterpret_cast<const unsigned *>(&arg)[t];
+    const LowArgs<T> &a = *reinterpret_cast<const LowArgs<T> *>(args_sm);
     __syncthreads();
     unsigned char *const sm = low_sm;
     pdl_trigger();

@@ -829,7 +829,6 @@ int turb_net_create(int nx, int ny, int nz, int train, turb_net **out)
         const LayerDef &d = DEFS[l];
         n->woff[l] = off; off += 27LL * d.cin * d.cout;
         n->boff[l] = off; off += d.cout;
-        int lv = d.lev;
         n->wf[l] = n->alloc<bf16>(conv_pack_elems(d.cin, d.cout));
         n->wd[l] = n->alloc<bf16>(conv_pack_elems(d.cout, d.cin));
     }

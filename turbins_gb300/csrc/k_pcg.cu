@@ -43,10 +43,6 @@ __device__ __forceinline__ void block_store256(const double (&v)[NV], double *ds
 constexpr int KC = 4;   // planes per thread in the 3-D stencil kernels
 __device__ __forceinline__ long long blk3() { return ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x; }
 
-struct Cell {
-    int i, j, k;
-};
-
 // (S x)_c = dz_k [cxy x_c - sum_xy a_n x_n] + (dx dy) [zs x_c - zb x_b - zf x_f]
 // (+ the corner pin): the x and y face coefficients times the other cell
 // widths are constants of the thread's (i, j) column and are formed once,
@@ -475,7 +471,6 @@ __global__ void k_max_parts(const double *__restrict__ part, int n, double *__re
     }
 }
 
-long long ncell(const MgDevLevel &L) { return (long long)L.nx * L.ny * L.nz; }
 
 }  // namespace
 
