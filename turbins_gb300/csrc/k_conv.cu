@@ -1263,7 +1263,10 @@ int conv3_wgrad(cudaStream_t s, const bf16 *x, const bf16 *dy, int X, int Y, int
     WgArgs a{};
     tile_dims(X, Y, Z, a.bx, a.by, a.bz);
     a.nb = a.bx * a.by * a.bz;
-    if (a.nb % 16) { snprintf(g_conv_err, sizeof(g_conv_err), "wgrad grid below 16 voxels"); return 1; }
+    if (a.nb % 16) {   // of k_wgrad; a grid is taken or refused whichever kernel its channels choose
+        snprintf(g_conv_err, sizeof(g_conv_err), "wgrad voxel tile %dx%dx%d is no multiple of 16", a.bx, a.by, a.bz);
+        return 1;
+    }
     if (cin <= 32 && cout <= 32) {
         WgRowArgs r{};
         r.zring = X < 128;
