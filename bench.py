@@ -330,24 +330,21 @@ def run_reference(a, dist):
 # ---------------------------------------------------------------------------
 # FP64-pipe instructions per DA point of one launch of the group's kernel:
 # ncu's sm__pipe_fp64_cycles_active share x launch duration x the DFMA rate
-# measured here, divided by the launch's points, on single launches at
-# 256x128x128 (profiles/fp64_pipe_multi_bump_256x128x128.md); this counts the
-# compares and moves the FP64 pipe executes besides DADD / DMUL / DFMA.  A
-# pass advected by a bilinear transpose of another velocity costs 21.4
-# (y / z) or 21.8 (x) per point, a self-advected one 15.0; a step's passes
-# mix them 4:6 (y / z) and 2:3 (x).  The jacobi group's kernel is the FP64
-# Helmholtz residual.  Since that capture the y passes divide by the
-# stretched y spacings with the two-term quotient alone (every y spacing of
-# this workload passes the set-up's check): 3 divisions x 2 DFMA fewer per
-# point in half of the y / z launches, 17.6 - 3.0.
-FP64_OPS = {"eno_yz": 14.6, "eno_x": 17.7, "jacobi": 12.1}
+# measured here, divided by the launch's points, averaged over the launches of
+# one step at 512x256x256 (profiles/fp64_pipe_multi_bump_512x256x256.md); this
+# counts the compares and moves the FP64 pipe executes besides DADD / DMUL /
+# DFMA, and the lanes of a warp past the end of a row.  A y / z pass costs 9.3 to
+# 17.6 per point, an x pass 9.8 to 14.6, by the direction's spacings, the
+# advecting velocity's interpolation and the share of zeros.  The jacobi group's
+# kernel is the FP64 Helmholtz residual.
+FP64_OPS = {"eno_yz": 12.9, "eno_x": 11.8, "jacobi": 10.0}
 
 # DRAM bytes of one V-cycle of the mixed method at 512x256x256 (all its
 # kernels, dram__bytes_read.sum + dram__bytes_write.sum, one ncu pass;
-# profiles/vcycle_dram_multi_bump_512x256x256.md): 7.18 GB over its 198
-# launches, against 8.42 GB of algorithmic bytes (the coarse levels stay in
+# profiles/vcycle_dram_multi_bump_512x256x256.md): 7.19 GB over its 147
+# launches, against 8.41 GB of algorithmic bytes (the coarse levels stay in
 # L2).  Per launch, as the roofline's traffic of the mg group.
-MG_TRAFFIC_PER_LAUNCH = 7.18e9 / 198
+MG_TRAFFIC_PER_LAUNCH = 7.19e9 / 147
 
 
 def step_arm(ctx, api, dt, mode, guess, guess_stages=None):
