@@ -173,20 +173,20 @@ int turb_reset_pressure_history(turb_ctx *ctx);
 /* kernel variants, all giving the same bits: TURB_KV_MARCHING, the FP32
  * Helmholtz Jacobi sweeps and FP32 red-black half sweeps march along k
  * through shared-memory plane tiles (else one point, four cells, per thread);
- * TURB_KV_ENO_SEGMENTS, every y / z ENO line is walked in segments of about
- * 64 nodes by separate threads (else one thread per line); TURB_KV_PDL,
- * the kernels of the V-cycle, the conjugate-gradient step, the Helmholtz
- * solves and the network that the context runs are launched with
- * programmatic dependent launch, so that each may be scheduled while the one
- * before it drains (else plain stream order); TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level
- * of at most turb_set_mg_cluster cells down runs as one launch of one
- * thread-block cluster (16 blocks of 1024 threads, or 8 where 16 do not fit),
- * its phases separated by the hardware cluster barrier; TURB_KV_SWEEP_PAIRS,
- * the finest FP32 level (colour-split, nx a multiple of 64, ny of 32)
- * applies its red-black sweeps two at a time in one pass over memory: z
- * planes staged in shared memory by TMA, a wavefront of four half sweeps
- * along z over overlapped 64 x 32 tiles, the result in a second x array.
- * Default:
+ * TURB_KV_ENO_SEGMENTS, every y / z ENO line is walked in segments by separate
+ * threads, of as many nodes (1 to 32) as leave about 65536 threads (else one
+ * thread per line); TURB_KV_PDL, the kernels of the V-cycle, the
+ * conjugate-gradient step, the Helmholtz solves and the network that the
+ * context runs are launched with programmatic dependent launch, so that each
+ * may be scheduled while the one before it drains (else plain stream order);
+ * TURB_KV_CLUSTER_VCYCLE, the V-cycle from the first level of at most
+ * turb_set_mg_cluster cells down runs as one launch of one thread-block
+ * cluster (16 blocks of 1024 threads, or 8 where 16 do not fit), its phases
+ * separated by the hardware cluster barrier; TURB_KV_SWEEP_PAIRS, the finest
+ * FP32 level (colour-split, nx a multiple of 64, ny of 32) applies its
+ * red-black sweeps two at a time in one pass over memory: z planes staged in
+ * shared memory by TMA, a wavefront of four half sweeps along z over
+ * overlapped 64 x 32 tiles, the result in a second x array.  Default:
  * TURB_KV_ENO_SEGMENTS | TURB_KV_PDL (measured fastest on GB300 at
  * 512x256x256). */
 #define TURB_KV_MARCHING 1

@@ -17,10 +17,13 @@
 // be an FP64 operation is not one: magnitude and sign tests, zero and range
 // tests are integer operations on the words (dwords, turb_div.cuh); weights of
 // 1/2 become one sum and an exact scaling; on a uniform power-of-two spacing
-// quotients are scalings and the products with g2, g3 ride in an FMA.  Per
-// point: y 27 -> 17, x and z 16..25 -> 10..15.  Measured us per pass, x and
-// y/z, before and after: 128x64x64 32 / 128 -> 23 / 29, 256x128x128 196 / 217 ->
-// 132 / 153, 512x256x256 1400 / 1500 -> 928 / 1051 (FP64 pipe 72-80 % busy).
+// quotients are scalings and the products with g2, g3 ride in an FMA.
+// Measured FP64-pipe instructions per point at 512x256x256: y passes 11 (the
+// velocity a field) and 18 (a transpose), z 11 and 15, x 10 and 14 (15 and 21 to
+// 22 before, at 256x128x128).  Us per pass, x and y/z, before and after:
+// 128x64x64 32 / 128 -> 23 / 29, 256x128x128 196 / 217 -> 121 / 142, 512x256x256
+// 1400 / 1500 -> 901 / 991, the FP64 pipe 75-84 % active at 256x128x128 and
+// 80-85 % at 512x256x256.
 #include <algorithm>
 #include <type_traits>
 

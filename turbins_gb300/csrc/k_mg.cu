@@ -4,12 +4,12 @@
 // Pressure_form_LHS_matrix (Pressure.c:691-936).  CG runs in FP64 on the
 // volume-weighted form S = W A (W = cell volume), which is symmetric; the
 // corner pin of Pressure.c:864-868 is kept as an extra diagonal term.  The
-// preconditioner is one V-cycle: red-black Gauss-Seidel smoothing (2 pre, 2
-// post, reversed colour order on the way up so the cycle is symmetric),
-// restriction by summing children, piecewise-constant prolongation (its
-// transpose), rediscretised coarse operators built from the coarse cell
+// preconditioner is one V-cycle: red-black Gauss-Seidel smoothing (sweeps per
+// level set by the context, reversed colour order on the way up so the cycle is
+// symmetric), linear prolongation between cell centres, restriction by its
+// transpose, rediscretised coarse operators built from the coarse cell
 // widths (so coarsening follows the y stretching), semi-coarsening of the
-// directions whose mean spacing is more than twice the finest, and a dense
+// directions whose mean spacing is at most twice the finest, and a dense
 // inverse on the coarsest (<= 64 cells) level.  The V-cycle is templated on
 // its precision: FP64 (plain method) or FP32 inside the FP64 CG (mixed).
 //
@@ -140,7 +140,9 @@ __global__ void k_rbgs(MgDevLevel Ld, int color, int zero_init, const T *b, cons
 // its coefficients, which along k change only where dz or the face distances
 // do.  A thread keeps those of its columns and forms them again when a plane's
 // differ from those two planes (half sweep) or one plane (residual) before, so
-// uniform planes cost eight or nine; the values and their order are s_row's.
+// uniform planes cost eight or nine and the three compares of planes_differ
+// (measured 12.0 and 11.5 FP64-pipe instructions per cell, the first planes of
+// a block included); the values and their order are s_row's.
 template <typename T>
 struct ColCoef {
     T f[6];
@@ -165,9 +167,9 @@ __device__ __forceinline__ bool planes_differ(const LevelT<T> &L, int k, int s)
 }
 
 // The half sweep: a thread alternates between the columns i = 2 m, 2 m + 1.
-// 70 us per launch at 256x128x128 before, 62 with three blocks per SM, 58 with
-// four (64 registers), 64 % of the FP64 pipe; 4 or 16 planes per block were
-// slower than 8, and colour-split storage no faster.
+// 70 us per launch at 256x128x128 before, 62 with three blocks per SM, 59 with
+// four (64 registers, 60 bytes spilled), the FP64 pipe 80 % active; 4 or 16
+// planes per block were slower than 8, and colour-split storage no faster.
 // Two planes are loaded before either is stored (the cells read are of the
 // colour that is not written; x and b are not __restrict__, so nothing is read
 // before pdl_wait).
@@ -215,7 +217,8 @@ __global__ void __launch_bounds__(256, 4) k_rbgs_col(MgDevLevel Ld, int color, i
     }
 }
 
-// the residual r = b - S x (r in natural order) of a column of cells
+// the residual r = b - S x (r in natural order) of a column of cells: 104 us at
+// 256x128x128, the FP64 pipe 88 % active
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_resid_col(MgDevLevel Ld, int planes, const T *b, const T *x, T *r)
 {
@@ -792,7 +795,8 @@ __global__ void k_coarse(int n, const double *__restrict__ ainv, const T *b, T *
     for (int r = threadIdx.x; r < n; r += blockDim.x) coarse_row<T>(n, ainv, b, x, r);
 }
 
-// The V-cycle from level l0 down to the coarsest and back in one block of
+// Where the shared-memory cluster (k_mglow.cu) does not take the levels: the
+// V-cycle from level l0 down to the coarsest and back in one block of
 // TAIL_THREADS threads (levels small enough that a launch per half sweep
 // costs more than the sweep): the same per-cell operations as the kernels,
 // phases separated by block barriers.

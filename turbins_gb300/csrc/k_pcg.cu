@@ -1,7 +1,7 @@
 // k_pcg.cu -- FP64 conjugate-gradient vector kernels for the pressure solve
 // (volume-weighted system on the compact physical-cell layout).  Dot products
-// reduce by warp shuffles into a fixed set of per-block partials that one
-// block sums in a fixed order, so results are run-to-run deterministic.
+// reduce into a fixed set of per-block partials that the block which finishes
+// last sums in a fixed order, so results are run-to-run deterministic.
 #include <algorithm>
 
 #include "turb_internal.cuh"
@@ -522,7 +522,7 @@ void pcg_scatter(cudaStream_t s, const Dims &d, const MgDevLevel &L0, const doub
 
 // plane groups per block of the stencil kernels: as many as leave about seven
 // 256-thread blocks per SM (k_apply at 256x128x128, 4096 partials: 125 us
-// with one group, 109 us with four; at 128x64x64, 512 partials, fewer blocks
+// with one group, 111 us with four, the FP64 pipe 88 % active; at 128x64x64, 512 partials, fewer blocks
 // than one group gives would leave SMs idle)
 static int groups(const MgDevLevel &L0)
 {

@@ -98,9 +98,8 @@ struct DevBuf {
 // read conv.  FP64 Jacobi sweep: x, b, status read, x' written; FP64
 // Helmholtz residual: x, b, status read, FP32 r and first e written; FP32
 // Jacobi sweep: r, e, status read, e' written (the last one reads and writes
-// x instead).  An
-// immersed row: its diagonal, count, eight columns, values and x entries, b
-// and the row's result.
+// x instead).  An immersed row: its diagonal, count, eight columns, values and
+// x entries, b and the row's result.
 constexpr double ENO_X_BYTES = 24.0, ENO_YZ_BYTES = 32.0;
 constexpr double HELM_JACOBI_BYTES = 25.0, HELM_RESID64_BYTES = 25.0;
 constexpr double HELM_JAC32_BYTES = 13.0;

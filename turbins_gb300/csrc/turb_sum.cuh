@@ -7,7 +7,9 @@
 // block (a dot product's 256 elements are 8).  Here the pairs of all eight
 // warps are gathered in shared memory and added once each, 4 + 2 + 1 + 1 + 1
 // + 3 warp instructions, the same pairs at every distance, so the sums are
-// the same bits.  Measured at 256x128x128: see the kernels that use it.
+// the same bits.  With this and the sums ending in the launches that form them
+// (below), a step of the conjugate gradients' vector kernels went from 68 to
+// 30 us at 32x16x16 and from 252 to 227 us at 256x128x128.
 #pragma once
 
 // sums of NV values; the results are valid in thread 0.  Every thread of the
