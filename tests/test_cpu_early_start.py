@@ -96,3 +96,24 @@ def test_every_early_launch_follows_the_switch():
     assert re.search(r"if \(pdl\) \{\s*at\[n\]\.id = cudaLaunchAttributeProgrammaticStreamSerialization", src["k_mglow.cu"])
     flags = [m.group(1) for s in src.values() for m in re.finditer(r"\b(?:launch_early|launch_k|net_launch|launch_pairs)\(([^,]+),", s)]
     assert set(flags) <= {"pdl", "early", "H.pdl", "n->pdl", "int early", "int pdl"} and len(flags) > 40
+
+
+def test_every_kernel_launched_early_waits():
+    """a kernel launched with the attribute that never waited would run beside
+    the one ahead of it"""
+    untriggered, n = [], 0
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith(".cu"):
+            continue
+        path = os.path.join(CSRC, f)
+        body = {k[0]: k[2] for k in kernels(path)}
+        src = open(path).read()
+        launched = set(re.findall(r"\b(?:launch_early|launch_k|net_launch|launch_pairs)\([^,]+,\s*(k_\w+)", src))
+        launched |= set(re.findall(r"cudaLaunchKernelEx\(&cfg,\s*(k_\w+)", src))
+        launched |= {"k_helm_jac32v"} & set(body)   # launched through a variable
+        assert all("pdl_wait()" in body[k] for k in launched), f
+        untriggered += [k for k in sorted(launched) if "pdl_trigger()" not in body[k]]
+        n += len(launched)
+    assert n > 25
+    # the immersed rows' kernels let nothing start before they end
+    assert sorted(untriggered) == ["k_ib_jac32", "k_ib_resid64"]
