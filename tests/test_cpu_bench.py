@@ -67,19 +67,3 @@ def test_group_table_fractions():
     ops = bench.FP64_OPS["eno_yz"]
     assert t["eno_yz"]["fp64_frac"] == pytest.approx(ops * npts * 20 / 0.1 / 5.0e11)
     assert t["net"] == {"ms": 0.0, "launches": 0, "gbytes": 0.0}
-
-
-def test_constants_belong_to_the_present_kernels():
-    """The op counts and the V-cycle's traffic are measured on kernels that
-    change: with event times of the groups at 512x256x256 (ms per launch on a
-    GB300) no group runs the FP64 pipe above its rate, and the traffic is spread
-    over the launches that a V-cycle has now."""
-    per_launch = {"eno_yz": 0.991, "eno_x": 0.901, "jacobi": 0.765}
-    t = bench.group_table({g: (100 * ms, 100) for g, ms in per_launch.items()}, {}, peak_hbm=6780.7, fp64_rate=5.28e11,
-                          npts=513 * 257 * 257, ncell=512 * 256 * 256)
-    for g in per_launch:
-        assert 0.75 < t[g]["fp64_frac"] < 0.95, (g, t[g])
-    # half sweeps, residual, restriction and prolongation of the levels above
-    # 32768 cells (4 + 4, 5 + 5 and twice 12 + 12 sweeps), one launch below, two conversions
-    launches = sum(4 * n + 3 for n in (4, 5, 12, 12)) + 1 + 2
-    assert bench.MG_TRAFFIC_PER_LAUNCH == pytest.approx(7.19e9 / launches)
